@@ -339,12 +339,13 @@ int pcg_persistent(Matrix* A, int mode, const double* b, double* x, double rtol,
                    int32_t* nupd, int32_t* iters64, double* relres);
 // scalar rows up to which a system is solved by the persistent kernel
 constexpr int64_t kPersistentMaxRows = 262144;
-// pcg_persistent for several systems of ctx at once (GT_SOLVE_FP64 or
-// GT_SOLVE_IR), in shared cooperative launches; results bitwise those of
-// pcg_persistent on each system alone
+// pcg_persistent for several systems on ctx, in shared launches; results
+// bitwise those of pcg_persistent on each system alone.  clusters: every
+// system on one thread-block cluster (results bitwise those of the same call
+// on it alone)
 int pcg_persistent_groups(Ctx* ctx, const std::vector<Matrix*>& As, int mode, const std::vector<const double*>& b,
                           const std::vector<double*>& x, double rtol, int maxit, std::vector<gt_solve_info>& infos,
-                          std::vector<int>& status);
+                          std::vector<int>& status, bool clusters = false);
 int spmv64(Matrix* A, const double* x, double* y);
 // the persistent solver's grid barrier run alone (gt_pcg.cu): ctas CTAs wait
 // for ctas + missing arrivals with the given time limit

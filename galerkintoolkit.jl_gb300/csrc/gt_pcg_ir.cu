@@ -1,0 +1,13 @@
+// gt_pcg_ir.cu -- instances of the persistent Jacobi-PCG: FP32 iteration with FP64 reliable updates.
+#include "gt_pcg_impl.cuh"
+
+namespace gt {
+namespace pcg {
+
+template int run_groups_dispatch<float, float, true>(
+    Ctx*, Place, int, const std::vector<Matrix*>&, const std::vector<const float*>&,
+    const std::vector<const double*>&, const std::vector<double*>&, double, int, double, const std::vector<const PRun*>&,
+    std::vector<PRun>&, std::vector<int>&);
+
+}  // namespace pcg
+}  // namespace gt
