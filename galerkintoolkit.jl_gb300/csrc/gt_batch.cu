@@ -3,11 +3,13 @@
 // A batch holds n assembled matrices of block size 1 (scalar problems) or
 // 3 (3-D linear elasticity).  Instances are split by size (scalar rows):
 //
-//  * small instances (rows <= kSmallRows) are solved by ONE persistent
-//    launch: each CTA takes the next instance from a queue (largest first)
-//    and runs its whole Jacobi-PCG alone -- SpMV with G lanes per row, CTA
-//    reductions through shared memory, no inter-CTA synchronisation -- then
-//    takes the next one, so the device stays full however uneven the sizes;
+//  * small instances (rows <= kSmallRows) up to kOneCtaRows rows are solved
+//    by ONE persistent launch: each CTA takes the next instance from a queue
+//    (largest first) and runs its whole Jacobi-PCG alone -- SpMV with G lanes
+//    per row, CTA reductions through shared memory, no inter-CTA
+//    synchronisation -- then takes the next one, so the device stays full
+//    however uneven the sizes; the others by one thread-block cluster each
+//    (gt_pcg_local.cuh), largest first, in one launch per lane count;
 //  * medium instances (up to the persistent solver's 262,144 rows, matrices
 //    of the batch's own context, FP64 or mixed mode) share cooperative
 //    launches of the persistent solver: each one on the CTAs its own solve
@@ -33,7 +35,12 @@ namespace gt {
 
 constexpr int BT = 256;                 // threads per CTA of the batched kernel
 constexpr int BNW = BT / 32;
-constexpr int64_t kSmallRows = 32768;   // instances up to this size run one per CTA
+constexpr int64_t kSmallRows = 32768;   // largest instance of the small tier
+// Small instances up to this size run one per CTA, the others one per
+// cluster.  Measured on 16 uneven Poisson problems of 256 to 4,096 cells
+// (225 to 30,000 rows; assembly and mixed solves to 1e-10): 9.8 ms, 114 ms
+// with every one on one CTA, whose SM then holds the largest alone.
+constexpr int64_t kOneCtaRows = 1024;
 
 struct BInst {
   const int64_t* rowptr;
@@ -428,15 +435,44 @@ static int batch_solve(gt_batch* B, const double* b, double* x, double rtol, int
   std::vector<gt_solve_info> info(ni);
   std::vector<BRes> hres(ni);
   int status = GT_OK;
-  // small instances: one persistent launch
+  // x = 0 at the instances ids and their addresses, then the shared launches
+  // of the persistent solver (clusters: one cluster per instance)
+  auto groups = [&](const std::vector<int>& ids, bool clusters) -> int {
+    if (ids.empty()) return GT_OK;
+    std::vector<Matrix*> As;
+    std::vector<const double*> bs;
+    std::vector<double*> xs;
+    for (int i : ids) {
+      const int64_t off = B->h_inst[i].off;
+      As.push_back(B->mats[i]);
+      bs.push_back(b + off);
+      xs.push_back(x + off);
+      GT_CUDA(ctx, cudaMemsetAsync(x + off, 0, sizeof(double) * B->mats[i]->nbrows * B->mats[i]->bs, ctx->stream));
+    }
+    std::vector<gt_solve_info> ginf;
+    std::vector<int> gst;
+    GT_TRY(pcg_persistent_groups(ctx, As, mode, bs, xs, rtol, maxit, ginf, gst, clusters));
+    for (size_t k = 0; k < ids.size(); k++) {
+      info[ids[k]] = ginf[k];
+      if (gst[k] != GT_OK && gst[k] != GT_ERR_NOT_CONVERGED) return gst[k];
+      if (gst[k] == GT_ERR_NOT_CONVERGED) status = gst[k];
+    }
+    return GT_OK;
+  };
+  // small instances: one persistent launch, and one of clusters
+  std::vector<int> one, clustered;
+  for (int i : B->small) {
+    const int64_t rows = B->h_inst[i].nrows * B->h_inst[i].bs;
+    (rows <= kOneCtaRows ? one : clustered).push_back(i);
+  }
   if (mode == GT_SOLVE_FP64) {
-    GT_TRY((launch_small<double, double, true>(B, B->small, b, x, rtol, maxit, 0.0, 0, hres)));
+    GT_TRY((launch_small<double, double, true>(B, one, b, x, rtol, maxit, 0.0, 0, hres)));
   } else if (mode == GT_SOLVE_FP32) {
-    GT_TRY((launch_small<float, float, false>(B, B->small, b, x, rtol, maxit, 0.0, 0, hres)));
+    GT_TRY((launch_small<float, float, false>(B, one, b, x, rtol, maxit, 0.0, 0, hres)));
   } else {
-    GT_TRY((launch_small<float, float, true>(B, B->small, b, x, rtol, maxit, ctx->ir_delta, 0, hres)));
+    GT_TRY((launch_small<float, float, true>(B, one, b, x, rtol, maxit, ctx->ir_delta, 0, hres)));
     std::vector<int> stalled;
-    for (int i : B->small)
+    for (int i : one)
       if (hres[i].status == 2) stalled.push_back(i);
     if (!stalled.empty()) {
       // FP32 stalled (eps32 * cond ~ 1): these instances go on in FP64 from
@@ -451,13 +487,14 @@ static int batch_solve(gt_batch* B, const double* b, double* x, double rtol, int
       }
     }
   }
-  for (int i : B->small) {
+  for (int i : one) {
     info[i].iterations = hres[i].iters;
     info[i].outer_iterations = mode == GT_SOLVE_FP32 ? 0 : hres[i].nupd;
     info[i].rel_residual = hres[i].bb > 0 ? sqrt(hres[i].rr / hres[i].bb) : 0.0;
     if (mode == GT_SOLVE_FP64) info[i].fp64_iterations = hres[i].iters;
     if (hres[i].status != 0) status = GT_ERR_NOT_CONVERGED;
   }
+  GT_TRY(groups(clustered, true));
   mark(ctx, "batch_small");
   // medium instances of this context: grouped persistent launches
   std::vector<int> rest;
@@ -470,26 +507,7 @@ static int batch_solve(gt_batch* B, const double* b, double* x, double rtol, int
       else
         rest.push_back(i);
     }
-    if (!grouped.empty()) {
-      std::vector<Matrix*> As;
-      std::vector<const double*> bs;
-      std::vector<double*> xs;
-      for (int i : grouped) {
-        const int64_t off = B->h_inst[i].off;
-        As.push_back(B->mats[i]);
-        bs.push_back(b + off);
-        xs.push_back(x + off);
-        GT_CUDA(ctx, cudaMemsetAsync(x + off, 0, sizeof(double) * B->mats[i]->nbrows * B->mats[i]->bs, ctx->stream));
-      }
-      std::vector<gt_solve_info> ginf;
-      std::vector<int> gst;
-      GT_TRY(pcg_persistent_groups(ctx, As, mode, bs, xs, rtol, maxit, ginf, gst));
-      for (size_t k = 0; k < grouped.size(); k++) {
-        info[grouped[k]] = ginf[k];
-        if (gst[k] != GT_OK && gst[k] != GT_ERR_NOT_CONVERGED) return gst[k];
-        if (gst[k] == GT_ERR_NOT_CONVERGED) status = gst[k];
-      }
-    }
+    GT_TRY(groups(grouped, false));
   }
   mark(ctx, "batch_grouped");
   // large instances: the single-system solver, one after the other (each
