@@ -62,7 +62,7 @@ inline TabLayout tab_layout(int ctype, int order) {
   return L;
 }
 
-__device__ void lagrange1d(int order, double x, double* v, double* dv) {
+__host__ __device__ inline void lagrange1d(int order, double x, double* v, double* dv) {
   if (order == 1) {
     v[0] = 1.0 - x; v[1] = x; dv[0] = -1.0; dv[1] = 1.0;
   } else {
@@ -87,6 +87,9 @@ __device__ __forceinline__ double recip_nr2(double d) {
   return fma(r, e, r);
 }
 
+// one thread per (point, share of the nodes): threadIdx.x, threadIdx.y (Q2
+// hexahedra: 41 us by one thread a point, a chain of FP64 instructions at 63
+// clocks each)
 __global__ void k_tabulate(int ctype, int order, TabLayout L, double* tab) {
   int q = threadIdx.x;
   if (q >= L.nq) return;
@@ -123,17 +126,18 @@ __global__ void k_tabulate(int ctype, int order, TabLayout L, double* tab) {
     w = 1.0;
     for (int d = 0; d < L.D; d++) { x[d] = g[i[d]]; w *= gw[i[d]]; }
   }
-  tab[L.off_w + q] = w;
+  const int n0 = threadIdx.y, dn = blockDim.y;
+  if (n0 == 0) tab[L.off_w + q] = w;
   // geometry map gradients (P1 / Q1)
   if (ctype == GT_TET4) {
     const double gr[4][3] = {{-1, -1, -1}, {1, 0, 0}, {0, 1, 0}, {0, 0, 1}};
     const double v[4] = {1.0 - x[0] - x[1] - x[2], x[0], x[1], x[2]};  // barycentric coordinates
-    for (int n = 0; n < 4; n++) {
+    for (int n = n0; n < 4; n += dn) {
       tab[L.off_gv + q * 4 + n] = v[n];
       for (int d = 0; d < 3; d++) tab[L.off_gg + (q * 4 + n) * 3 + d] = gr[n][d];
     }
     if (order == 1) {
-      for (int n = 0; n < 4; n++) {
+      for (int n = n0; n < 4; n += dn) {
         tab[L.off_sv + q * 4 + n] = v[n];
         for (int d = 0; d < 3; d++) tab[L.off_sg + (q * 4 + n) * 3 + d] = gr[n][d];
       }
@@ -143,7 +147,7 @@ __global__ void k_tabulate(int ctype, int order, TabLayout L, double* tab) {
     // 4 l_i l_j, at the node order of the exponents (first index fastest)
     const int vi[10] = {0, -1, 1, -1, -1, 2, -1, -1, -1, 3};
     const int ei[10][2] = {{0, 0}, {0, 1}, {0, 0}, {0, 2}, {1, 2}, {0, 0}, {0, 3}, {1, 3}, {2, 3}, {0, 0}};
-    for (int n = 0; n < 10; n++) {
+    for (int n = n0; n < 10; n += dn) {
       double val, g[3];
       if (vi[n] >= 0) {
         const int i = vi[n];
@@ -161,12 +165,12 @@ __global__ void k_tabulate(int ctype, int order, TabLayout L, double* tab) {
   }
   double v1[3][3], d1[3][3];
   for (int d = 0; d < L.D; d++) lagrange1d(1, x[d], v1[d], d1[d]);
-  for (int n = 0; n < L.nlv; n++) {
+  for (int n = n0; n < L.nlv; n += dn) {
     double g = 1.0;
     for (int e = 0; e < L.D; e++) g *= v1[e][(n >> e) & 1];
     tab[L.off_gv + q * L.nlv + n] = g;
   }
-  for (int n = 0; n < L.nlv; n++)
+  for (int n = n0; n < L.nlv; n += dn)
     for (int d = 0; d < L.D; d++) {
       double g = 1.0;
       for (int e = 0; e < L.D; e++) {
@@ -178,7 +182,7 @@ __global__ void k_tabulate(int ctype, int order, TabLayout L, double* tab) {
   double vk[3][3], dk[3][3];
   for (int d = 0; d < L.D; d++) lagrange1d(order, x[d], vk[d], dk[d]);
   int m = order + 1;
-  for (int n = 0; n < L.nn; n++) {
+  for (int n = n0; n < L.nn; n += dn) {
     int e[3] = {n % m, (n / m) % m, n / (m * m)};
     double p = 1.0;
     for (int d = 0; d < L.D; d++) p *= vk[d][e[d]];
@@ -194,7 +198,7 @@ __global__ void k_tabulate(int ctype, int order, TabLayout L, double* tab) {
 static int get_tab(Ctx* ctx, int ctype, int order, double** tab, TabLayout* L) {
   *L = tab_layout(ctype, order);
   GT_TRY(dalloc(ctx, tab, L->total));
-  k_tabulate<<<GT_KC(ctx, 1), 32, 0, ctx->stream>>>(ctype, order, *L, *tab);
+  k_tabulate<<<GT_KC(ctx, 1), dim3(32, 8), 0, ctx->stream>>>(ctype, order, *L, *tab);
   GT_LAUNCH(ctx, "k_tabulate");
   return GT_OK;
 }
@@ -1117,8 +1121,11 @@ static int dispatch_form(const Space* sp, int form, const double* coef, double n
                          T* Ke, double* be, const double* f, const double* scoef, int want_matrix) {
   int bs = sp->ncomp;
   if (bs == 1) {
-    if (form == GT_LAPLACE)
-      return launch_elements<D, NLV, NN, NQ, 1, GT_LAPLACE, T, CPB, AFFINE>(sp, coef, nu, tab, L, Ke, be, f, scoef, want_matrix);
+    // (hexahedra and P2 tetrahedra: launch_direct)
+    if constexpr (!(D == 3 && (NN == 8 || NN == 10 || NN == 27)))
+      if (form == GT_LAPLACE)
+        return launch_elements<D, NLV, NN, NQ, 1, GT_LAPLACE, T, CPB, AFFINE>(sp, coef, nu, tab, L, Ke, be, f, scoef,
+                                                                              want_matrix);
     if (form == GT_MASS)
       return launch_elements<D, NLV, NN, NQ, 1, GT_MASS, T, CPB, AFFINE>(sp, coef, nu, tab, L, Ke, be, f, scoef, want_matrix);
   } else {
@@ -1133,6 +1140,42 @@ static int dispatch_form(const Space* sp, int form, const double* coef, double n
   return set_error(ctx_of(sp), GT_ERR_UNSUPPORTED, "weak form not supported on this space");
 }
 
+
+#include "gt_elements.cuh"
+
+// spaces whose Laplacian blocks and element vectors need no tabulation
+// (gt_elements.cuh).  The element vectors always come from there, whatever
+// the matrix's form: one source, so assemble_vector is bitwise the vector of
+// assemble_matrix_and_vector.
+static bool direct_space(const Space* sp) {
+  const int ct = sp->mesh->ctype;
+  return sp->ncomp == 1 && (ct == GT_HEX8 || (ct == GT_TET4 && sp->order == 2));
+}
+static bool direct_elements(const Space* sp, int form, int want_matrix) {
+  return direct_space(sp) && (form == GT_LAPLACE || !want_matrix);
+}
+template <class T>
+static int launch_direct(const Space* sp, const double* coef, T* Ke, double* be, const double* f, const double* scoef,
+                         int want_matrix) {
+  Ctx* ctx = ctx_of(sp);
+  const int64_t nc = sp->mesh->ncells;
+  const double* X = sp->mesh->coords;
+  const int32_t* cn = sp->mesh->cell_nodes;
+  if (sp->mesh->ctype == GT_TET4) {
+    const int smem = want_matrix ? (int)(128 * 101 * sizeof(T)) : 0;
+    GT_CUDA(ctx, cudaFuncSetAttribute(k_elements_p2<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    k_elements_p2<T><<<GT_KC(ctx, grid_for(nc, 128)), 128, smem, ctx->stream>>>(X, cn, coef, nc, Ke, be, f, scoef,
+                                                                                want_matrix, ctx->d_err);
+  } else if (sp->order == 1) {
+    k_elements_hex<2, T, 16><<<GT_KC(ctx, grid_for(nc, 16)), 256, 0, ctx->stream>>>(
+        X, cn, coef, line_1d(1), nc, Ke, be, f, scoef, want_matrix, ctx->d_err);
+  } else {
+    k_elements_hex<3, T, 4><<<GT_KC(ctx, grid_for(nc, 4)), 256, 0, ctx->stream>>>(
+        X, cn, coef, line_1d(2), nc, Ke, be, f, scoef, want_matrix, ctx->d_err);
+  }
+  GT_LAUNCH(ctx, "k_elements");
+  return GT_OK;
+}
 
 // P1 tetrahedra, scalar Laplacian / mass: one thread per cell.  The map is
 // affine, so J = [x1-x0, x2-x0, x3-x0] is constant over the cell and the
@@ -1414,6 +1457,11 @@ static int elements_T(const Space* sp, int form, const double* coef, double nu, 
     }
     return GT_OK;
   }
+  if (direct_elements(sp, form, want_matrix)) return launch_direct<T>(sp, coef, Ke, be, f, scoef, want_matrix);
+  if (be && direct_space(sp)) {
+    GT_TRY(launch_direct<T>(sp, nullptr, (T*)nullptr, be, f, scoef, 0));
+    be = nullptr;
+  }
   // P2 tets: the map is affine but the shape gradients vary over the cell, so
   // they are kept per quadrature point (the non-affine form of the kernel)
   if (ct == GT_TET4 && o == 2) return dispatch_form<3, 4, 10, 11, 8, false, T>(sp, form, coef, nu, tab, L, Ke, be, f, scoef, want_matrix);
@@ -1434,8 +1482,8 @@ int compute_elements(const Space* sp, int form, const double* d_coef, double nu,
   if (form == GT_ELASTICITY && sp->ncomp != sp->mesh->D)
     return set_error(ctx, GT_ERR_UNSUPPORTED, "linear elasticity needs a vector space (tensor_size = (D,))");
   double* tab = nullptr;
-  TabLayout L;
-  GT_TRY(get_tab(ctx, sp->mesh->ctype, sp->order, &tab, &L));
+  TabLayout L = tab_layout(sp->mesh->ctype, sp->order);
+  if (!direct_elements(sp, form, want_matrix)) GT_TRY(get_tab(ctx, sp->mesh->ctype, sp->order, &tab, &L));
   int s;
   if (precision == GT_FP32)
     s = elements_T<float>(sp, form, d_coef, nu, tab, L, (float*)Ke, be, f, d_scoef, want_matrix, chunks);
@@ -1655,7 +1703,8 @@ int compute_elements_with_tab(const Space* sp, int form, const double* d_coef, d
   if (form == GT_ELASTICITY && sp->ncomp != sp->mesh->D)
     return set_error(ctx, GT_ERR_UNSUPPORTED, "linear elasticity needs a vector space (tensor_size = (D,))");
   TabLayout L = tab_layout(sp->mesh->ctype, sp->order);
-  k_tabulate<<<GT_KC(ctx, 1), 32, 0, ctx->stream>>>(sp->mesh->ctype, sp->order, L, tab);
+  if (!direct_elements(sp, form, 1))
+    k_tabulate<<<GT_KC(ctx, 1), dim3(32, 8), 0, ctx->stream>>>(sp->mesh->ctype, sp->order, L, tab);
   GT_LAUNCH(ctx, "k_tabulate");
   if (precision == GT_FP32)
     return elements_T<float>(sp, form, d_coef, nu, tab, L, (float*)Ke, nullptr, nullptr, nullptr, 1);
@@ -3078,7 +3127,7 @@ struct HostCsr {
 // scattered in row chunks, each chunk's download overlapping the next chunk's
 // scatter (*values_done set when that happened).
 static int numeric_pass(Matrix* A, int form, NumIn& in, double nu, double* b_out, const HostCsr* hc,
-                        cudaEvent_t pat_down, bool* values_done, EarlyElems* early) {
+                        cudaEvent_t pat_down, bool* values_done, EarlyElems* early, bool* affine = nullptr) {
   const Space* sp = A->space;
   Ctx* ctx = ctx_of(sp);
   int64_t nc = sp->mesh->ncells;
@@ -3129,6 +3178,7 @@ static int numeric_pass(Matrix* A, int form, NumIn& in, double nu, double* b_out
   // scatter, over the same incidences
   if (s == GT_OK && !pre)
     s = kron_numeric(A, form, coef.p, nu, f.p, scoef.p, be, b_out ? bd : nullptr, b_out ? xd.p : nullptr, &used_kron);
+  if (affine) *affine = used_kron;
   if (s == GT_OK && !used_kron) {
     if (!pre) {
       s = dalloc(ctx, (unsigned char**)&Ke, (int64_t)(nc * ke_per_cell(sp) * esz));
@@ -3218,12 +3268,12 @@ static int numeric_pass(Matrix* A, int form, NumIn& in, double nu, double* b_out
 
 // FP32 values of a GT_MIXED matrix integrated in FP32 (FP64 Jacobian, its
 // inverse and determinant; FP32 element blocks and FP32 accumulation), on the
-// pattern the FP64 pass built
-static int fp32_values_pass(Matrix* A, int form, NumIn& in, double nu) {
+// pattern the FP64 pass built; affine: that pass took the factored path
+static int fp32_values_pass(Matrix* A, int form, NumIn& in, double nu, bool affine) {
   const Space* sp = A->space;
   Ctx* ctx = ctx_of(sp);
   int used = 0;
-  GT_TRY(kron_numeric(A, form, in.coef.p, nu, nullptr, nullptr, nullptr, nullptr, nullptr, &used));
+  if (affine) GT_TRY(kron_numeric(A, form, in.coef.p, nu, nullptr, nullptr, nullptr, nullptr, nullptr, &used));
   if (used) return GT_OK;
   void* Ke = nullptr;
   GT_TRY(dalloc(ctx, (unsigned char**)&Ke, (int64_t)(sp->mesh->ncells * ke_per_cell(sp) * sizeof(float))));
@@ -3241,9 +3291,10 @@ static int numeric_in(Matrix* A, int form, NumIn& in, double nu, double* b_out, 
                       cudaEvent_t pat_down = nullptr, bool* values_done = nullptr, EarlyElems* early = nullptr) {
   if (A->precision != GT_MIXED) return numeric_pass(A, form, in, nu, b_out, hc, pat_down, values_done, early);
   A->precision = GT_FP64;
-  int s = numeric_pass(A, form, in, nu, b_out, hc, pat_down, values_done, early);
+  bool affine = false;
+  int s = numeric_pass(A, form, in, nu, b_out, hc, pat_down, values_done, early, &affine);
   A->precision = GT_FP32;
-  if (s == GT_OK) s = fp32_values_pass(A, form, in, nu);
+  if (s == GT_OK) s = fp32_values_pass(A, form, in, nu, affine);
   A->precision = GT_MIXED;
   if (s == GT_OK && hc && values_done && *values_done && hc->v32 && A->bs == 1 && A->bnnz > 0)
     s = copy_out(ctx_of(A->space), hc->v32, A->val32, A->bnnz);

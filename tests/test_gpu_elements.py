@@ -1,0 +1,47 @@
+"""The element kernels without a quadrature loop over node pairs
+(csrc/gt_elements.cuh) against the oracle's quadrature, at cell counts around
+the cells per block (16 Q1 and 4 Q2 hexahedra, 32 and 128 P2 tetrahedra).
+
+An entry is a sum over at most 27 points (or an exact integral) of products of
+about ten factors: its rounding error stays below 100 eps of the sum of the
+terms' magnitudes, which is at most a few times the largest entry.  FP64: 100
+eps x 8 < 2e-13 of the largest entry; FP32 (FP64 geometry): 100 eps32 x 8 <
+1e-4, and 5e-6 for the 27 FP32 products of one entry added in sequence.
+"""
+import numpy as np
+import pytest
+
+import gtgpu as GT
+import oracle as O
+from test_gpu_parity import _oracle_space
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("cells,simplex,order", [
+    ((1, 1, 1), False, 1), ((2, 2, 3), False, 1), ((2, 2, 4), False, 1), ((2, 3, 3), False, 1),
+    ((1, 1, 1), False, 2), ((2, 2, 2), False, 2), ((3, 3, 3), False, 2), ((5, 3, 2), False, 2),
+    ((1, 1, 1), True, 2), ((2, 4, 2), True, 2), ((11, 2, 2), True, 2), ((4, 4, 4), True, 2),
+])
+def test_laplacian_blocks(cells, simplex, order):
+    m = GT.cartesian_mesh((0.0, 1.0, -0.5, 2.0, 0.0, 0.7), cells, simplexify=simplex)
+    # every node moved, also those on the boundary (single layers of cells)
+    m.coords += np.random.default_rng(3).uniform(-0.1, 0.1, m.coords.shape) / max(cells)
+    coef = GT.lognormal_cells(m.num_cells, 1.0, 17)
+    ref, _ = _oracle_space(m, order, 1, None)
+    cp, rv, nz = O.assemble_matrix(ref, O.LAPLACE, 2 * order, coef=coef)
+    orp, oci, ov = O.csc_to_csr(cp, rv, nz, ref["nfree"])
+    ob = O.assemble_vector(ref, 2 * order, 1.0)
+    V = GT.lagrange_space(GT.interior(m), order)
+    A, b = GT.assemble_matrix_and_vector(GT.laplacian(coef), GT.source(1.0), "mixed", V)
+    rp, ci, v = A.csr()
+    assert np.array_equal(rp, orp) and np.array_equal(ci, oci)
+    scale = np.abs(ov).max()
+    assert np.abs(v - ov).max() <= 2e-13 * scale
+    assert np.abs(A.values32() - ov).max() <= 5e-6 * scale
+    assert np.abs(b - ob).max() <= 2e-13 * np.abs(ob).max()
+    # the row sums of a pure Neumann Laplacian vanish, and the matrix is symmetric
+    import scipy.sparse as sp
+    M = sp.csr_matrix((v, ci, rp))
+    assert np.abs(M @ np.ones(M.shape[0])).max() <= 2e-12 * scale
+    assert abs(M - M.T).max() <= 2e-13 * scale
