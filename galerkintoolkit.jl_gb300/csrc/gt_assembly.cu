@@ -357,20 +357,48 @@ __device__ __forceinline__ int32_t warp_sort(int32_t v, int lane) {
   return v;
 }
 
+// ascending bitonic sort of NR * 32 keys, key r * 32 + lane in v[r] of a lane:
+// the steps below 32 are shuffles, those above exchange registers of a lane
+template <int NR>
+__device__ __forceinline__ void warp_sort_regs(int32_t (&v)[NR], int lane) {
+#pragma unroll
+  for (int k = 2; k <= NR * 32; k <<= 1)
+#pragma unroll
+    for (int j = k >> 1; j > 0; j >>= 1)
+#pragma unroll
+      for (int r = 0; r < NR; r++) {
+        // ascending where bit k of the key's index is clear
+        const bool up = k < 32 ? (lane & k) == 0 : ((r * 32) & k) == 0;
+        if (j < 32) {
+          const int32_t o = __shfl_xor_sync(0xffffffffu, v[r], j);
+          v[r] = ((lane & j) == 0) == up ? min(v[r], o) : max(v[r], o);
+        } else {
+          const int p = r ^ (j >> 5);
+          if (p > r) {
+            const int32_t a = min(v[r], v[p]), b = max(v[r], v[p]);
+            v[r] = up ? a : b;
+            v[p] = up ? b : a;
+          }
+        }
+      }
+}
+
 // Per block row: the sorted union of the free node DOFs of its cells.
 // One warp per row.  The row's incidences are sorted ascending (= by cell;
 // the count pass writes them back, which fixes the scatter's summation
 // order) and held one per lane.  The row's own DOF (block row r is node
 // r + 1, present in every incident cell) goes in first; the other nodes of
-// the incident cells follow in rounds of 32 candidates.  In a round, lanes
-// holding the same key elect one leader (match.any), so a shared-memory hash
-// set (linear probing, empty = -1) sees each key at most once per round and
-// its compare-and-swaps never serialise on one address; a leader that
-// inserted appends its key to the row's list (ballot + prefix count).  The
-// count pass counts the distinct keys and, for rows of at most S columns,
-// sorts them (register shuffles for <= 32 keys, shared-memory bitonic sort
-// above) into the row's slot of S entries; the fill pass copies those slots
-// and runs the hash again only for longer rows.
+// the incident cells follow in rounds of 32 candidates.  A shared-memory hash
+// set (linear probing, empty = -1, sized by the row's candidates) takes each
+// key once; a lane that inserted appends its key to the row's list (ballot +
+// prefix count).  (A cell's nodes are distinct, so at most two or three lanes
+// of a round hold the same key; electing one by match.any first cost more than
+// their compare-and-swaps do.)  The count pass counts the distinct keys and,
+// for rows of at most S columns, sorts them (in registers up to 128 keys,
+// bitonic in shared memory above) into the row's slot of S entries; the fill
+// pass copies those slots and runs the hash again only for longer rows.
+// Bound by instruction issue: 65^2 x 64 Q2 hexahedron rows (64 columns on
+// average, up to 125) 511 -> 228 us, 41^3 P2 tetrahedron rows 62 -> 45 us.
 template <int NN, int S, bool FILL>
 __global__ void __launch_bounds__(256) k_pattern(const int64_t* __restrict__ inc_ptr, int32_t* __restrict__ inc,
                                                  const int32_t* __restrict__ cnd, int64_t nrows, int hcap, int icap,
@@ -398,7 +426,9 @@ __global__ void __launch_bounds__(256) k_pattern(const int64_t* __restrict__ inc
     if (lane == 0) { atomicOr(err, DEV_ERR_ROW_CAP); if (!FILL) { rowcnt[r] = 0; small[r] = 1; } }
     return;
   }
-  for (int i = lane; i < (hcap >> 2); i += 32) reinterpret_cast<int4*>(tab)[i] = make_int4(-1, -1, -1, -1);
+  // load factor <= 0.8 even if every candidate were distinct
+  const int hsz = ncand <= 25 ? 32 : 1 << (32 - __clz(ncand + (ncand >> 2) - 1));
+  for (int i = lane; i < (hsz >> 2); i += 32) reinterpret_cast<int4*>(tab)[i] = make_int4(-1, -1, -1, -1);
   int32_t myinc = INT_MAX;  // lane k: the k-th incidence (rows of at most 32)
   if (ninc <= 32) {
     const int32_t u = lane < ninc ? inc[ib + lane] : INT_MAX;
@@ -419,7 +449,7 @@ __global__ void __launch_bounds__(256) k_pattern(const int64_t* __restrict__ inc
     for (int i = lane; i < ninc; i += 32) ibuf[i] = inc[ib + i];
   }
   __syncwarp();
-  const unsigned hmask = (unsigned)hcap - 1u;
+  const unsigned hmask = (unsigned)hsz - 1u;
   const unsigned lt = (1u << lane) - 1u;
   if (lane == 0 && ninc > 0) {
     tab[((unsigned)r * 2654435761u) & hmask] = (int32_t)r;
@@ -443,9 +473,8 @@ __global__ void __launch_bounds__(256) k_pattern(const int64_t* __restrict__ inc
         if (d > 0) key = d - 1;
       }
     }
-    const unsigned peers = __match_any_sync(0xffffffffu, key);
     bool ins = false;
-    if (key >= 0 && (peers & lt) == 0) {
+    if (key >= 0) {
       unsigned h = ((unsigned)key * 2654435761u) & hmask;
       bool done = false;
       for (unsigned probe = 0; probe <= hmask; probe++) {
@@ -486,7 +515,20 @@ __global__ void __launch_bounds__(256) k_pattern(const int64_t* __restrict__ inc
     }
     return;
   }
-  int P = 64;
+  auto sorted = [&](auto nr) {
+    constexpr int NR = decltype(nr)::value;
+    int32_t v[NR];
+#pragma unroll
+    for (int q = 0; q < NR; q++) v[q] = q * 32 + lane < total ? keys[q * 32 + lane] : INT_MAX;
+    warp_sort_regs<NR>(v, lane);
+    int32_t* out = FILL ? colind + rowptr[r] : slots + r * S;
+#pragma unroll
+    for (int q = 0; q < NR; q++)
+      if (q * 32 + lane < total) out[q * 32 + lane] = v[q];
+  };
+  if (total <= 64) return sorted(std::integral_constant<int, 2>());
+  if (total <= 128) return sorted(std::integral_constant<int, 4>());
+  int P = 256;
   while (P < total) P <<= 1;
   for (int i = total + lane; i < P; i += 32) keys[i] = INT_MAX;
   __syncwarp();
@@ -662,26 +704,27 @@ __global__ void __launch_bounds__(128) k_pattern_rows(const int64_t* __restrict_
 }
 
 // colind of the rows whose sorted columns the count pass left in their slot
-// of S entries: four lanes per row, each copying a quarter of the row with
-// 16-byte slot loads (slots are 16-byte aligned), all loads in flight
+// of S entries: S / 8 lanes per row (4 of short rows, 16 of long ones), each
+// with two 16-byte slot loads in flight (slots are 16-byte aligned), spaced so
+// that the row's lanes read and write adjacent entries
 template <int S>
 __global__ void k_copy_slots(const int64_t* __restrict__ rowptr, const int32_t* __restrict__ slots, int64_t nrows,
                              int32_t* __restrict__ colind) {
+  constexpr int LPR = S / 8;
   int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  int64_t r = t >> 2;
-  int q = (int)(t & 3);
+  int64_t r = t / LPR;
+  int q = (int)(t % LPR);
   if (r >= nrows) return;
   const int64_t o = rowptr[r];
   const int n = (int)(rowptr[r + 1] - o);
-  constexpr int V4 = S / 16;  // int4 loads per lane
-  const int4* src = reinterpret_cast<const int4*>(slots + r * S) + q * V4;
-  int4 v[V4];
+  const int4* src = reinterpret_cast<const int4*>(slots + r * S);
+  int4 v[2];
 #pragma unroll
-  for (int k = 0; k < V4; k++)
-    if ((q * V4 + k) * 4 < n) v[k] = __ldg(src + k);
+  for (int k = 0; k < 2; k++)
+    if ((k * LPR + q) * 4 < n) v[k] = __ldg(src + k * LPR + q);
 #pragma unroll
-  for (int k = 0; k < V4; k++) {
-    const int b = (q * V4 + k) * 4;
+  for (int k = 0; k < 2; k++) {
+    const int b = (k * LPR + q) * 4;
     if (b < n) colind[o + b] = v[k].x;
     if (b + 1 < n) colind[o + b + 1] = v[k].y;
     if (b + 2 < n) colind[o + b + 2] = v[k].z;
@@ -756,13 +799,16 @@ static int launch_pattern(Matrix* A, int32_t maxinc, const int32_t* bucket, bool
   int64_t nrows = A->nbrows;
   // hash table: load factor <= 0.8 even if every candidate were distinct;
   // ibuf holds the row's incidences, then the compacted keys (<= candidates)
-  // (the warp kernel's sizes need the longest incidence list, maxinc < 0:
-  // not known yet -- the row-per-thread pass does without it)
+  // (the warp kernel's exact sizes need the longest incidence list, a host
+  // round trip; it first runs with room for kCandFirst candidates a row -- 8
+  // hexahedra, 25 tetrahedra -- and again with the exact sizes if a row has
+  // more)
+  constexpr int kCandFirst = 256;
   int hcap = 32, icap = 32, warps = 8;
   size_t smem = 0;
-  auto setup_warp = [&]() -> int {
-    if (maxinc < 0) GT_TRY(max_diff(ctx, A->inc_ptr, nrows, &maxinc));
-    const int ncand_max = maxinc * NN;
+  auto setup_warp = [&](bool exact) -> int {
+    if (exact && maxinc < 0) GT_TRY(max_diff(ctx, A->inc_ptr, nrows, &maxinc));
+    const int ncand_max = exact ? maxinc * NN : kCandFirst;
     hcap = 32;
     icap = 32;
     while (hcap < ncand_max + ncand_max / 4) hcap <<= 1;
@@ -783,8 +829,8 @@ static int launch_pattern(Matrix* A, int32_t maxinc, const int32_t* bucket, bool
   GT_TRY(dalloc(ctx, &A->rowptr, nrows + 1));
   // count pass: one thread per row where rows are short enough, else (or when
   // a row turned out longer than 32 incidences or columns) one warp per row
-  bool rows_pass = NN <= 8 && S == kRowsS && ctx->pattern_rows;
-  if (!rows_pass) GT_TRY(setup_warp());
+  bool rows_pass = NN <= 8 && S == kRowsS && ctx->pattern_rows, exact = false;
+  if (!rows_pass) GT_TRY(setup_warp(false));
   int32_t* dredo = nullptr;
   GT_TRY(dalloc(ctx, &dredo, 1));
   int32_t* dlast = nullptr;
@@ -826,10 +872,17 @@ static int launch_pattern(Matrix* A, int32_t maxinc, const int32_t* bucket, bool
     // bits of kernels on other streams (element checks) go back for the next take
     const uint32_t own = DEV_ERR_ROW_CAP | DEV_ERR_HASH_FULL;
     ctx->held_err |= bits & ~own;
-    if (bits & own) return set_error(ctx, GT_ERR_INVALID, "sparsity: row capacity exceeded");
+    const bool cap = bits & DEV_ERR_ROW_CAP;
+    if ((bits & DEV_ERR_HASH_FULL) || (cap && (rows_pass || exact)))
+      return set_error(ctx, GT_ERR_INVALID, "sparsity: row capacity exceeded");
     int32_t redo = 0;
     memcpy(&redo, &ctx->h_scratch[2], sizeof(int32_t));
-    if (!rows_pass || !redo) break;
+    if (!(rows_pass ? redo != 0 : cap)) break;
+    exact = true;
+    if (!rows_pass) {  // a row beyond kCandFirst candidates
+      GT_TRY(setup_warp(true));
+      continue;
+    }
     rows_pass = false;  // a row beyond 32 incidences or columns: count again, one warp per row
     if (bucket) {
       // the buckets kept only the first kIncBucket incidences of each row:
@@ -838,7 +891,7 @@ static int launch_pattern(Matrix* A, int32_t maxinc, const int32_t* bucket, bool
       dfree(ctx, A->inc);
       GT_TRY(build_incidence(ctx, sp, &A->inc_ptr, &A->inc, &A->ninc, false));
     }
-    GT_TRY(setup_warp());
+    GT_TRY(setup_warp(true));
   }
   dfree(ctx, dredo);
   dfree(ctx, dlast);
@@ -853,10 +906,10 @@ static int launch_pattern(Matrix* A, int32_t maxinc, const int32_t* bucket, bool
   GT_TRY(dalloc(ctx, &A->colind, A->bnnz));
   if (nrows > 0 && mr <= S) {
     // every row fit its slot: a plain coalesced copy
-    k_copy_slots<S><<<GT_KC(ctx, grid_for(nrows * 4, 256)), 256, 0, st>>>(A->rowptr, slots, nrows, A->colind);
+    k_copy_slots<S><<<GT_KC(ctx, grid_for(nrows * (S / 8), 256)), 256, 0, st>>>(A->rowptr, slots, nrows, A->colind);
     GT_LAUNCH(ctx, "k_copy_slots");
   } else if (nrows > 0) {
-    if (smem == 0) GT_TRY(setup_warp());
+    if (smem == 0) GT_TRY(setup_warp(true));
     const int grid = grid_for(nrows, warps);
     k_pattern<NN, S, true><<<GT_KC(ctx, grid), warps * 32, smem, st>>>(A->inc_ptr, A->inc, sp->cell_ndofs, nrows,
                                                                        hcap, icap, nullptr, A->rowptr, A->colind,
