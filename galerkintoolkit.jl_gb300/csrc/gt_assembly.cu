@@ -1804,16 +1804,29 @@ __device__ __forceinline__ void load_partial(const int64_t ib, int64_t ie, int j
 // s_j; two butterfly steps combine them): one FP64 add per lane per four
 // incidences, where a single lane summing in sequence would issue a warp
 // FP64 instruction per incidence.  Every lane of the group gets the sums.
-template <int BS>
+template <int BS, int G>
 __device__ __forceinline__ void row_load_sum(const int64_t ib, int64_t ie, const int32_t* __restrict__ inc, int nn,
                                              const double* __restrict__ be, int gl, unsigned gmask, double* out) {
-  double s[BS];
-  load_partial<BS>(ib, gl < 4 ? ie : ib, gl, inc, nn, BS, be, s);
+  if constexpr (BS > 1 && G >= 4 * BS) {
+    // block rows: lane j + 4 cc forms component cc's s_j, so a step is one
+    // FP64 instruction for all components
+    const int j = gl & 3, cc = gl >> 2;
+    double s = 0.0;
+    if (cc < BS)
+      for (int64_t k = ib + j; k < ie; k += 4) s += __ldg(be + (int64_t)__ldg(inc + k) * BS + cc);
+    s += __shfl_xor_sync(gmask, s, 1);
+    s += __shfl_xor_sync(gmask, s, 2);
 #pragma unroll
-  for (int cc = 0; cc < BS; cc++) {
-    s[cc] += __shfl_xor_sync(gmask, s[cc], 1);
-    s[cc] += __shfl_xor_sync(gmask, s[cc], 2);
-    out[cc] = s[cc];
+    for (int c = 0; c < BS; c++) out[c] = __shfl_sync(gmask, s, 4 * c, G);
+  } else {
+    double s[BS];
+    load_partial<BS>(ib, gl < 4 ? ie : ib, gl, inc, nn, BS, be, s);
+#pragma unroll
+    for (int cc = 0; cc < BS; cc++) {
+      s[cc] += __shfl_xor_sync(gmask, s[cc], 1);
+      s[cc] += __shfl_xor_sync(gmask, s[cc], 2);
+      out[cc] = s[cc];
+    }
   }
 }
 
@@ -1860,7 +1873,7 @@ __global__ void k_scatter(const int64_t* __restrict__ rowptr, const int32_t* __r
     double bsum[BS];
     int64_t ib = inc_ptr[r], ie = inc_ptr[r + 1];
     if (be != nullptr) {
-      row_load_sum<BS>(ib, ie, inc, nn, be, gl, gmask, bsum);
+      row_load_sum<BS, G>(ib, ie, inc, nn, be, gl, gmask, bsum);
     } else {
 #pragma unroll
       for (int cc = 0; cc < BS; cc++) bsum[cc] = 0.0;
@@ -2021,7 +2034,7 @@ __global__ void __launch_bounds__(128) k_scatter_p1(const int64_t* __restrict__ 
   }
   const int64_t ib = inc_ptr[r], ie = inc_ptr[r + 1];
   double bsum = 0.0;
-  if (be != nullptr) row_load_sum<1>(ib, ie, inc, 4, be, b, gmask, &bsum);
+  if (be != nullptr) row_load_sum<1, G>(ib, ie, inc, 4, be, b, gmask, &bsum);
   for (int64_t k0 = ib; k0 < ie; k0 += U) {
     int32_t jj[U], key[U];
     int pos[U];
@@ -2179,31 +2192,25 @@ int scatter_matrix(Matrix* A, const void* Ke, int ke_precision, int out_precisio
 // ---------------------------------------------------------------------------
 constexpr int GSTRIDE = 10;  // per-cell geometry record: 9 + 1 values
 
-__device__ void lagrange_table_1d(int order, double* M, double* Dm, double* Kd, double* m1) {
-  int n1 = order + 1;
-  double g[3], gw[3];
-  if (n1 == 2) {
-    double s = 0.5 / sqrt(3.0);
-    g[0] = 0.5 - s; g[1] = 0.5 + s; gw[0] = gw[1] = 0.5;
-  } else {
-    double s = 0.5 * sqrt(0.6);
-    g[0] = 0.5 - s; g[1] = 0.5; g[2] = 0.5 + s;
-    gw[0] = 5.0 / 18.0; gw[1] = 8.0 / 18.0; gw[2] = 5.0 / 18.0;
-  }
-  for (int i = 0; i < 9; i++) M[i] = Dm[i] = Kd[i] = 0.0;
-  for (int i = 0; i < 3; i++) m1[i] = 0.0;
-  for (int q = 0; q < n1; q++) {
-    double v[3], dv[3];
-    lagrange1d(order, g[q], v, dv);
-    for (int i = 0; i < n1; i++) {
-      m1[i] += gw[q] * v[i];
-      for (int j = 0; j < n1; j++) {
-        M[i * 3 + j] += gw[q] * v[i] * v[j];
-        Dm[i * 3 + j] += gw[q] * dv[i] * v[j];
-        Kd[i * 3 + j] += gw[q] * dv[i] * dv[j];
+// the 1-D matrices of the factored path, formed on the host and passed by
+// value (by one thread of every block they took 10 us, a chain of FP64
+// instructions at 63 clocks each)
+struct Tables1D {
+  double M[9], Dm[9], Kd[9], m1[3];
+};
+static Tables1D tables_1d(int order) {
+  const Line1D l = line_1d(order);
+  Tables1D t{};
+  for (int q = 0; q <= order; q++)
+    for (int i = 0; i <= order; i++) {
+      t.m1[i] += l.w[q] * l.L[q][i];
+      for (int j = 0; j <= order; j++) {
+        t.M[i * 3 + j] += l.w[q] * l.L[q][i] * l.L[q][j];
+        t.Dm[i * 3 + j] += l.w[q] * l.dL[q][i] * l.L[q][j];
+        t.Kd[i * 3 + j] += l.w[q] * l.dL[q][i] * l.dL[q][j];
       }
     }
-  }
+  return t;
 }
 
 // geometry record of one affine QUAD4/HEX8 cell: J^-1 (elasticity) or the
@@ -2285,70 +2292,78 @@ __device__ __forceinline__ bool affine_record(const double* __restrict__ coords,
   return affine;
 }
 
-// the record of cell 0: the reference of the uniformity test
-// (gref[0..GSTRIDE-1) the record, gref[GSTRIDE-1] |det J|)
-template <int D, int NV>
-__global__ void k_geom_ref(const double* __restrict__ coords, const int32_t* __restrict__ cell_nodes, int form,
-                           double* __restrict__ gref) {
-  if (blockIdx.x != 0 || threadIdx.x != 0) return;
-  double gv[GSTRIDE], adet, det;
-  affine_record<D, NV>(coords, cell_nodes, 0, form, gv, adet, det);
-  gv[GSTRIDE - 1] = adet;
-#pragma unroll
-  for (int i = 0; i < GSTRIDE; i++) gref[i] = gv[i];
-}
-
-// per-cell records G[c] = {record, scale = |det J| coef_c} (+ the load
-// vector), affinity check, and -- with gref -- the uniformity test: a cell
+// Per-cell records G[c] = {record, scale = |det J| coef_c} (+ the element
+// vectors), affinity check, and -- with gref -- the uniformity test: a cell
 // whose record and |det J| differ from cell 0's by more than 1e-13 of the
-// largest record entry (of |det J|) sets *nonuniform
+// largest record entry (of |det J|) sets *nonuniform.  gref receives cell 0's
+// record (gref[0..GSTRIDE-1)) and |det J| (gref[GSTRIDE-1]); every block forms
+// it in a warp of its own beside the cells'.
+// A chain of about 110 FP64 instructions at 63 clocks each, so blocks of 64
+// cells spread the cells over the SMs, and the element vectors are written by
+// all threads in order (one multiplication an entry).  Measured, Q2
+// elasticity 15^3 FP64: 40 -> 14 us (and 4 us of a launch for cell 0), 2-D Q1
+// 64^2: 12 + 3 -> 7 us.
+constexpr int GCELLS = 64;  // cells per block
 template <int D, int NV>
-__global__ void __launch_bounds__(256) k_geom_affine(const double* __restrict__ coords,
-                                                     const int32_t* __restrict__ cell_nodes,
-                                                     const double* __restrict__ coef, int form, int order,
-                                                     int64_t ncells, int nn, int bs, void* __restrict__ Gout, int g64,
-                                                     double* __restrict__ be, const double* __restrict__ fsrc,
-                                                     const double* __restrict__ scoef, uint32_t* nonaffine,
-                                                     uint32_t* err, const double* __restrict__ gref,
-                                                     uint32_t* nonuniform) {
-  __shared__ double s_m1[3];
-  if (threadIdx.x == 0) {
-    double M[9], Dm[9], Kd[9];
-    lagrange_table_1d(order, M, Dm, Kd, s_m1);
+__global__ void __launch_bounds__(GCELLS + 32) k_geom_affine(
+    const double* __restrict__ coords, const int32_t* __restrict__ cell_nodes, const double* __restrict__ coef, int form,
+    int order, Tables1D tab, int64_t ncells, int nn, int bs, void* __restrict__ Gout, int g64, double* __restrict__ be,
+    const double* __restrict__ fsrc, const double* __restrict__ scoef, uint32_t* nonaffine, uint32_t* err,
+    double* __restrict__ gref, uint32_t* nonuniform) {
+  __shared__ double s_w[kMaxNodesPerCell], s_sf[GCELLS][3], s_ref[GSTRIDE];
+  const int tid = threadIdx.x;
+  const int64_t c0 = blockIdx.x * (int64_t)GCELLS, c = c0 + tid;
+  const bool cell = tid < GCELLS && c < ncells;
+  double gv[GSTRIDE], adet = 0.0, det;
+  if (cell) {
+    if (!affine_record<D, NV>(coords, cell_nodes, c, form, gv, adet, det)) atomicOr(nonaffine, 1u);
+    if (!(det != 0.0)) atomicOr(err, DEV_ERR_DEGENERATE);
+  } else if (tid == GCELLS && gref) {
+    affine_record<D, NV>(coords, cell_nodes, 0, form, gv, adet, det);
+    gv[GSTRIDE - 1] = adet;
+#pragma unroll
+    for (int i = 0; i < GSTRIDE; i++) {
+      s_ref[i] = gv[i];
+      if (blockIdx.x == 0) gref[i] = gv[i];
+    }
+  }
+  if (be && tid < nn) {
+    const int m1 = order + 1, e0 = tid % m1, e1 = (tid / m1) % m1, e2 = tid / (m1 * m1);
+    s_w[tid] = tab.m1[e0] * tab.m1[e1] * (D == 3 ? tab.m1[e2] : 1.0);
   }
   __syncthreads();
-  int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (c >= ncells) return;
-  double gv[GSTRIDE], adet, det;
-  if (!affine_record<D, NV>(coords, cell_nodes, c, form, gv, adet, det)) atomicOr(nonaffine, 1u);
-  if (!(det != 0.0)) atomicOr(err, DEV_ERR_DEGENERATE);
-  if (gref) {
-    double gm = 0.0;
+  if (cell) {
+    if (gref) {
+      double gm = 0.0;
 #pragma unroll
-    for (int i = 0; i < D * D; i++) gm = fmax(gm, fabs(gref[i]));
-    bool same = fabs(adet - gref[GSTRIDE - 1]) <= 1e-13 * gref[GSTRIDE - 1];
+      for (int i = 0; i < D * D; i++) gm = fmax(gm, fabs(s_ref[i]));
+      bool same = fabs(adet - s_ref[GSTRIDE - 1]) <= 1e-13 * s_ref[GSTRIDE - 1];
 #pragma unroll
-    for (int i = 0; i < D * D; i++) same = same && fabs(gv[i] - gref[i]) <= 1e-13 * gm;
-    if (!same) atomicOr(nonuniform, 1u);
-  }
-  const double scale = adet * (coef ? coef[c] : 1.0);
-  gv[GSTRIDE - 1] = scale;
-  if (g64) {
-    double* G = (double*)Gout + c * GSTRIDE;
+      for (int i = 0; i < D * D; i++) same = same && fabs(gv[i] - s_ref[i]) <= 1e-13 * gm;
+      if (!same) atomicOr(nonuniform, 1u);
+    }
+    gv[GSTRIDE - 1] = adet * (coef ? coef[c] : 1.0);
+    if (g64) {
+      double* G = (double*)Gout + c * GSTRIDE;
 #pragma unroll
-    for (int i = 0; i < GSTRIDE; i++) G[i] = gv[i];
-  } else {
-    float* G = (float*)Gout + c * GSTRIDE;
+      for (int i = 0; i < GSTRIDE; i++) G[i] = gv[i];
+    } else {
+      float* G = (float*)Gout + c * GSTRIDE;
 #pragma unroll
-    for (int i = 0; i < GSTRIDE; i++) G[i] = (float)gv[i];
+      for (int i = 0; i < GSTRIDE; i++) G[i] = (float)gv[i];
+    }
+    if (be) {
+      const double sc = (scoef ? scoef[c] : 1.0) * adet;
+      for (int k = 0; k < bs; k++) s_sf[tid][k] = sc * fsrc[k];
+    }
   }
   if (be) {
-    int m1 = order + 1;
-    double sc = (scoef ? scoef[c] : 1.0) * adet;
-    for (int n = 0; n < nn; n++) {
-      int e0 = n % m1, e1 = (n / m1) % m1, e2 = n / (m1 * m1);
-      double w = s_m1[e0] * s_m1[e1] * (D == 3 ? s_m1[e2] : 1.0);
-      for (int k = 0; k < bs; k++) be[(c * nn + n) * bs + k] = sc * fsrc[k] * w;
+    __syncthreads();
+    const int nloc = nn * bs, cnt = (int)min((int64_t)GCELLS, ncells - c0) * nloc;
+    double* b = be + c0 * nloc;
+    for (int i = tid; i < cnt; i += GCELLS + 32) {
+      const int cl = i / nloc, r = i - cl * nloc, n = r / bs;
+      b[i] = s_sf[cl][r - n * bs] * s_w[n];
     }
   }
 }
@@ -2430,17 +2445,18 @@ template <int D, int ORDER, int BS, int FORM, int G, class T, class TA>
 __global__ void k_scatter_kron(const int64_t* __restrict__ rowptr, const int32_t* __restrict__ colind,
                                const int64_t* __restrict__ inc_ptr, const int32_t* __restrict__ inc,
                                const int32_t* __restrict__ cnd, int64_t nrows, int lmax, const T* __restrict__ Gc,
-                               T lamf, T muf, double* __restrict__ v64, float* __restrict__ v32,
+                               Tables1D tab, T lamf, T muf, double* __restrict__ v64, float* __restrict__ v32,
                                const double* __restrict__ be, double* __restrict__ bvec, const double* __restrict__ xd) {
   constexpr int M1 = ORDER + 1;
   constexpr int NN = D == 2 ? M1 * M1 : M1 * M1 * M1;
   constexpr int RPW = 32 / G;
   extern __shared__ __align__(16) unsigned char s_raw[];
   __shared__ T s_M[9], s_D[9], s_K[9];
-  if (threadIdx.x == 0) {
-    double M[9], Dm[9], Kd[9], m1[3];
-    lagrange_table_1d(ORDER, M, Dm, Kd, m1);
-    for (int i = 0; i < 9; i++) { s_M[i] = (T)M[i]; s_D[i] = (T)Dm[i]; s_K[i] = (T)Kd[i]; }
+  if (threadIdx.x < 9) {
+    const int i = threadIdx.x;
+    s_M[i] = (T)tab.M[i];
+    s_D[i] = (T)tab.Dm[i];
+    s_K[i] = (T)tab.Kd[i];
   }
   __syncthreads();
   int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -2470,7 +2486,7 @@ __global__ void k_scatter_kron(const int64_t* __restrict__ rowptr, const int32_t
     double bsum[BS];
     int64_t ib = inc_ptr[r], ie = inc_ptr[r + 1];
     if (be != nullptr) {
-      row_load_sum<BS>(ib, ie, inc, NN, be, gl, gmask, bsum);
+      row_load_sum<BS, G>(ib, ie, inc, NN, be, gl, gmask, bsum);
     } else {
 #pragma unroll
       for (int cc = 0; cc < BS; cc++) bsum[cc] = 0.0;
@@ -2535,14 +2551,15 @@ __global__ void k_scatter_kron(const int64_t* __restrict__ rowptr, const int32_t
 // k_scatter_kron (row owner, incidences in ascending cell order, load vector
 // and Dirichlet lift in the same pass).
 template <int D, int ORDER, int BS, int FORM, class T>
-__global__ void k_kref(const double* __restrict__ gref, T lamf, T muf, T* __restrict__ kref) {
+__global__ void k_kref(const double* __restrict__ gref, Tables1D tab, T lamf, T muf, T* __restrict__ kref) {
   constexpr int M1 = ORDER + 1;
   constexpr int NN = D == 2 ? M1 * M1 : M1 * M1 * M1;
   __shared__ T s_M[9], s_D[9], s_K[9];
-  if (threadIdx.x == 0) {
-    double M[9], Dm[9], Kd[9], m1[3];
-    lagrange_table_1d(ORDER, M, Dm, Kd, m1);
-    for (int i = 0; i < 9; i++) { s_M[i] = (T)M[i]; s_D[i] = (T)Dm[i]; s_K[i] = (T)Kd[i]; }
+  if (threadIdx.x < 9) {
+    const int i = threadIdx.x;
+    s_M[i] = (T)tab.M[i];
+    s_D[i] = (T)tab.Dm[i];
+    s_K[i] = (T)tab.Kd[i];
   }
   __syncthreads();
   const int ab = blockIdx.x * blockDim.x + threadIdx.x;
@@ -2602,7 +2619,7 @@ __global__ void k_scatter_uniform(const int64_t* __restrict__ rowptr, const int3
     double bsum[BS];
     const int64_t ib = inc_ptr[r], ie = inc_ptr[r + 1];
     if (be != nullptr) {
-      row_load_sum<BS>(ib, ie, inc, NN, be, gl, gmask, bsum);
+      row_load_sum<BS, G>(ib, ie, inc, NN, be, gl, gmask, bsum);
     } else {
 #pragma unroll
       for (int cc = 0; cc < BS; cc++) bsum[cc] = 0.0;
@@ -2721,7 +2738,8 @@ static int launch_uniform(Matrix* A, const double* gref, const double* coef, dou
   GT_TRY(dalloc(ctx, &kref, KREF_N));
   matrix_values_changed(A);
   T lamf = (T)(nu / ((1.0 + nu) * (1.0 - 2.0 * nu))), muf = (T)(1.0 / (2.0 * (1.0 + nu)));
-  k_kref<D, ORDER, BS, FORM, T><<<GT_KC(ctx, (NN * NN + 127) / 128), 128, 0, ctx->stream>>>(gref, lamf, muf, kref);
+  k_kref<D, ORDER, BS, FORM, T><<<GT_KC(ctx, (NN * NN + 127) / 128), 128, 0, ctx->stream>>>(gref, tables_1d(ORDER), lamf,
+                                                                                            muf, kref);
   GT_LAUNCH(ctx, "k_kref");
   const int64_t rows_per_block = (int64_t)warps * RPW;
   const int64_t nblk = (A->nbrows + rows_per_block - 1) / rows_per_block;
@@ -2772,7 +2790,7 @@ static int launch_kron(Matrix* A, const T* Gc, double nu, const double* be, doub
   int64_t grid = (A->nbrows + rows_per_block - 1) / rows_per_block;
   T lamf = (T)(nu / ((1.0 + nu) * (1.0 - 2.0 * nu))), muf = (T)(1.0 / (2.0 * (1.0 + nu)));
   kern<<<GT_KC(ctx, (unsigned)(grid > 0 ? grid : 1)), warps * 32, smem, ctx->stream>>>(
-      A->rowptr, A->colind, A->inc_ptr, A->inc, sp->cell_ndofs, A->nbrows, lmax, Gc, lamf, muf, v64, v32, be, bvec, xd);
+      A->rowptr, A->colind, A->inc_ptr, A->inc, sp->cell_ndofs, A->nbrows, lmax, Gc, tables_1d(ORDER), lamf, muf, v64, v32, be, bvec, xd);
   GT_LAUNCH(ctx, "k_scatter_kron");
   return GT_OK;
 }
@@ -2815,17 +2833,13 @@ static int kron_numeric(Matrix* A, int form, const double* coef, double nu, cons
   GT_TRY(dalloc(ctx, &gref, GSTRIDE));
   GT_CUDA(ctx, cudaMemsetAsync(flag, 0, 2 * sizeof(uint32_t), ctx->stream));
   double* gr = ctx->uniform_geom ? gref : nullptr;
-  if (ct == GT_QUAD4) {
-    if (gr) k_geom_ref<2, 4><<<GT_KC(ctx, 1), 32, 0, ctx->stream>>>(sp->mesh->coords, sp->mesh->cell_nodes, form, gr);
-    k_geom_affine<2, 4><<<GT_KC(ctx, grid_for(nc, 256)), 256, 0, ctx->stream>>>(
-        sp->mesh->coords, sp->mesh->cell_nodes, coef, form, sp->order, nc, sp->nn, sp->ncomp, Gc, g64, be, f, scoef,
-        flag, ctx->d_err, gr, flag + 1);
-  } else {
-    if (gr) k_geom_ref<3, 8><<<GT_KC(ctx, 1), 32, 0, ctx->stream>>>(sp->mesh->coords, sp->mesh->cell_nodes, form, gr);
-    k_geom_affine<3, 8><<<GT_KC(ctx, grid_for(nc, 256)), 256, 0, ctx->stream>>>(
-        sp->mesh->coords, sp->mesh->cell_nodes, coef, form, sp->order, nc, sp->nn, sp->ncomp, Gc, g64, be, f, scoef,
-        flag, ctx->d_err, gr, flag + 1);
-  }
+  auto geom = [&](auto kern) {
+    kern<<<GT_KC(ctx, grid_for(nc, GCELLS)), GCELLS + 32, 0, ctx->stream>>>(
+        sp->mesh->coords, sp->mesh->cell_nodes, coef, form, sp->order, tables_1d(sp->order), nc, sp->nn, sp->ncomp, Gc,
+        g64, be, f, scoef, flag, ctx->d_err, gr, flag + 1);
+  };
+  if (ct == GT_QUAD4) geom(k_geom_affine<2, 4>);
+  else geom(k_geom_affine<3, 8>);
   GT_LAUNCH(ctx, "k_geom_affine");
   GT_CUDA(ctx, cudaMemcpyAsync(&ctx->h_scratch[2], flag, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
   GT_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
