@@ -105,19 +105,20 @@ __global__ void k_corner_first(const int32_t* corners, int64_t nc, int32_t* firs
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i < nc) atomicMin(&first[corners[i]], (int32_t)i);
 }
-__global__ void k_corner_flags(const int32_t* corners, int64_t nc, const int32_t* first, int32_t* flag) {
-  int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i < nc) flag[i] = first[corners[i]] == (int32_t)i;
+// cflag: corner i is the first to name its node; nflag: node i is no corner
+__global__ void k_vertex_flags(const int32_t* corners, int64_t nc, const int32_t* first, int64_t nnodes, int32_t* cflag,
+                               int32_t* nflag) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < max(nc, nnodes); i += (int64_t)gridDim.x * blockDim.x) {
+    if (i < nc) cflag[i] = first[corners[i]] == (int32_t)i;
+    if (i < nnodes) nflag[i] = first[i] == INT_MAX;
+  }
 }
-__global__ void k_noncorner_flags(const int32_t* first, int64_t nnodes, int32_t* flag) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nnodes; i += (int64_t)gridDim.x * blockDim.x)
-    flag[i] = first[i] == INT_MAX;
-}
-__global__ void k_vertex_ids(const int32_t* corners, int64_t nc, const int32_t* first, const int32_t* cpos,
-                             const int32_t* npos, int32_t ncu, int64_t nnodes, int32_t* node_vertex) {
+// ncu: the number of distinct corners
+__global__ void k_vertex_ids(const int32_t* first, const int32_t* cpos, const int32_t* npos, const int32_t* ncu,
+                             int64_t nnodes, int32_t* node_vertex) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nnodes; i += (int64_t)gridDim.x * blockDim.x) {
     int32_t f = first[i];
-    node_vertex[i] = f == INT_MAX ? ncu + npos[i] : cpos[f];
+    node_vertex[i] = f == INT_MAX ? *ncu + npos[i] : cpos[f];
   }
 }
 
@@ -147,43 +148,48 @@ __global__ void k_insert_instances(Hash h, const int32_t* fverts, int64_t nf, in
   for (int i = 0; i < ndv; i++) v[i] = fverts[f * nlv + ld.v[l][i]];
   int64_t s = hash_insert(h, face_key(v, ndv, err), err);
   inst_slot[r] = s;
-  if (s >= 0) atomicMin(&h.rank[s], (int32_t)r);
+  if (s >= 0) atomicMin(reinterpret_cast<unsigned*>(&h.rank[s]), (unsigned)r);
 }
-__global__ void k_first_flags(Hash h, int32_t* flag) {
-  for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < h.cap; s += (int64_t)gridDim.x * blockDim.x)
-    if (h.keys[s] != EMPTY_KEY && h.vals[s] == 0 && h.rank[s] != INT_MAX) flag[h.rank[s]] = 1;
+// The id of a face from its slot: a parent's own, else the position of the
+// instance that first met it among all such instances
+__device__ __forceinline__ int32_t slot_id(const Hash& h, int64_t s, const int32_t* __restrict__ pos, int32_t npar) {
+  const int32_t v = h.vals[s];
+  return v > 0 ? v : npar + pos[h.rank[s]] + 1;
 }
-__global__ void k_assign_new(Hash h, const int32_t* pos, int32_t npar) {
-  for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < h.cap; s += (int64_t)gridDim.x * blockDim.x)
-    if (h.keys[s] != EMPTY_KEY && h.vals[s] == 0 && h.rank[s] != INT_MAX) h.vals[s] = npar + pos[h.rank[s]] + 1;
+__global__ void k_first_flags(Hash h, const int64_t* __restrict__ inst_slot, int64_t n, int32_t* __restrict__ flag) {
+  const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (r >= n) return;
+  const int64_t s = inst_slot[r];
+  flag[r] = s >= 0 && h.vals[s] < 0 && h.rank[s] == (int32_t)r;
 }
-__global__ void k_instance_ids(Hash h, const int64_t* inst_slot, int64_t n, int32_t* out, uint32_t* err) {
-  for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) {
-    int64_t s = inst_slot[r];
-    out[r] = s >= 0 ? h.vals[s] : 0;
-    if (s < 0) atomicOr(err, DEV_ERR_LOOKUP);
+// ids of the instances; vertices of every d-face (dverts, optional): parents
+// from their own list, new ones from the instance that first met them
+// (generate_face_vertices, topology.jl:1468-1540).  One pass over the
+// instances: on 31^3 hexahedra sweeps over the hash table's slots, two to
+// four times as many, took 97 us in all where this and k_first_flags take 36.
+__global__ void k_face_ids(Hash h, const int64_t* __restrict__ inst_slot, int64_t n, const int32_t* __restrict__ pos,
+                           int32_t npar, const int32_t* __restrict__ fverts, int nlv, int nld, int ndv, LocalFaces ld,
+                           const int32_t* __restrict__ pverts, int32_t* __restrict__ out, int32_t* __restrict__ dverts,
+                           uint32_t* err) {
+  const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (dverts && r < (int64_t)npar * ndv) dverts[r] = pverts[r];
+  if (r >= n) return;
+  const int64_t s = inst_slot[r];
+  if (s < 0) {
+    atomicOr(err, DEV_ERR_LOOKUP);
+    out[r] = 0;
+    return;
   }
-}
-// vertices of every d-face: parents from their own list, new ones from the
-// instance that first met them (generate_face_vertices, topology.jl:1468-1540)
-__global__ void k_face_verts_parent(const int32_t* pverts, int64_t npar, int ndv, int32_t* dverts) {
-  int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i < npar * ndv) dverts[i] = pverts[i];
-}
-__global__ void k_face_verts_new(Hash h, int32_t npar, const int32_t* fverts, int nlv, int nld, int ndv,
-                                 LocalFaces ld, int32_t* dverts) {
-  for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < h.cap; s += (int64_t)gridDim.x * blockDim.x) {
-    if (h.keys[s] == EMPTY_KEY) continue;
-    int32_t id = h.vals[s];
-    if (id <= npar) continue;
-    int64_t r = h.rank[s];
-    int64_t f = r / nld;
-    int l = (int)(r - f * nld);
+  const int32_t id = slot_id(h, s, pos, npar);
+  out[r] = id;
+  if (dverts && h.vals[s] < 0 && h.rank[s] == (int32_t)r) {
+    const int64_t f = r / nld;
+    const int l = (int)(r - f * nld);
     for (int i = 0; i < ndv; i++) dverts[(int64_t)(id - 1) * ndv + i] = fverts[f * nlv + ld.v[l][i]];
   }
 }
-__global__ void k_lookup_instances(Hash h, const int32_t* fverts, int64_t nf, int nlv, int nld, int ndv, LocalFaces ld,
-                                   int32_t* out, uint32_t* err) {
+__global__ void k_lookup_instances(Hash h, const int32_t* __restrict__ pos, int32_t npar, const int32_t* fverts,
+                                   int64_t nf, int nlv, int nld, int ndv, LocalFaces ld, int32_t* out, uint32_t* err) {
   int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (r >= nf * nld) return;
   int64_t f = r / nld;
@@ -191,98 +197,95 @@ __global__ void k_lookup_instances(Hash h, const int32_t* fverts, int64_t nf, in
   int32_t v[4];
   for (int i = 0; i < ndv; i++) v[i] = fverts[f * nlv + ld.v[l][i]];
   int64_t s = hash_find(h, face_key(v, ndv, err));
-  if (s < 0) { atomicOr(err, DEV_ERR_LOOKUP); out[r] = 0; } else out[r] = h.vals[s];
+  if (s < 0) { atomicOr(err, DEV_ERR_LOOKUP); out[r] = 0; } else out[r] = slot_id(h, s, pos, npar);
 }
 
+// keys, vals and rank in one block, empty after one memset: keys EMPTY_KEY,
+// vals -1 (no parent), rank the largest unsigned
 struct HashBuf {
   Hash h{};
   int alloc(Ctx* ctx, int64_t nkeys) {
     int64_t cap = 1024;
     while (cap < 2 * nkeys) cap <<= 1;
     h.cap = cap;
-    GT_TRY(dalloc(ctx, &h.keys, cap));
-    GT_TRY(dalloc(ctx, &h.vals, cap));
-    GT_TRY(dalloc(ctx, &h.rank, cap));
-    GT_CUDA(ctx, cudaMemsetAsync(h.keys, 0xFF, sizeof(unsigned long long) * cap, ctx->stream));
-    GT_CUDA(ctx, cudaMemsetAsync(h.vals, 0, sizeof(int32_t) * cap, ctx->stream));
-    k_fill_i32<<<GT_KC(ctx, grid_for(cap, 256)), 256, 0, ctx->stream>>>(h.rank, cap, INT_MAX);
-    GT_LAUNCH(ctx, "k_fill_i32");
+    static_assert(EMPTY_KEY == ~0ull, "the memset below");
+    GT_TRY(dalloc(ctx, &h.keys, 2 * cap));
+    h.vals = reinterpret_cast<int32_t*>(h.keys + cap);
+    h.rank = h.vals + cap;
+    GT_CUDA(ctx, cudaMemsetAsync(h.keys, 0xFF, 2 * sizeof(unsigned long long) * cap, ctx->stream));
     return GT_OK;
   }
+  void release(Ctx* ctx) { dfree(ctx, h.keys); }
+};
+
+// The d-faces of a numbering (number_faces): their table, the positions of
+// the instances that first met one, and the parents' count -- what the id of
+// any face follows from (slot_id)
+struct FaceNumbers {
+  HashBuf hb;
+  int32_t* pos = nullptr;
+  int32_t npar = 0;
+  int64_t nd = 0;
   void release(Ctx* ctx) {
-    dfree(ctx, h.keys);
-    dfree(ctx, h.vals);
-    dfree(ctx, h.rank);
+    hb.release(ctx);
+    dfree(ctx, pos);
   }
 };
 
 // Numbers the d-faces of nf higher-dimensional faces (see file header).
-// Outputs inst_ids[nf*nld] (1-based) and, if dverts != NULL, the vertices of
-// every d-face (capacity npar + nf*nld faces).  Returns the count in *nd.
+// Outputs inst_ids[nf*nld] (1-based) and, if dverts_out, the vertices of every
+// d-face; F->nd is their count.  The caller releases F.
 static int number_faces(Ctx* ctx, const int32_t* fverts, int64_t nf, int nlv, int nld, int ndv, const LocalFaces& ld,
-                        const int32_t* pverts, int64_t npar, int32_t* inst_ids, int32_t** dverts_out, int64_t* nd) {
-  HashBuf hb;
+                        const int32_t* pverts, int64_t npar, int32_t* inst_ids, int32_t** dverts_out, FaceNumbers* F) {
   int64_t ninst = nf * nld;
-  int s = hb.alloc(ctx, npar + ninst);
+  int s = F->hb.alloc(ctx, npar + ninst);
+  const Hash h = F->hb.h;
+  F->npar = (int32_t)npar;
   int64_t* inst_slot = nullptr;
-  int32_t *flag = nullptr, *pos = nullptr;
+  int32_t* flag = nullptr;
+  cudaStream_t st = ctx->stream;
   if (s == GT_OK) s = dalloc(ctx, &inst_slot, ninst);
   if (s == GT_OK) s = dalloc(ctx, &flag, ninst);
-  if (s == GT_OK) s = dalloc(ctx, &pos, ninst + 1);
+  if (s == GT_OK) s = dalloc(ctx, &F->pos, ninst + 1);
   if (s == GT_OK) {
-    cudaStream_t st = ctx->stream;
-    cudaMemsetAsync(flag, 0, sizeof(int32_t) * ninst, st);
-    if (npar > 0) k_insert_parents<<<GT_KC(ctx, grid_for(npar, 256)), 256, 0, st>>>(hb.h, pverts, npar, ndv, ctx->d_err);
-    k_insert_instances<<<GT_KC(ctx, grid_for(ninst, 256)), 256, 0, st>>>(hb.h, fverts, nf, nlv, nld, ndv, ld, inst_slot, ctx->d_err);
-    k_first_flags<<<GT_KC(ctx, grid_for(hb.h.cap, 256)), 256, 0, st>>>(hb.h, flag);
+    if (npar > 0) k_insert_parents<<<GT_KC(ctx, grid_for(npar, 256)), 256, 0, st>>>(h, pverts, npar, ndv, ctx->d_err);
+    k_insert_instances<<<GT_KC(ctx, grid_for(ninst, 256)), 256, 0, st>>>(h, fverts, nf, nlv, nld, ndv, ld, inst_slot, ctx->d_err);
+    k_first_flags<<<GT_KC(ctx, grid_for(ninst, 256)), 256, 0, st>>>(h, inst_slot, ninst, flag);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) s = check_cuda(ctx, e, "face numbering");
   }
-  if (s == GT_OK) s = exclusive_scan_i32(ctx, flag, pos, ninst);
-  if (s == GT_OK) {
-    cudaStream_t st = ctx->stream;
-    k_assign_new<<<GT_KC(ctx, grid_for(hb.h.cap, 256)), 256, 0, st>>>(hb.h, pos, (int32_t)npar);
-    k_instance_ids<<<GT_KC(ctx, grid_for(ninst, 256)), 256, 0, st>>>(hb.h, inst_slot, ninst, inst_ids, ctx->d_err);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) s = check_cuda(ctx, e, "face ids");
-  }
+  if (s == GT_OK) s = exclusive_scan_i32(ctx, flag, F->pos, ninst);
   if (s == GT_OK) {
     int32_t nnew = 0;
-    cudaMemcpyAsync(&ctx->h_scratch[0], pos + ninst, sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream);
-    cudaStreamSynchronize(ctx->stream);
+    cudaMemcpyAsync(&ctx->h_scratch[0], F->pos + ninst, sizeof(int32_t), cudaMemcpyDeviceToHost, st);
+    cudaStreamSynchronize(st);
     memcpy(&nnew, &ctx->h_scratch[0], sizeof(int32_t));
-    *nd = npar + nnew;
+    F->nd = npar + nnew;
+    int32_t* dv = nullptr;
     if (dverts_out) {
-      int32_t* dv = nullptr;
-      s = dalloc(ctx, &dv, (*nd) * ndv);
-      if (s == GT_OK) {
-        cudaStream_t st = ctx->stream;
-        if (npar > 0) k_face_verts_parent<<<GT_KC(ctx, grid_for(npar * ndv, 256)), 256, 0, st>>>(pverts, npar, ndv, dv);
-        k_face_verts_new<<<GT_KC(ctx, grid_for(hb.h.cap, 256)), 256, 0, st>>>(hb.h, (int32_t)npar, fverts, nlv, nld, ndv, ld, dv);
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) s = check_cuda(ctx, e, "face vertices");
-        *dverts_out = dv;
-      }
+      s = dalloc(ctx, &dv, F->nd * ndv);
+      *dverts_out = dv;
+    }
+    if (s == GT_OK) {
+      const int64_t items = std::max<int64_t>(ninst, dv ? npar * ndv : 0);
+      k_face_ids<<<GT_KC(ctx, grid_for(items, 256)), 256, 0, st>>>(h, inst_slot, ninst, F->pos, F->npar, fverts, nlv, nld,
+                                                                   ndv, ld, pverts, inst_ids, dv, ctx->d_err);
+      cudaError_t e = cudaGetLastError();
+      if (e != cudaSuccess) s = check_cuda(ctx, e, "face ids");
     }
   }
   dfree(ctx, inst_slot);
   dfree(ctx, flag);
-  dfree(ctx, pos);
-  hb.release(ctx);
   return s;
 }
 
-// lookup of existing d-faces (fill_face_boundary_mesh_topology!,
+// lookup of numbered d-faces (fill_face_boundary_mesh_topology!,
 // src/topology.jl:515-591)
-static int lookup_faces(Ctx* ctx, const int32_t* dverts, int64_t nd, int ndv, const int32_t* fverts, int64_t nf,
-                        int nlv, int nld, const LocalFaces& ld, int32_t* out) {
-  HashBuf hb;
-  GT_TRY(hb.alloc(ctx, nd));
-  cudaStream_t st = ctx->stream;
-  k_insert_parents<<<GT_KC(ctx, grid_for(nd, 256)), 256, 0, st>>>(hb.h, dverts, nd, ndv, ctx->d_err);
-  k_lookup_instances<<<GT_KC(ctx, grid_for(nf * nld, 256)), 256, 0, st>>>(hb.h, fverts, nf, nlv, nld, ndv, ld, out, ctx->d_err);
+static int lookup_faces(Ctx* ctx, const FaceNumbers& F, int ndv, const int32_t* fverts, int64_t nf, int nlv, int nld,
+                        const LocalFaces& ld, int32_t* out) {
+  k_lookup_instances<<<GT_KC(ctx, grid_for(nf * nld, 256)), 256, 0, ctx->stream>>>(F.hb.h, F.pos, F.npar, fverts, nf, nlv,
+                                                                                   nld, ndv, ld, out, ctx->d_err);
   cudaError_t e = cudaGetLastError();
-  hb.release(ctx);
   if (e != cudaSuccess) return check_cuda(ctx, e, "face lookup");
   return GT_OK;
 }
@@ -312,26 +315,23 @@ __global__ void k_cell_node_dofs(RefTables t, int order, int64_t nc, const int32
   }
 }
 
-// tag the closure nodes of tagged local (D-1)-faces (step_2, src/space.jl:487-508)
-__global__ void k_tag_dirichlet(Hash tagged, RefTables t, int64_t nc, const int32_t* cverts, const int32_t* cnd,
-                                int32_t* tag, uint32_t* err) {
+// tag the closure nodes of tagged local (D-1)-faces (step_2, src/space.jl:487-508):
+// cfid: the ids of the cells' local faces, tagged by id
+__global__ void k_tag_dirichlet(const int32_t* __restrict__ tagged, int32_t nb, const int32_t* __restrict__ cfid,
+                                RefTables t, int64_t nc, const int32_t* __restrict__ cnd, int32_t* tag) {
   int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (r >= nc * t.nlf) return;
+  const int32_t id = cfid[r];
+  if (id < 1 || id > nb || !tagged[id - 1]) return;  // only parents are tagged
   int64_t c = r / t.nlf;
   int f = (int)(r - c * t.nlf);
-  int32_t v[4];
-  for (int i = 0; i < t.nlfv; i++) v[i] = cverts[c * t.nlv + t.lf_verts[f][i]];
-  if (hash_find(tagged, face_key(v, t.nlfv, err)) < 0) return;
   for (int i = 0; i < t.nclosure; i++) tag[cnd[c * t.nn + t.closure[f][i]] - 1] = 1;
 }
-__global__ void k_free_flags(const int32_t* tag, int64_t n, int32_t* freef) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    freef[i] = 1 - tag[i];
-}
-__global__ void k_renumber(int32_t* cnd, int64_t n, const int32_t* tag, const int32_t* fpos, const int32_t* dpos) {
+// dpos: Dirichlet nodes before a node (the free ones are the others)
+__global__ void k_renumber(int32_t* cnd, int64_t n, const int32_t* tag, const int32_t* dpos) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     int32_t g = cnd[i] - 1;
-    cnd[i] = tag[g] ? -(dpos[g] + 1) : fpos[g] + 1;
+    cnd[i] = tag[g] ? -(dpos[g] + 1) : g - dpos[g] + 1;
   }
 }
 __global__ void k_select_faces(const int32_t* bfaces, const int32_t* bgroup, int64_t nb, int nbfv, const int32_t* node_vertex,
@@ -346,10 +346,13 @@ __global__ void k_select_faces(const int32_t* bfaces, const int32_t* bgroup, int
   keep[i] = k;
   for (int j = 0; j < nbfv; j++) out_verts[i * nbfv + j] = k ? node_vertex[bfaces[i * nbfv + j]] + 1 : 0;
 }
-__global__ void k_insert_tagged(Hash h, const int32_t* verts, const int32_t* keep, int64_t nb, int ndv, uint32_t* err) {
+// the selected boundary faces' ids (a face listed twice has one)
+__global__ void k_mark_tagged(Hash h, const int32_t* verts, const int32_t* keep, int64_t nb, int ndv, int32_t* tagged,
+                              uint32_t* err) {
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= nb || !keep[i]) return;
-  hash_insert(h, face_key(verts + i * ndv, ndv, err), err);
+  const int64_t s = hash_find(h, face_key(verts + i * ndv, ndv, err));
+  if (s >= 0 && h.vals[s] > 0) tagged[h.vals[s] - 1] = 1;
 }
 __global__ void k_tag_vertices(const int32_t* sel, int64_t n, int32_t* tag) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
@@ -409,19 +412,14 @@ int number_dofs(Space* sp, int ngroups, const int32_t* groups_host) {
   GT_TRY(dalloc(ctx, &npos, nn_ + 1));
   GT_TRY(dalloc(ctx, &node_vertex, nn_));
   k_fill_i32<<<GT_KC(ctx, grid_for(nn_, 256)), 256, 0, st>>>(first, nn_, INT_MAX);
-  if (M->ncorners > 0) {
+  if (M->ncorners > 0)
     k_corner_first<<<GT_KC(ctx, grid_for(M->ncorners, 256)), 256, 0, st>>>(M->corners, M->ncorners, first);
-    k_corner_flags<<<GT_KC(ctx, grid_for(M->ncorners, 256)), 256, 0, st>>>(M->corners, M->ncorners, first, cflag);
-  }
-  k_noncorner_flags<<<GT_KC(ctx, grid_for(nn_, 256)), 256, 0, st>>>(first, nn_, nflag);
+  k_vertex_flags<<<GT_KC(ctx, grid_for(std::max(nn_, M->ncorners), 256)), 256, 0, st>>>(M->corners, M->ncorners, first, nn_,
+                                                                                       cflag, nflag);
   GT_LAUNCH(ctx, "vertex flags");
   GT_TRY(exclusive_scan_i32(ctx, cflag, cpos, M->ncorners));
   GT_TRY(exclusive_scan_i32(ctx, nflag, npos, nn_));
-  GT_CUDA(ctx, cudaMemcpyAsync(&ctx->h_scratch[0], cpos + M->ncorners, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-  GT_CUDA(ctx, cudaStreamSynchronize(st));
-  int32_t ncu = 0;
-  memcpy(&ncu, &ctx->h_scratch[0], sizeof(int32_t));
-  k_vertex_ids<<<GT_KC(ctx, grid_for(nn_, 256)), 256, 0, st>>>(M->corners, M->ncorners, first, cpos, npos, ncu, nn_, node_vertex);
+  k_vertex_ids<<<GT_KC(ctx, grid_for(nn_, 256)), 256, 0, st>>>(first, cpos, npos, cpos + M->ncorners, nn_, node_vertex);
   GT_LAUNCH(ctx, "k_vertex_ids");
   int64_t nverts = nn_;
   dfree(ctx, first);
@@ -437,6 +435,7 @@ int number_dofs(Space* sp, int ngroups, const int32_t* groups_host) {
   // ---- edges / faces (Q2)
   int32_t *cedges = nullptr, *cfaces = nullptr;
   int64_t nedges = 0, nfaces = 0;
+  FaceNumbers FN, EN;  // 2-faces, edges
   if (sp->order == 2) {
     LocalFaces lq{}, lh{}, le{};
     if (t.D == 2) {
@@ -446,7 +445,7 @@ int number_dofs(Space* sp, int ngroups, const int32_t* groups_host) {
       k_map_vertices<<<GT_KC(ctx, grid_for(M->nbfaces * 2, 256)), 256, 0, st>>>(M->bfaces, M->nbfaces * 2, node_vertex, pv);
       GT_LAUNCH(ctx, "k_map_vertices");
       GT_TRY(dalloc(ctx, &cedges, nc * 4));
-      s = number_faces(ctx, cverts, nc, 4, 4, 2, lq, pv, M->nbfaces, cedges, nullptr, &nedges);
+      s = number_faces(ctx, cverts, nc, 4, 4, 2, lq, pv, M->nbfaces, cedges, nullptr, &EN);
       dfree(ctx, pv);
       GT_TRY(s);
     } else if (M->ctype == GT_TET4) {
@@ -460,7 +459,7 @@ int number_dofs(Space* sp, int ngroups, const int32_t* groups_host) {
       static const int TRE[3][2] = {{0, 1}, {0, 2}, {1, 2}};  // edges of the unit triangle, src/domain.jl:413-424
       for (int e = 0; e < 3; e++) { ltri.v[e][0] = TRE[e][0]; ltri.v[e][1] = TRE[e][1]; }
       for (int e = 0; e < 6; e++) { lte.v[e][0] = t.le_verts[e][0]; lte.v[e][1] = t.le_verts[e][1]; }
-      int32_t *pf = nullptr, *pe = nullptr, *fverts = nullptr, *fedges = nullptr, *everts = nullptr;
+      int32_t *pf = nullptr, *pe = nullptr, *fverts = nullptr, *fedges = nullptr;
       GT_TRY(dalloc(ctx, &pf, M->nbfaces * 3 + 1));
       GT_TRY(dalloc(ctx, &pe, M->nbedges * 2 + 1));
       if (M->nbfaces > 0)
@@ -469,23 +468,22 @@ int number_dofs(Space* sp, int ngroups, const int32_t* groups_host) {
         k_map_vertices<<<GT_KC(ctx, grid_for(M->nbedges * 2, 256)), 256, 0, st>>>(M->bedges, M->nbedges * 2, node_vertex, pe);
       GT_LAUNCH(ctx, "k_map_vertices");
       GT_TRY(dalloc(ctx, &cfaces, nc * 4));
-      GT_TRY(number_faces(ctx, cverts, nc, 4, 4, 3, ltf, pf, M->nbfaces, cfaces, &fverts, &nfaces));
-      GT_TRY(dalloc(ctx, &fedges, nfaces * 3));
-      GT_TRY(number_faces(ctx, fverts, nfaces, 3, 3, 2, ltri, pe, M->nbedges, fedges, &everts, &nedges));
+      GT_TRY(number_faces(ctx, cverts, nc, 4, 4, 3, ltf, pf, M->nbfaces, cfaces, &fverts, &FN));
+      GT_TRY(dalloc(ctx, &fedges, FN.nd * 3));
+      GT_TRY(number_faces(ctx, fverts, FN.nd, 3, 3, 2, ltri, pe, M->nbedges, fedges, nullptr, &EN));
       GT_TRY(dalloc(ctx, &cedges, nc * 6));
-      GT_TRY(lookup_faces(ctx, everts, nedges, 2, cverts, nc, 4, 6, lte, cedges));
+      GT_TRY(lookup_faces(ctx, EN, 2, cverts, nc, 4, 6, lte, cedges));
       dfree(ctx, pf);
       dfree(ctx, pe);
       dfree(ctx, fverts);
       dfree(ctx, fedges);
-      dfree(ctx, everts);
     } else {
       for (int f = 0; f < 6; f++)
         for (int i = 0; i < 4; i++) lh.v[f][i] = t.lf_verts[f][i];
       static const int QE[4][2] = {{0, 1}, {2, 3}, {0, 2}, {1, 3}};
       for (int e = 0; e < 4; e++) { lq.v[e][0] = QE[e][0]; lq.v[e][1] = QE[e][1]; }
       for (int e = 0; e < 12; e++) { le.v[e][0] = t.le_verts[e][0]; le.v[e][1] = t.le_verts[e][1]; }
-      int32_t *pf = nullptr, *pe = nullptr, *fverts = nullptr, *fedges = nullptr, *everts = nullptr;
+      int32_t *pf = nullptr, *pe = nullptr, *fverts = nullptr, *fedges = nullptr;
       GT_TRY(dalloc(ctx, &pf, M->nbfaces * 4));
       GT_TRY(dalloc(ctx, &pe, M->nbedges * 2 + 1));
       k_map_vertices<<<GT_KC(ctx, grid_for(M->nbfaces * 4, 256)), 256, 0, st>>>(M->bfaces, M->nbfaces * 4, node_vertex, pf);
@@ -493,18 +491,19 @@ int number_dofs(Space* sp, int ngroups, const int32_t* groups_host) {
         k_map_vertices<<<GT_KC(ctx, grid_for(M->nbedges * 2, 256)), 256, 0, st>>>(M->bedges, M->nbedges * 2, node_vertex, pe);
       GT_LAUNCH(ctx, "k_map_vertices");
       GT_TRY(dalloc(ctx, &cfaces, nc * 6));
-      GT_TRY(number_faces(ctx, cverts, nc, 8, 6, 4, lh, pf, M->nbfaces, cfaces, &fverts, &nfaces));
-      GT_TRY(dalloc(ctx, &fedges, nfaces * 4));
-      GT_TRY(number_faces(ctx, fverts, nfaces, 4, 4, 2, lq, pe, M->nbedges, fedges, &everts, &nedges));
+      GT_TRY(number_faces(ctx, cverts, nc, 8, 6, 4, lh, pf, M->nbfaces, cfaces, &fverts, &FN));
+      GT_TRY(dalloc(ctx, &fedges, FN.nd * 4));
+      GT_TRY(number_faces(ctx, fverts, FN.nd, 4, 4, 2, lq, pe, M->nbedges, fedges, nullptr, &EN));
       GT_TRY(dalloc(ctx, &cedges, nc * 12));
-      GT_TRY(lookup_faces(ctx, everts, nedges, 2, cverts, nc, 8, 12, le, cedges));
+      GT_TRY(lookup_faces(ctx, EN, 2, cverts, nc, 8, 12, le, cedges));
       dfree(ctx, pf);
       dfree(ctx, pe);
       dfree(ctx, fverts);
       dfree(ctx, fedges);
-      dfree(ctx, everts);
     }
   }
+  nedges = EN.nd;
+  nfaces = FN.nd;
   // ---- node dofs before the split
   // node dofs: vertices, then (order 2) edges, 2-faces and cells that own a node
   if (!t.face_nodes) nfaces = 0;
@@ -514,7 +513,7 @@ int number_dofs(Space* sp, int ngroups, const int32_t* groups_host) {
                                                        sp->cell_ndofs);
   GT_LAUNCH(ctx, "k_cell_node_dofs");
   // ---- Dirichlet tags
-  int32_t *tag = nullptr, *freef = nullptr, *fpos = nullptr, *dpos = nullptr;
+  int32_t *tag = nullptr, *dpos = nullptr;
   GT_TRY(dalloc(ctx, &tag, nnodes_sp));
   GT_CUDA(ctx, cudaMemsetAsync(tag, 0, sizeof(int32_t) * nnodes_sp, st));
   if (ngroups != 0 && M->nbfaces > 0) {
@@ -533,27 +532,29 @@ int number_dofs(Space* sp, int ngroups, const int32_t* groups_host) {
       k_tag_vertices<<<GT_KC(ctx, grid_for(M->nbfaces * M->nbfv, 256)), 256, 0, st>>>(sel, M->nbfaces * M->nbfv, tag);
       GT_LAUNCH(ctx, "k_tag_vertices");
     } else {
-      HashBuf hb;
-      GT_TRY(hb.alloc(ctx, M->nbfaces));
-      k_insert_tagged<<<GT_KC(ctx, grid_for(M->nbfaces, 256)), 256, 0, st>>>(hb.h, sel, keep, M->nbfaces, M->nbfv, ctx->d_err);
-      k_tag_dirichlet<<<GT_KC(ctx, grid_for(nc * t.nlf, 256)), 256, 0, st>>>(hb.h, t, nc, cverts, sp->cell_ndofs, tag, ctx->d_err);
+      // boundary faces are the numbering's parents (edges in 2-D)
+      const FaceNumbers& BF = t.D == 2 ? EN : FN;
+      int32_t* tagged = nullptr;
+      GT_TRY(dalloc(ctx, &tagged, M->nbfaces));
+      GT_CUDA(ctx, cudaMemsetAsync(tagged, 0, sizeof(int32_t) * M->nbfaces, st));
+      k_mark_tagged<<<GT_KC(ctx, grid_for(M->nbfaces, 256)), 256, 0, st>>>(BF.hb.h, sel, keep, M->nbfaces, M->nbfv, tagged,
+                                                                           ctx->d_err);
+      k_tag_dirichlet<<<GT_KC(ctx, grid_for(nc * t.nlf, 256)), 256, 0, st>>>(tagged, (int32_t)M->nbfaces,
+                                                                             t.D == 2 ? cedges : cfaces, t, nc,
+                                                                             sp->cell_ndofs, tag);
       GT_LAUNCH(ctx, "k_tag_dirichlet");
-      hb.release(ctx);
+      dfree(ctx, tagged);
     }
     dfree(ctx, sel);
     dfree(ctx, keep);
     dfree(ctx, dgroups);
   }
-  GT_TRY(dalloc(ctx, &freef, nnodes_sp));
-  GT_TRY(dalloc(ctx, &fpos, nnodes_sp + 1));
+  FN.release(ctx);
+  EN.release(ctx);
   GT_TRY(dalloc(ctx, &dpos, nnodes_sp + 1));
-  k_free_flags<<<GT_KC(ctx, grid_for(nnodes_sp, 256)), 256, 0, st>>>(tag, nnodes_sp, freef);
-  GT_LAUNCH(ctx, "k_free_flags");
-  GT_TRY(exclusive_scan_i32(ctx, freef, fpos, nnodes_sp));
   GT_TRY(exclusive_scan_i32(ctx, tag, dpos, nnodes_sp));
-  k_renumber<<<GT_KC(ctx, grid_for(nc * t.nn, 256)), 256, 0, st>>>(sp->cell_ndofs, nc * t.nn, tag, fpos, dpos);
+  k_renumber<<<GT_KC(ctx, grid_for(nc * t.nn, 256)), 256, 0, st>>>(sp->cell_ndofs, nc * t.nn, tag, dpos);
   GT_LAUNCH(ctx, "k_renumber");
-  GT_CUDA(ctx, cudaMemcpyAsync(&ctx->h_scratch[0], fpos + nnodes_sp, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
   GT_CUDA(ctx, cudaMemcpyAsync(&ctx->h_scratch[1], dpos + nnodes_sp, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
   int32_t* dspread = nullptr;
   GT_TRY(dalloc(ctx, &dspread, 1));
@@ -564,16 +565,13 @@ int number_dofs(Space* sp, int ngroups, const int32_t* groups_host) {
   const int ds = device_error_status(ctx, "lagrange_space");  // synchronises
   dfree(ctx, dspread);
   GT_TRY(ds);
-  int32_t nf = 0, ndr = 0, spread = 0;
-  memcpy(&nf, &ctx->h_scratch[0], sizeof(int32_t));
+  int32_t ndr = 0, spread = 0;
   memcpy(&ndr, &ctx->h_scratch[1], sizeof(int32_t));
   memcpy(&spread, &ctx->h_scratch[2], sizeof(int32_t));
-  sp->nfree_nodes = nf;
+  sp->nfree_nodes = nnodes_sp - ndr;
   sp->ndiri_nodes = ndr;
   sp->dof_spread = spread;
   dfree(ctx, tag);
-  dfree(ctx, freef);
-  dfree(ctx, fpos);
   dfree(ctx, dpos);
   dfree(ctx, cverts);
   dfree(ctx, cedges);
@@ -877,11 +875,16 @@ int gt_space_cell_dofs(const gt_space* sp, int32_t* out) {
   if (!sp || !out) return GT_ERR_INVALID;
   Ctx* ctx = sp->mesh->ctx;
   int64_t n = sp->mesh->ncells * sp->nloc;
+  // a device output is written in place, a host one through a staging block
+  cudaPointerAttributes at{};
+  const bool here = cudaPointerGetAttributes(&at, out) == cudaSuccess && at.type == cudaMemoryTypeDevice && at.device == ctx->device;
+  cudaGetLastError();
   int32_t* tmp = nullptr;
-  GT_TRY(dalloc(ctx, &tmp, n));
-  k_expand_cell_dofs<<<GT_KC(ctx, grid_for(n, 256)), 256, 0, ctx->stream>>>(sp->cell_ndofs, sp->mesh->ncells, sp->nn, sp->ncomp, tmp);
+  if (!here) GT_TRY(dalloc(ctx, &tmp, n));
+  k_expand_cell_dofs<<<GT_KC(ctx, grid_for(n, 256)), 256, 0, ctx->stream>>>(sp->cell_ndofs, sp->mesh->ncells, sp->nn, sp->ncomp,
+                                                                            here ? out : tmp);
   GT_LAUNCH(ctx, "k_expand_cell_dofs");
-  int s = copy_out(ctx, out, tmp, n);
+  int s = here ? GT_OK : copy_out(ctx, out, tmp, n);
   if (s == GT_OK) {
     cudaError_t e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) s = check_cuda(ctx, e, "gt_space_cell_dofs");
