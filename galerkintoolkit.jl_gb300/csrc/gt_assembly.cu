@@ -203,6 +203,15 @@ static int get_tab(Ctx* ctx, int ctype, int order, double** tab, TabLayout* L) {
   return GT_OK;
 }
 
+// Lets a kernel be launched with any dynamic shared memory these launches use
+// (at most 210 KB).  A constant, not the launch's own size: the attribute is
+// the process's, and another thread may launch the same kernel with another
+// size in between.
+template <class K>
+static cudaError_t dynamic_smem(K kern) {
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 210 * 1024);
+}
+
 // ---------------------------------------------------------------------------
 // 1. incidence
 // ---------------------------------------------------------------------------
@@ -325,7 +334,7 @@ int build_incidence_arr(Ctx* ctx, const int32_t* dofs, int64_t n, int64_t nrows,
     if (icap > 4096) return set_error(ctx, GT_ERR_UNSUPPORTED, "a DOF touches too many cells");
     int warps = 8;
     size_t smem = (size_t)warps * icap * sizeof(int32_t);
-    if (smem > 48 * 1024) cudaFuncSetAttribute(k_inc_sort, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 * 1024) dynamic_smem(k_inc_sort);
     if (nrows > 0)
       k_inc_sort<<<GT_KC(ctx, grid_for(nrows, warps)), warps * 32, smem, st>>>(*inc_ptr, *inc, nrows, icap);
     GT_LAUNCH(ctx, "k_inc_sort");
@@ -816,8 +825,8 @@ static int launch_pattern(Matrix* A, int32_t maxinc, const int32_t* bucket, bool
     if (hcap > 8192) return set_error(ctx, GT_ERR_UNSUPPORTED, "a DOF touches too many cells for the sparsity kernel");
     warps = hcap >= 4096 ? 2 : (hcap >= 2048 ? 4 : 8);
     smem = (size_t)warps * (hcap + 2 * icap) * sizeof(int32_t);
-    cudaFuncSetAttribute(k_pattern<NN, S, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(k_pattern<NN, S, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    dynamic_smem(k_pattern<NN, S, false>);
+    dynamic_smem(k_pattern<NN, S, true>);
     return GT_OK;
   };
   int32_t *rowcnt = nullptr, *dmax = nullptr, *slots = nullptr;
@@ -1216,7 +1225,7 @@ static int launch_direct(const Space* sp, const double* coef, T* Ke, double* be,
   const int32_t* cn = sp->mesh->cell_nodes;
   if (sp->mesh->ctype == GT_TET4) {
     const int smem = want_matrix ? (int)(128 * 101 * sizeof(T)) : 0;
-    GT_CUDA(ctx, cudaFuncSetAttribute(k_elements_p2<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    GT_CUDA(ctx, dynamic_smem(k_elements_p2<T>));
     k_elements_p2<T><<<GT_KC(ctx, grid_for(nc, 128)), 128, smem, ctx->stream>>>(X, cn, coef, nc, Ke, be, f, scoef,
                                                                                 want_matrix, ctx->d_err);
   } else if (sp->order == 1) {
@@ -2122,7 +2131,7 @@ static int launch_scatter(Matrix* A, const TK* Ke, double* v64, float* v32, cons
     int64_t rows_per_block = (int64_t)warps * RPW;
     int64_t grid = (r1 - r0 + rows_per_block - 1) / rows_per_block;
     auto launch = [&](auto kern) {
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      dynamic_smem(kern);
       kern<<<GT_KC(ctx, (unsigned)(grid > 0 ? grid : 1)), warps * 32, smem, ctx->stream>>>(
           A->rowptr, A->colind, A->inc_ptr, A->inc, sp->cell_ndofs, nn, r0, r1, lmax, Ke, v64, v32, be, bvec, xd);
     };
@@ -2730,7 +2739,7 @@ static int launch_uniform(Matrix* A, const double* gref, const double* coef, dou
   if (smem > 210 * 1024) return GT_ERR_UNSUPPORTED;
   auto kern = (be != nullptr && xd != nullptr) ? k_scatter_uniform<D, ORDER, BS, G, T, true>
                                                : k_scatter_uniform<D, ORDER, BS, G, T, false>;
-  GT_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  GT_CUDA(ctx, dynamic_smem(kern));
   int per_sm = 0;
   GT_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, warps * 32, smem));
   if (per_sm < 1) return GT_ERR_UNSUPPORTED;
@@ -2785,7 +2794,7 @@ static int launch_kron(Matrix* A, const T* Gc, double nu, const double* be, doub
   size_t smem = (size_t)warps * RPW * per_row;
   if (smem > 200 * 1024) return set_error(ctx, GT_ERR_UNSUPPORTED, "sparsity row too wide for the scatter kernel");
   auto kern = k_scatter_kron<D, ORDER, BS, FORM, G, T, T>;
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  dynamic_smem(kern);
   int64_t rows_per_block = (int64_t)warps * RPW;
   int64_t grid = (A->nbrows + rows_per_block - 1) / rows_per_block;
   T lamf = (T)(nu / ((1.0 + nu) * (1.0 - 2.0 * nu))), muf = (T)(1.0 / (2.0 * (1.0 + nu)));
