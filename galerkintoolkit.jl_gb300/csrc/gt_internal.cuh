@@ -263,6 +263,8 @@ inline void matrix_values_changed(Matrix* A) {
 }
 // frees the sliced-ELL copy
 void sell_release(Matrix* A);
+// makes the sliced-ELL copies of the named values current; *ok: they exist
+int sell_ready(Matrix* A, bool f64, bool f32, bool* ok);
 
 // ---------------------------------------------------------------------------
 // library-internal entry points (implemented across the .cu files)
@@ -335,8 +337,11 @@ constexpr double kRestartRatio64 = 4.0;
 constexpr int kStagnation = 3;
 
 // persistent cooperative Jacobi-PCG (gt_pcg.cu); x holds the start value
+// sliced: in the matrix's sliced form (sell_ready); kPcgNoFit, with nothing
+// done, when the system's local sets do not fit in shared memory
+constexpr int kPcgNoFit = 2;
 int pcg_persistent(Matrix* A, int mode, const double* b, double* x, double rtol, int maxit, int32_t* iters,
-                   int32_t* nupd, int32_t* iters64, double* relres);
+                   int32_t* nupd, int32_t* iters64, double* relres, bool sliced = false);
 // scalar rows up to which a system is solved by the persistent kernel
 constexpr int64_t kPersistentMaxRows = 262144;
 // pcg_persistent for several systems on ctx, in shared launches; results
@@ -350,6 +355,44 @@ int spmv64(Matrix* A, const double* x, double* y);
 // the persistent solver's grid barrier run alone (gt_pcg.cu): ctas CTAs wait
 // for ctas + missing arrivals with the given time limit
 int barrier_probe(Ctx* ctx, int ctas, int missing, int64_t timeout_ns);
+
+// A chunk of iterations of a CG loop, captured once into a CUDA graph and
+// replayed for every chunk: one graph launch instead of about five kernel
+// launches per iteration (the programmatic-launch edges between the kernels
+// are kept by the capture; every launch argument is a device pointer or a
+// size fixed for the solve), or instead of a persistent launch and its
+// readbacks.  When the capture or the instantiation fails
+// (e.g. on the legacy default stream), the chunk runs as direct launches.
+struct ChunkGraph {
+  cudaGraphExec_t exec = nullptr;
+  bool tried = false;
+  ChunkGraph() = default;
+  ChunkGraph(const ChunkGraph&) = delete;
+  ChunkGraph& operator=(const ChunkGraph&) = delete;
+  ~ChunkGraph() {
+    if (exec) cudaGraphExecDestroy(exec);
+  }
+  template <class F>
+  int run(Ctx* ctx, cudaStream_t s, F&& body) {
+    if (!tried) {
+      tried = true;
+      cudaGraph_t g = nullptr;
+      if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
+        const int rc = body();
+        const cudaError_t e = cudaStreamEndCapture(s, &g);
+        if (rc == GT_OK && e == cudaSuccess && g && cudaGraphInstantiate(&exec, g, 0) != cudaSuccess) exec = nullptr;
+        if (g) cudaGraphDestroy(g);
+      }
+      cudaGetLastError();  // a failed capture leaves its error here; the direct path follows
+    }
+    if (exec) {
+      GT_CUDA(ctx, cudaGraphLaunch(exec, s));
+      ctx->graph_launches++;
+      return GT_OK;
+    }
+    return body();
+  }
+};
 
 // device scans (exclusive prefix sum; out has n+1 entries, out[n] = total)
 int exclusive_scan_i64(Ctx* ctx, const int32_t* in, int64_t* out, int64_t n);

@@ -5,6 +5,8 @@
 namespace gt {
 namespace pcg {
 
+template int run_sliced<double, double, true>(Ctx*, Matrix*, const double*, const double*, double*, double, int, double,
+                                    const PRun*, PRun*, int);
 template int run_groups_dispatch<double, double, true>(
     Ctx*, Place, int, const std::vector<Matrix*>&, const std::vector<const double*>&,
     const std::vector<const double*>&, const std::vector<double*>&, double, int, double, const std::vector<const PRun*>&,
@@ -147,28 +149,34 @@ int pcg_persistent_groups(Ctx* ctx, const std::vector<Matrix*>& As, int mode, co
 }
 
 int pcg_persistent(Matrix* A, int mode, const double* b, double* x, double rtol, int maxit, int32_t* iters,
-                   int32_t* nupd, int32_t* iters64, double* relres) {
+                   int32_t* nupd, int32_t* iters64, double* relres, bool sliced) {
   PRun run;
   int s;
   *iters64 = 0;
+  Ctx* ctx = A->ctx;
   if (mode == GT_SOLVE_FP64) {
-    s = run_dispatch<double, double, true>(A, A->val64, b, x, rtol, maxit, 0.0, nullptr, &run);
+    s = sliced ? run_sliced<double, double, true>(ctx, A, A->val64, b, x, rtol, maxit, 0.0, nullptr, &run, 0)
+               : run_dispatch<double, double, true>(A, A->val64, b, x, rtol, maxit, 0.0, nullptr, &run);
     *iters64 = run.st.iters;
   } else if (mode == GT_SOLVE_IR) {
-    s = run_dispatch<float, float, true>(A, A->val32, b, x, rtol, maxit, A->ctx->ir_delta, nullptr, &run);
+    s = sliced ? run_sliced<float, float, true>(ctx, A, A->val32, b, x, rtol, maxit, ctx->ir_delta, nullptr, &run, 0)
+               : run_dispatch<float, float, true>(A, A->val32, b, x, rtol, maxit, ctx->ir_delta, nullptr, &run);
     if (s == PCG_STALLED) {
       // the FP32 iteration stalled or lost its rate (eps32 * cond(A) too
       // large): the same Krylov iteration goes on in FP64 from the current
       // FP64 solution and the FP32 direction
       PRun r32 = run;
       PRun r64;
-      s = run_dispatch<double, double, true>(A, A->val64, b, x, rtol, maxit, 0.0, &r32, &r64);
+      s = sliced ? run_sliced<double, double, true>(ctx, A, A->val64, b, x, rtol, maxit, 0.0, &r32, &r64, 0) : PCG_NOFIT;
+      if (s == PCG_NOFIT) s = run_dispatch<double, double, true>(A, A->val64, b, x, rtol, maxit, 0.0, &r32, &r64);
       *iters64 = r64.st.iters - r32.st.iters;
       run = r64;
     }
   } else {
-    s = run_dispatch<float, float, false>(A, A->val32, b, x, rtol, maxit, 0.0, nullptr, &run);
+    s = sliced ? run_sliced<float, float, false>(ctx, A, A->val32, b, x, rtol, maxit, 0.0, nullptr, &run, 0)
+               : run_dispatch<float, float, false>(A, A->val32, b, x, rtol, maxit, 0.0, nullptr, &run);
   }
+  if (s == PCG_NOFIT) return s;
   *iters = run.st.iters;
   *nupd = run.st.nupd;
   *relres = run.st.bb > 0 ? sqrt(run.st.rr / run.st.bb) : 0.0;

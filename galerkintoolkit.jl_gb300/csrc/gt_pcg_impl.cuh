@@ -52,6 +52,7 @@ constexpr int NW = PT / 32;      // warps per CTA
 constexpr int PSLOT = 4;         // doubles per CTA partial
 constexpr uint64_t BAR_TIMEOUT_NS = 1000000000ull;
 constexpr int PCG_STALLED = 1;   // internal status: the FP32 iteration stalled
+constexpr int PCG_NOFIT = kPcgNoFit;  // internal status: the sliced form's local sets do not fit
 
 struct PState {
   double rz, rzold, rr, rmax2, bb, tol2;
@@ -59,6 +60,7 @@ struct PState {
   double thr;       // ||r||^2 of the next reliable update (local kernel)
   uint32_t epoch;   // sums done so far (local kernel)
   int32_t iters, nupd;
+  int32_t started;  // sliced form: a chunk has run
   int32_t done;     // 1 converged or maxit, 2 FP32 iteration stalled or slowed down: continue in FP64
   int32_t stall;    // consecutive reliable updates with less than a halving of the true residual
   int32_t it_upd;   // iteration of the last reliable update
@@ -78,6 +80,8 @@ struct PArgs {
   const void* dinv;
   double* part;          // 3 slots x gridDim.x x PSLOT; local kernel: its slots and counters, zero at the start
   int lanes;             // local kernel: entry lanes per scalar row (with_lanes)
+  double* resid;         // sliced form: FP64 products of the residual
+  int init;              // sliced form: how its first chunk starts
   uint16_t* lcol;        // local kernel: local columns of the entries not held in shared memory
   uint32_t* bar;         // barrier counter, zero at launch
   int32_t* err;          // set to 1 when a barrier timed out
@@ -446,17 +450,17 @@ __global__ void __launch_bounds__(PT) k_pcg(PArgs a, int init, int it_end) {
 // args[map[c].x].nb CTAs that solve system map[c].x, exactly as that system's
 // own launch would (map null: one system, the whole grid); in the cluster
 // form cluster c solves system c.
-template <int BS, class V, class X, bool RELIABLE, bool CL>
+template <int BS, class V, class X, bool RELIABLE, bool CL, bool SL = false>
 __device__ __forceinline__ void local_group_entry(const PArgs* args, int sys, int nb, int blk, int init, int chunk,
                                                   unsigned char* smem, int smem_bytes, LShared& S, LCluster* C) {
   const PArgs a = args[sys];
   if (a.st->done) return;  // finished in an earlier launch (the same in all its CTAs)
   int it_end = a.st->iters + chunk;
   if (it_end > a.maxit || it_end < 0) it_end = a.maxit;
-  pcg_local_body<BS, V, X, RELIABLE, CL>(a, CL ? nb : a.nb, blk, init, it_end, smem, smem_bytes, S, C);
+  pcg_local_body<BS, V, X, RELIABLE, CL, SL>(a, CL ? nb : a.nb, blk, init, it_end, smem, smem_bytes, S, C);
 }
 template <int BS, class V, class X, bool RELIABLE>
-__global__ void __launch_bounds__(LT) k_pcg_local(const PArgs* __restrict__ args, const int2* __restrict__ map,
+__global__ void __launch_bounds__(LT, 1) k_pcg_local(const PArgs* __restrict__ args, const int2* __restrict__ map,
                                                          int init, int chunk, int smem_bytes) {
   extern __shared__ __align__(16) unsigned char s_dyn[];
   __shared__ LShared S;
@@ -464,13 +468,21 @@ __global__ void __launch_bounds__(LT) k_pcg_local(const PArgs* __restrict__ args
   local_group_entry<BS, V, X, RELIABLE, false>(args, m.x, 0, m.y, init, chunk, s_dyn, smem_bytes, S, nullptr);
 }
 template <int BS, class V, class X, bool RELIABLE>
-__global__ void __launch_bounds__(LT) k_pcg_cluster(const PArgs* __restrict__ args, int init, int chunk,
+__global__ void __launch_bounds__(LT, 1) k_pcg_cluster(const PArgs* __restrict__ args, int init, int chunk,
                                                     int smem_bytes) {
   extern __shared__ __align__(16) unsigned char s_dyn[];
   __shared__ LShared S;
   __shared__ LCluster C;
   local_group_entry<BS, V, X, RELIABLE, true>(args, blockIdx.x / LCLUSTER, LCLUSTER, blockIdx.x % LCLUSTER, init,
                                                  chunk, s_dyn, smem_bytes, S, &C);
+}
+
+// one system in its sliced form (SL), the whole grid
+template <class V, class X, bool RELIABLE>
+__global__ void __launch_bounds__(LT, 1) k_pcg_sliced(const PArgs* __restrict__ args, int chunk, int smem_bytes) {
+  extern __shared__ __align__(16) unsigned char s_dyn[];
+  __shared__ LShared S;
+  local_group_entry<1, V, X, RELIABLE, false, true>(args, 0, 0, blockIdx.x, args->st->started ? 0 : args->init, chunk, s_dyn, smem_bytes, S, nullptr);
 }
 
 template <int BS, class V, class X>
@@ -500,6 +512,7 @@ struct PSolve {
   X *xs = nullptr, *r = nullptr, *z = nullptr, *p = nullptr, *q = nullptr, *dinv = nullptr;
   double* part = nullptr;
   uint16_t* lcol = nullptr; // local kernel only
+  double* resid = nullptr;  // sliced form only
   uint32_t* bar = nullptr;  // own (stand-alone) or a slot of a grouped launch's array
   int32_t* err = nullptr;
   PState* st = nullptr;
@@ -525,6 +538,8 @@ static int pcg_ctas(Ctx* ctx, const Matrix* A, int* nb) {
 // expected need (the halo about seven times the rows; a grid gets no more
 // than it can use, so that systems of several contexts run side by side),
 // most: the device's limit, for systems whose local sets do not fit est.
+// The kernels' attribute is always set to most: it is the process's, and
+// another thread may launch the same kernel with another size.
 struct LPlan {
   int nb = 1;
   int est = 0, most = 0;
@@ -573,7 +588,7 @@ static bool cluster_place(const Matrix* A, bool fp64, Place place) {
 // diagonal of one system; bar / err / st come from the caller when given
 template <int BS, int G, class V, class X, bool REL>
 static int pcg_prepare(Ctx* ctx, PSolve<BS, G, V, X, REL>& P, Matrix* A, const V* val, const double* b, double* x,
-                       double rtol, int maxit, double delta, const PRun* from, int nb, bool local,
+                       double rtol, int maxit, double delta, const PRun* from, int nb, bool local, bool sliced = false,
                        uint32_t* bar = nullptr, int32_t* err = nullptr, PState* st = nullptr) {
   cudaStream_t s = ctx->stream;
   const int64_t n = A->nbrows * BS;
@@ -587,7 +602,8 @@ static int pcg_prepare(Ctx* ctx, PSolve<BS, G, V, X, REL>& P, Matrix* A, const V
   GT_TRY(dalloc(ctx, &P.dinv, n));
   if (local) {
     GT_TRY(dalloc(ctx, &P.part, (int64_t)LSLOTS * P.nb + LCTRS));
-    GT_TRY(dalloc(ctx, &P.lcol, A->bnnz));
+    GT_TRY(dalloc(ctx, &P.lcol, sliced ? A->sell_total : A->bnnz));
+    if (sliced) GT_TRY(dalloc(ctx, &P.resid, n));
     GT_CUDA(ctx, cudaMemsetAsync(P.part, 0, sizeof(double) * (LSLOTS * P.nb + LCTRS), s));
   } else {
     GT_TRY(dalloc(ctx, &P.q, n));
@@ -610,6 +626,7 @@ static int pcg_prepare(Ctx* ctx, PSolve<BS, G, V, X, REL>& P, Matrix* A, const V
     *h0 = from->st;
     h0->done = 0;
     h0->epoch = 0;
+    h0->started = 0;
     GT_CUDA(ctx, cudaMemcpyAsync(P.st, h0, sizeof(PState), cudaMemcpyHostToDevice, s));
     GT_CUDA(ctx, cudaStreamSynchronize(s));
   } else {
@@ -628,6 +645,12 @@ static int pcg_prepare(Ctx* ctx, PSolve<BS, G, V, X, REL>& P, Matrix* A, const V
   args.colind = A->colind;
   args.val = val;
   args.val64 = dval;
+  if (sliced) {
+    args.rowptr = A->sell_ptr;
+    args.colind = A->sell_col;
+    args.val = sizeof(V) == sizeof(double) ? (const void*)A->sell_v64 : (const void*)A->sell_v32;
+    args.val64 = A->sell_v64;
+  }
   args.nrows = A->nbrows;
   args.nb = P.nb;
   args.b = b;
@@ -640,6 +663,8 @@ static int pcg_prepare(Ctx* ctx, PSolve<BS, G, V, X, REL>& P, Matrix* A, const V
   args.dinv = P.dinv;
   args.part = P.part;
   args.lcol = P.lcol;
+  args.resid = P.resid;
+  args.init = from ? 2 : 1;
   const double avg = A->nbrows > 0 ? (double)A->bnnz / (double)A->nbrows : 1.0;
   args.lanes = sizeof(X) == sizeof(double) && avg <= 20 ? 1 : (avg <= 40 ? 2 : 4);
   args.bar = P.bar;
@@ -664,6 +689,7 @@ static void pcg_release(PSolve<BS, G, V, X, REL>& P) {
   dfree(ctx, P.dinv);
   dfree(ctx, P.part);
   dfree(ctx, P.lcol);
+  dfree(ctx, P.resid);
   if (P.own_sync) {
     dfree(ctx, P.bar);
     dfree(ctx, P.err);
@@ -707,7 +733,7 @@ int run_typed(Ctx* ctx, Matrix* A, const V* val, const double* b, double* x, dou
   for (bool local = L.ok;;) {
     int nb = L.nb;
     if (!local) GT_TRY((pcg_ctas<BS, G, V, X, REL>(ctx, A, &nb)));
-    else GT_CUDA(ctx, cudaFuncSetAttribute(lkern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    else GT_CUDA(ctx, cudaFuncSetAttribute(lkern, cudaFuncAttributeMaxDynamicSharedMemorySize, L.most));
     PSolve<BS, G, V, X, REL> P;
     GT_TRY((pcg_prepare<BS, G, V, X, REL>(ctx, P, A, val, b, x, rtol, maxit, delta, from, nb, local)));
     PArgs& args = P.args;
@@ -757,6 +783,62 @@ int run_typed(Ctx* ctx, Matrix* A, const V* val, const double* b, double* x, dou
     }
     return pcg_finish<BS, G, V, X, REL>(P, h, err, out);
   }
+}
+
+// A scalar system in its sliced form; PCG_NOFIT, with nothing done, when it has
+// no sliced copy or its local sets do not fit in shared memory.  smem: a CTA's
+// shared memory (0: the expected need)
+template <class V, class X, bool REL>
+int run_sliced(Ctx* ctx, Matrix* A, const V* val, const double* b, double* x, double rtol, int maxit, double delta,
+               const PRun* from, PRun* out, int smem) {
+  cudaStream_t s = ctx->stream;
+  auto kern = k_pcg_sliced<V, X, REL>;
+  LPlan L;
+  GT_TRY(local_plan(ctx, A, kern, false, sizeof(X), sizeof(V), &L));
+  // r, q, p and the column numbers (and x) of rows and halo: at most a band of
+  // the space's DOF spread on both sides; on a three-dimensional mesh in
+  // lexicographic order about three planes' shares
+  const int64_t rows = (A->nbrows + L.nb - 1) / L.nb, spread = A->space->dof_spread;
+  int64_t local = rows * 13 / 4 + 512;
+  if (spread >= 0) local = std::min<int64_t>(local, rows + 2 * spread);
+  const int64_t need = rows * 5 / 4 * 2 * (int64_t)sizeof(X) + local * (int64_t)(sizeof(X) + 4 + (REL && sizeof(X) == 4 ? 8 : 0)) + 8192;
+  if (need > L.most + 8192) return PCG_NOFIT;
+  bool ready = false;
+  GT_TRY(sell_ready(A, REL, sizeof(V) == 4, &ready));
+  if (!ready) return PCG_NOFIT;
+  if (smem == 0) smem = (int)std::min<int64_t>(L.most, (need + 1023) & ~int64_t(1023));
+  GT_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L.most));
+  PSolve<1, 2, V, X, REL> P;
+  GT_TRY((pcg_prepare<1, 2, V, X, REL>(ctx, P, A, val, b, x, rtol, maxit, delta, from, L.nb, true, true)));
+  PArgs* dargs = nullptr;
+  GT_TRY(dalloc(ctx, (unsigned char**)&dargs, (int64_t)sizeof(PArgs)));
+  GT_TRY(copy_in(ctx, (unsigned char*)dargs, (const unsigned char*)&P.args, (int64_t)sizeof(PArgs)));
+  PState h{};
+  int32_t e = 0;
+  int chunk = 512;
+  ChunkGraph graph;
+  auto body = [&]() -> int {
+    ctx->launches++;
+    void* kargs[] = {&dargs, &chunk, &smem};
+    GT_CUDA(ctx, cudaLaunchCooperativeKernel((const void*)kern, dim3(P.nb), dim3(LT), kargs, smem, s));
+    GT_CUDA(ctx, cudaMemcpyAsync(ctx->h_dscratch, P.st, sizeof(PState), cudaMemcpyDeviceToHost, s));
+    GT_CUDA(ctx, cudaMemcpyAsync(ctx->h_scratch, P.err, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+    return GT_OK;
+  };
+  while (true) {
+    GT_TRY(graph.run(ctx, s, body));
+    GT_CUDA(ctx, cudaStreamSynchronize(s));
+    memcpy(&h, ctx->h_dscratch, sizeof(PState));
+    memcpy(&e, ctx->h_scratch, sizeof(int32_t));
+    if (e || h.done || h.iters >= maxit) break;
+  }
+  pool_free(ctx, dargs);
+  if (!e && h.done == LOVERFLOW) {
+    pcg_release(P);
+    if (smem < L.most) return run_sliced<V, X, REL>(ctx, A, val, b, x, rtol, maxit, delta, from, out, L.most);
+    return PCG_NOFIT;
+  }
+  return pcg_finish<1, 2, V, X, REL>(P, h, e != 0, out);
 }
 
 // Systems of one block size, each on the CTAs its stand-alone
@@ -838,7 +920,7 @@ static int run_groups_typed(Ctx* ctx, Place place, const std::vector<Matrix*>& A
         const int i = ids[k];
         prepared++;
         GT_TRY((pcg_prepare<BS, G, V, X, REL>(ctx, P[k], As[i], vals[i], bs[i], xs[i], rtol, maxit, delta, froms[i],
-                                              cluster ? LCLUSTER : plan[i].nb, true, bars + 2 * k, errs + 2 * k,
+                                              cluster ? LCLUSTER : plan[i].nb, true, false, bars + 2 * k, errs + 2 * k,
                                               sts + k)));
         hargs[k] = P[k].args;
         for (int j = 0; !cluster && j < P[k].nb; j++) hmap.push_back(make_int2(k, j));
@@ -905,7 +987,7 @@ static int run_groups_typed(Ctx* ctx, Place place, const std::vector<Matrix*>& A
   size_t i0 = 0;
   while (i0 < order.size()) {
     const int smem = plan[order[i0]].est;
-    GT_CUDA(ctx, cudaFuncSetAttribute(gkern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    GT_CUDA(ctx, cudaFuncSetAttribute(gkern, cudaFuncAttributeMaxDynamicSharedMemorySize, plan[order[i0]].most));
     int per_sm = 0;
     GT_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gkern, LT, smem));
     const int64_t cap = (int64_t)per_sm * ctx->num_sms;
@@ -954,6 +1036,12 @@ extern template int run_groups_dispatch<float, float, false>(
     Ctx*, Place, int, const std::vector<Matrix*>&, const std::vector<const float*>&,
     const std::vector<const double*>&, const std::vector<double*>&, double, int, double, const std::vector<const PRun*>&,
     std::vector<PRun>&, std::vector<int>&);
+extern template int run_sliced<double, double, true>(Ctx*, Matrix*, const double*, const double*, double*, double, int, double,
+                                    const PRun*, PRun*, int);
+extern template int run_sliced<float, float, true>(Ctx*, Matrix*, const float*, const double*, double*, double, int, double,
+                                    const PRun*, PRun*, int);
+extern template int run_sliced<float, float, false>(Ctx*, Matrix*, const float*, const double*, double*, double, int, double,
+                                    const PRun*, PRun*, int);
 
 }  // namespace pcg
 }  // namespace gt

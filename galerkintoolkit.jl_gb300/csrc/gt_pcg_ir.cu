@@ -4,6 +4,8 @@
 namespace gt {
 namespace pcg {
 
+template int run_sliced<float, float, true>(Ctx*, Matrix*, const float*, const double*, double*, double, int, double,
+                                    const PRun*, PRun*, int);
 template int run_groups_dispatch<float, float, true>(
     Ctx*, Place, int, const std::vector<Matrix*>&, const std::vector<const float*>&,
     const std::vector<const double*>&, const std::vector<double*>&, double, int, double, const std::vector<const PRun*>&,

@@ -26,6 +26,12 @@
 // in L2 polled by the CTAs of a grid (and 1,500 more for the partials behind
 // it).  Small systems, for which the barriers are the iteration, take it.
 //
+// SL: systems too large for that (scalar rows).  xs and Dinv stay in global
+// memory (a thread only touches its own rows' entries), the matrix streams
+// from its sliced copy (32-row slices, a lane per row, coalesced) with 16-bit
+// local columns in the same layout, and the bitmap covers only the window of
+// columns the CTA touches.
+//
 // What bounds it.  GB300 issues one FP64 warp instruction per SM sub-partition
 // every 63 clocks (measured; 304 clocks for one FP64 add in each of 16 warps,
 // 570 for a division), whatever the number of active lanes.  So
@@ -47,6 +53,7 @@ constexpr int LNW = LT / 32;   // warps per CTA
 constexpr int LMAXCTA = 160;   // most CTAs of one system in a grid (five partials per lane)
 constexpr int LCLUSTER = 16;   // CTAs of one system in a cluster
 constexpr int kLocalRows = 64; // scalar rows per CTA up to a CTA per SM
+constexpr int kSliceRowCost = 5;  // a row's cost beside its entries in the sliced form, in entries
 constexpr int LOVERFLOW = 3;   // PState::done: a CTA's local set does not fit
 // a scalar row's cost beside its entries, in FMAs: the vector updates, the
 // combination of its partial sums and its lanes' idle last step
@@ -190,6 +197,7 @@ struct LShared {
   int next;             // next row group of local_rows
   int rsm;              // rows whose matrix part is in shared memory
   int nloc;             // local columns
+  int cmin, cmax;       // the columns' range (SL)
   int64_t rows[2];      // the CTA's first row and its end
   int wsum[LNW];
 };
@@ -364,6 +372,42 @@ __device__ __forceinline__ void local_group(int row0, int re, const int32_t* rp,
   if (ok && j == 0) put(row, c, s);
 }
 
+// One sweep over the CTA's ns slices, a lane per row, a warp taking its own
+// number's slice, then the next one nobody took (*next); sp[i]: first entry of
+// slice i (its steps' 32 entries are adjacent).  put(row, sum).  U steps are
+// loaded at once: 4 of FP64, where the FP64 pipe is the limit (8 and 16: 6 and
+// 13% slower), 16 of FP32 (8: 2% slower); loading ahead of the additions, also
+// across slices, gained nothing over the other warps' loads in flight.
+template <int U, class A, class V, class GET, class PUT>
+__device__ __forceinline__ void local_slices(int ns, const int32_t* sp, const V* __restrict__ val, const uint16_t* lc,
+                                             int* next, GET&& get, PUT&& put) {
+  const int lane = threadIdx.x & 31;
+  int si = threadIdx.x >> 5;
+  while (si < ns) {
+    const int o = sp[si] + lane, n = (sp[si + 1] - sp[si]) >> 5;
+    A s = (A)0;
+    V a[U];
+    int c[U];
+    auto load = [&](int t, V (&v)[U], int (&j)[U]) {
+#pragma unroll
+      for (int u = 0; u < U; u++)
+        if (t + u < n) {
+          v[u] = __ldcg(val + o + (t + u) * 32);
+          j[u] = __ldcg(lc + o + (t + u) * 32);
+        }
+    };
+    for (int t = 0; t < n; t += U) {
+      load(t, a, c);
+#pragma unroll
+      for (int u = 0; u < U; u++)
+        if (t + u < n) s = fma((A)a[u], get(c[u]), s);
+    }
+    put(si * 32 + lane, s);
+    if (lane == 0) si = atomicAdd(next, 1);
+    si = __shfl_sync(0xffffffffu, si, 0);
+  }
+}
+
 // The CTA's row groups, the streamed rows [rsm, nr) first (their loads take
 // longest), then the resident ones; a warp takes its own first group, then
 // the next one nobody took (S.next, reset by local_total's callers).
@@ -382,21 +426,21 @@ __device__ __forceinline__ void local_sweep(int nr, int rsm, LShared& S, F1&& st
   }
 }
 
-// first row of CTA blk of nb: the rows are split at equal shares of
-// cost(r) = FMAs of the rows before r + row_cost per scalar row.  Called by
-// one warp (32 probes a step).
-template <int BS>
-__device__ __forceinline__ int64_t local_first_row(const int64_t* __restrict__ rowptr, int64_t n, int nb, int blk) {
+// first row (slice) of CTA blk of nb: the rows are split at equal shares of
+// cost(r) = per_entry x the entries before r + per_row x r.  Called by one
+// warp (32 probes a step).
+__device__ __forceinline__ int64_t local_first_row(const int64_t* __restrict__ rowptr, int64_t n, int nb, int blk,
+                                                   int per_entry, int per_row) {
   const int lane = threadIdx.x & 31;
   if (blk <= 0) return 0;
   if (blk >= nb) return n;
-  const int64_t total = __ldg(rowptr + n) * (BS * BS) + n * (BS * row_cost(BS));
+  const int64_t total = __ldg(rowptr + n) * per_entry + n * per_row;
   const int64_t want = total / nb * blk + total % nb * blk / nb;
   int64_t lo = 0, hi = n;  // cost(lo) < want <= cost(hi)
   while (hi - lo > 1) {
     const int64_t step = (hi - lo + 32) / 33;
     const int64_t r = lo + step * (lane + 1);
-    const bool ge = r >= hi || __ldg(rowptr + r) * (BS * BS) + r * (BS * row_cost(BS)) >= want;
+    const bool ge = r >= hi || __ldg(rowptr + r) * per_entry + r * per_row >= want;
     const unsigned m = __ballot_sync(0xffffffffu, ge);
     const int f = m ? __ffs(m) - 1 : 32;
     const int64_t nlo = lo + step * f;
@@ -422,13 +466,13 @@ __device__ __forceinline__ void with_lanes(int j, F&& f) {
   else f(std::integral_constant<int, 4>());
 }
 
-template <int BS, class V, class X, bool RELIABLE, bool CL>
+template <int BS, class V, class X, bool RELIABLE, bool CL, bool SL>
 __device__ __forceinline__ void pcg_local_body(const PArgs& a, int nb, int blk, int init, int it_end,
                                                unsigned char* smem, int smem_bytes, LShared& S, LCluster* C) {
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   if constexpr (CL) {
     for (int i = wid; i <= nb; i += LNW) {
-      const int64_t r = local_first_row<BS>(a.rowptr, a.nrows, nb, i);
+      const int64_t r = local_first_row(a.rowptr, a.nrows, nb, i, BS * BS, BS * row_cost(BS));
       if (lane == 0) {
         C->first[i] = r;
         if (i == blk) S.rows[0] = r;
@@ -436,18 +480,23 @@ __device__ __forceinline__ void pcg_local_body(const PArgs& a, int nb, int blk, 
       }
     }
   } else if (wid < 2) {
-    const int64_t r = local_first_row<BS>(a.rowptr, a.nrows, nb, blk + wid);
+    const int64_t r = SL ? local_first_row(a.rowptr, (a.nrows + 31) / 32, nb, blk + wid, 1, 32 * kSliceRowCost)
+                         : local_first_row(a.rowptr, a.nrows, nb, blk + wid, BS * BS, BS * row_cost(BS));
     if (lane == 0) S.rows[wid] = r;
   }
   if (tid == 0) {
     S.abort = 0;
+    S.cmin = INT_MAX;
+    S.cmax = 0;
     S.next = LNW;
     S.st = *a.st;
   }
   uint32_t epoch = a.st->epoch;
   if constexpr (CL) cluster_sync();  // every CTA of the cluster runs: its shared memory may be written
   else __syncthreads();
-  const int64_t r0 = S.rows[0], r1 = S.rows[1];
+  // SL: the rows of slices [f0, f1), a.rowptr being the slices' pointers
+  const int64_t f0 = S.rows[0], f1 = S.rows[1];
+  const int64_t r0 = SL ? min(a.nrows, f0 * 32) : f0, r1 = SL ? min(a.nrows, f1 * 32) : f1;
   const int nr = (int)(r1 - r0);
   const int n_own = nr * BS;
   const int64_t e0 = r0 * BS;
@@ -459,34 +508,62 @@ __device__ __forceinline__ void pcg_local_body(const PArgs& a, int nb, int blk, 
   X* s_r = s_z + (CL ? n_own : 0);
   X* s_q = s_r + n_own;
   X* s_xs = s_q + n_own;
-  X* s_di = s_xs + n_own;
-  X* s_p = s_di + n_own;
-  const int nwords = (int)((a.nrows + 31) / 32);
+  X* s_di = s_xs + (SL ? 0 : n_own);
+  X* s_p = s_di + (SL ? 0 : n_own);
+  X* const w_xs = SL ? (X*)a.xs + e0 : s_xs;
+  const X* const w_di = SL ? (const X*)a.dinv + e0 : s_di;
+  const int64_t k0 = a.rowptr[f0];
+  const int nk = (int)(a.rowptr[f1] - k0);
+  // bitmap words [w0, w0 + nwords)
+  int w0 = 0, nwords = (int)((a.nrows + 31) / 32);
+  if constexpr (SL) {
+    int lo = INT_MAX, hi = 0;
+    for (int i = tid; i < nk; i += LT) {
+      const int c = __ldg(a.colind + k0 + i);
+      lo = min(lo, c);
+      hi = max(hi, c);
+    }
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    if (lane == 0) {
+      atomicMin(&S.cmin, lo);
+      atomicMax(&S.cmax, hi);
+    }
+    __syncthreads();
+    lo = min(S.cmin, nr > 0 ? (int)r0 : INT_MAX);
+    hi = max(S.cmax, (int)r1 - 1);
+    w0 = nr > 0 ? lo >> 5 : 0;
+    nwords = nr > 0 ? (hi >> 5) - w0 + 1 : 0;
+  }
   const int tail = ((nwords * 6 + 15) & ~15);  // 32-bit bitmap words + 16-bit prefix
-  uint32_t* s_bit = reinterpret_cast<uint32_t*>(smem + smem_bytes - tail);
+  // (a window beyond the shared memory: no columns are marked, and the local
+  // set counts as not fitting below)
+  const bool window = !SL || tail + 4096 <= smem_bytes;
+  if (!window) nwords = 0;
+  uint32_t* s_bit = reinterpret_cast<uint32_t*>(smem + smem_bytes - (window ? tail : 0));
   uint16_t* s_base = reinterpret_cast<uint16_t*>(s_bit + nwords);
 
   // --- the local columns
-  const int64_t k0 = a.rowptr[r0];
-  const int nk = (int)(a.rowptr[r1] - k0);
   for (int i = tid; i < nwords; i += LT) s_bit[i] = 0;
   __syncthreads();
-  for (int i = tid; i < nk; i += LT) {
-    const int c = __ldg(a.colind + k0 + i);
-    const uint32_t m = 1u << (c & 31);
-    if (!(*(volatile uint32_t*)&s_bit[c >> 5] & m)) atomicOr(&s_bit[c >> 5], m);
-  }
-  for (int i = tid; i < nr; i += LT) {
-    const int c = (int)r0 + i;
-    atomicOr(&s_bit[c >> 5], 1u << (c & 31));
+  if (window) {
+    for (int i = tid; i < nk; i += LT) {
+      const int c = __ldg(a.colind + k0 + i);
+      const uint32_t m = 1u << (c & 31);
+      if (!(*(volatile uint32_t*)&s_bit[(c >> 5) - w0] & m)) atomicOr(&s_bit[(c >> 5) - w0], m);
+    }
+    for (int i = tid; i < nr; i += LT) {
+      const int c = (int)r0 + i;
+      atomicOr(&s_bit[(c >> 5) - w0], 1u << (c & 31));
+    }
   }
   __syncthreads();
   {
     // exclusive prefix of the words' bit counts: a run of words per thread
     const int per = (nwords + LT - 1) / LT;
-    const int w0 = min(nwords, tid * per), w1 = min(nwords, w0 + per);
+    const int v0 = min(nwords, tid * per), v1 = min(nwords, v0 + per);
     int t = 0;
-    for (int i = w0; i < w1; i++) t += __popc(s_bit[i]);
+    for (int i = v0; i < v1; i++) t += __popc(s_bit[i]);
     int inc = t;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -501,7 +578,7 @@ __device__ __forceinline__ void pcg_local_body(const PArgs& a, int nb, int blk, 
       all += S.wsum[i];
     }
     b += inc - t;
-    for (int i = w0; i < w1; i++) {
+    for (int i = v0; i < v1; i++) {
       s_base[i] = (uint16_t)min(b, 65535);
       b += __popc(s_bit[i]);
     }
@@ -518,10 +595,10 @@ __device__ __forceinline__ void pcg_local_body(const PArgs& a, int nb, int blk, 
   int32_t* s_g = reinterpret_cast<int32_t*>(s_x + (XL ? (size_t)nloc * BS : 0));
   int32_t* s_gc = XL && CL ? s_g + nloc : s_g;
   int32_t* s_rp = s_gc + nloc;
-  size_t used = reinterpret_cast<unsigned char*>(s_rp + nr + 1) - smem;
+  size_t used = reinterpret_cast<unsigned char*>(s_rp + (int)(f1 - f0) + 1) - smem;
   used = (used + 15) & ~size_t(15);
   {
-    const bool fits = nloc < 65535 && used + tail <= (size_t)smem_bytes;
+    const bool fits = window && nloc < 65535 && used + tail <= (size_t)smem_bytes;
     const float v[1] = {fits ? 0.0f : 1.0f};
     if (!local_total<1, CL>(v, 1, nb, blk, a.part, epoch, a.err, S, C,
                             [&](const double* tot) { S.overflow = __double_as_longlong(tot[0]) != 0; }))
@@ -540,7 +617,7 @@ __device__ __forceinline__ void pcg_local_body(const PArgs& a, int nb, int blk, 
     uint32_t m = s_bit[i];
     int b = s_base[i], own = 0;
     while (m) {
-      const int c = i * 32 + __ffs(m) - 1;
+      const int c = (w0 + i) * 32 + __ffs(m) - 1;
       if constexpr (CL) {
         // the column's z in its owner's shared memory
         while (c >= C->first[own + 1]) own++;
@@ -552,10 +629,12 @@ __device__ __forceinline__ void pcg_local_body(const PArgs& a, int nb, int blk, 
       m &= m - 1;
     }
   }
-  for (int i = tid; i <= nr; i += LT) s_rp[i] = (int)(a.rowptr[r0 + i] - k0);
+  for (int i = tid; i <= (int)(f1 - f0); i += LT) s_rp[i] = (int)(a.rowptr[f0 + i] - k0);
   __syncthreads();
-  const int ownb = nr > 0 ? s_base[r0 >> 5] + __popc(s_bit[r0 >> 5] & ((1u << (r0 & 31)) - 1u)) : 0;
-  if (tid == 0) {
+  const int ownb = nr > 0 ? s_base[(r0 >> 5) - w0] + __popc(s_bit[(r0 >> 5) - w0] & ((1u << (r0 & 31)) - 1u)) : 0;
+  if (SL) {
+    if (tid == 0) S.rsm = 0;
+  } else if (tid == 0) {
     // the most rows whose entries fit
     const size_t avail = smem_bytes - tail - used;
     const int cap = (int)min((size_t)nk, avail / (sizeof(V) * BS * BS + sizeof(uint16_t)));
@@ -577,7 +656,7 @@ __device__ __forceinline__ void pcg_local_body(const PArgs& a, int nb, int blk, 
   for (int i = tid; i < ksm * BS * BS; i += LT) s_val[i] = __ldg(gval + i);
   for (int i = tid; i < nk; i += LT) {
     const int c = __ldg(gcol + i);
-    const uint16_t lc = (uint16_t)(s_base[c >> 5] + __popc(s_bit[c >> 5] & ((1u << (c & 31)) - 1u)));
+    const uint16_t lc = (uint16_t)(s_base[(c >> 5) - w0] + __popc(s_bit[(c >> 5) - w0] & ((1u << (c & 31)) - 1u)));
     if (i < ksm) s_lc[i] = lc;
     else glc[i] = lc;  // read back by this CTA only, after the barriers below
   }
@@ -588,7 +667,15 @@ __device__ __forceinline__ void pcg_local_body(const PArgs& a, int nb, int blk, 
   X* z = (X*)a.z;
   X* p = (X*)a.p;
   const X* dinv = (const X*)a.dinv;
-  for (int i = tid; i < n_own; i += LT) s_di[i] = dinv[e0 + i];
+  if constexpr (!SL)
+    for (int i = tid; i < n_own; i += LT) s_di[i] = dinv[e0 + i];
+  // one sweep over the CTA's slices with values v (SL): put(row, sum)
+  auto slices = [&](auto* v, auto zero, auto&& get, auto&& put) {
+    local_slices<sizeof(*v) == 8 ? 4 : 16, decltype(zero)>((int)(f1 - f0), s_rp, v, glc, &S.next, get,
+                                                            [&](int row, auto t) {
+                                                              if (row < nr) put(row, t);
+                                                            });
+  };
 
   // FP64 residual r = b - A x of the own rows -> s_r, z; v: r.z, ||r||^2, ||b||^2
   auto residual = [&](double (&v)[3]) {
@@ -604,7 +691,7 @@ __device__ __forceinline__ void pcg_local_body(const PArgs& a, int nb, int blk, 
     auto put = [&](int row, int c, double o) {
       const int i = row * BS + c;
       const double bi = a.b[e0 + i], ri = bi - o;
-      const X rx = (X)ri, zx = s_di[i] * rx;
+      const X rx = (X)ri, zx = w_di[i] * rx;
       s_r[i] = rx;
       if constexpr (CL) s_z[i] = zx;
       else __stcg(z + e0 + i, zx);
@@ -612,6 +699,16 @@ __device__ __forceinline__ void pcg_local_body(const PArgs& a, int nb, int blk, 
       v[1] += ri * ri;
       v[2] += bi * bi;
     };
+    if constexpr (SL) {
+      // (the rows' sums first: a thread's own rows follow its number alone)
+      auto sq = [&](int row, double o) { a.resid[r0 + row] = o; };
+      if constexpr (XL) slices(a.val64 + k0, 0.0, [&](int c) { return s_x[c]; }, sq);
+      else if constexpr (RELIABLE) slices(a.val64 + k0, 0.0, [&](int c) { return __ldcg(a.x + s_g[c]); }, sq);
+      else slices(gval, 0.0, [&](int c) { return __ldcg(a.x + s_g[c]); }, sq);
+      __syncthreads();
+      if (tid == 0) S.next = LNW;
+      for (int i = tid; i < nr; i += LT) put(i, 0, a.resid[r0 + i]);
+    } else
     // (a thread's rows follow the warp's number alone: the sums are reproducible)
     with_lanes<BS>(a.lanes, [&](auto jt) {
       constexpr int J = decltype(jt)::value, GPW = 32 / (BS * J), U = BS == 1 ? 8 : 4;
@@ -644,10 +741,11 @@ __device__ __forceinline__ void pcg_local_body(const PArgs& a, int nb, int blk, 
     // diverge at tolerances near the attainable accuracy (measured)
     double v[3] = {0.0, 0.0, 0.0};
     residual(v);
-    for (int i = tid; i < n_own; i += LT) s_xs[i] = (X)0;
+    for (int i = tid; i < n_own; i += LT) w_xs[i] = (X)0;
     for (int i = tid; i < nl; i += LT) s_p[i] = (X)0;
     if (!local_total<3, CL>(v, LT, nb, blk, a.part, epoch, a.err, S, C, [&](const double* tot) {
           PState& T = S.st;
+          T.started = 1;
           T.rz = tot[0];
           T.rr = tot[1];
           T.rmax2 = T.rr;
@@ -672,7 +770,7 @@ __device__ __forceinline__ void pcg_local_body(const PArgs& a, int nb, int blk, 
   } else {
     for (int i = tid; i < n_own; i += LT) {
       s_r[i] = r[e0 + i];
-      s_xs[i] = xs[e0 + i];
+      if constexpr (!SL) s_xs[i] = xs[e0 + i];
     }
     for (int i = tid; i < n_own; i += LT)
       if constexpr (CL) s_z[i] = s_di[i] * s_r[i];
@@ -681,7 +779,7 @@ __device__ __forceinline__ void pcg_local_body(const PArgs& a, int nb, int blk, 
       uint32_t m = s_bit[i];
       int b = s_base[i];
       while (m) {
-        const int64_t c = i * 32 + __ffs(m) - 1;
+        const int64_t c = (int64_t)(w0 + i) * 32 + __ffs(m) - 1;
         for (int d = 0; d < BS; d++) s_p[b * BS + d] = __ldcg(p + c * BS + d);
         b++;
         m &= m - 1;
@@ -721,7 +819,8 @@ __device__ __forceinline__ void pcg_local_body(const PArgs& a, int nb, int blk, 
     {
       auto get = [&](int c, int d) { return s_p[c * BS + d]; };
       auto put = [&](int row, int c, X o) { s_q[row * BS + c] = o; };
-      with_lanes<BS>(a.lanes, [&](auto jt) {
+      if constexpr (SL) slices(gval, (X)0, [&](int c) { return s_p[c]; }, [&](int row, X o) { s_q[row] = o; });
+      else with_lanes<BS>(a.lanes, [&](auto jt) {
         constexpr int J = decltype(jt)::value;
         local_sweep<BS, J>(
             nr, rsm, S, [&](int row0) { local_group<BS, J, 4, X>(row0, nr, s_rp, gval, glc, get, put); },
@@ -740,15 +839,29 @@ __device__ __forceinline__ void pcg_local_body(const PArgs& a, int nb, int blk, 
     {
       const X alpha = (X)S.alpha;
       X v[2] = {(X)0, (X)0};
-      for (int i = tid; i < n_own; i += LT) {
-        const X ri = s_r[i] - alpha * s_q[i];
-        const X zi = s_di[i] * ri;
-        s_xs[i] += alpha * s_po[i];
-        s_r[i] = ri;
-        if constexpr (CL) s_z[i] = zi;
-        else __stcg(z + e0 + i, zi);
-        v[0] += ri * zi;
-        v[1] += ri * ri;
+      constexpr int U = SL ? 4 : 1;
+      for (int i0 = tid; i0 < n_own; i0 += U * LT) {
+        X dv[U], xv[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+          const int i = i0 + u * LT;
+          dv[u] = i < n_own ? w_di[i] : (X)0;
+          xv[u] = i < n_own ? w_xs[i] : (X)0;
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+          const int i = i0 + u * LT;
+          if (i < n_own) {
+            const X ri = s_r[i] - alpha * s_q[i];
+            const X zi = dv[u] * ri;
+            w_xs[i] = xv[u] + alpha * s_po[i];
+            s_r[i] = ri;
+            if constexpr (CL) s_z[i] = zi;
+            else __stcg(z + e0 + i, zi);
+            v[0] += ri * zi;
+            v[1] += ri * ri;
+          }
+        }
       }
       if (!local_total<2, CL>(v, n_own, nb, blk, a.part, epoch, a.err, S, C, [&](const double* tot) {
             PState& T = S.st;
@@ -782,8 +895,8 @@ __device__ __forceinline__ void pcg_local_body(const PArgs& a, int nb, int blk, 
         // x += xs; then the FP64 true residual replaces the recurrence's
         const bool slow = S.act & 4;
         for (int i = tid; i < n_own; i += LT) {
-          a.x[e0 + i] += (double)s_xs[i];
-          s_xs[i] = (X)0;
+          a.x[e0 + i] += (double)w_xs[i];
+          w_xs[i] = (X)0;
         }
         const float w[1] = {0.0f};
         if (!local_total<1, CL>(w, 1, nb, blk, a.part, epoch, a.err, S, C, none)) return;
@@ -832,13 +945,13 @@ __device__ __forceinline__ void pcg_local_body(const PArgs& a, int nb, int blk, 
   }
   if (!RELIABLE && S.st.done)
     for (int i = tid; i < n_own; i += LT) {
-      a.x[e0 + i] += (double)s_xs[i];
-      s_xs[i] = (X)0;
+      a.x[e0 + i] += (double)w_xs[i];
+      w_xs[i] = (X)0;
     }
   if (!S.st.done)
     for (int i = tid; i < n_own; i += LT) {
       r[e0 + i] = s_r[i];
-      xs[e0 + i] = s_xs[i];
+      if constexpr (!SL) xs[e0 + i] = s_xs[i];
       p[e0 + i] = s_po[i];
     }
   if (blk == 0 && tid == 0) {

@@ -54,43 +54,6 @@ static void launch_pdl(Ctx* ctx, void (*kern)(KArgs...), unsigned grid, cudaStre
   cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
 }
 
-// CHUNK iterations of a CG loop, captured once into a CUDA graph and
-// replayed for every chunk: one graph launch instead of about five kernel
-// launches per iteration (the programmatic-launch edges between the kernels
-// are kept by the capture; every launch argument is a device pointer or a
-// size fixed for the solve).  When the capture or the instantiation fails
-// (e.g. on the legacy default stream), the chunk runs as direct launches.
-struct ChunkGraph {
-  cudaGraphExec_t exec = nullptr;
-  bool tried = false;
-  ChunkGraph() = default;
-  ChunkGraph(const ChunkGraph&) = delete;
-  ChunkGraph& operator=(const ChunkGraph&) = delete;
-  ~ChunkGraph() {
-    if (exec) cudaGraphExecDestroy(exec);
-  }
-  template <class F>
-  int run(Ctx* ctx, cudaStream_t s, F&& body) {
-    if (!tried) {
-      tried = true;
-      cudaGraph_t g = nullptr;
-      if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
-        const int rc = body();
-        const cudaError_t e = cudaStreamEndCapture(s, &g);
-        if (rc == GT_OK && e == cudaSuccess && g && cudaGraphInstantiate(&exec, g, 0) != cudaSuccess) exec = nullptr;
-        if (g) cudaGraphDestroy(g);
-      }
-      cudaGetLastError();  // a failed capture leaves its error here; the direct path follows
-    }
-    if (exec) {
-      GT_CUDA(ctx, cudaGraphLaunch(exec, s));
-      ctx->graph_launches++;
-      return GT_OK;
-    }
-    return body();
-  }
-};
-
 // device-resident CG state (one per solve)
 struct CGState {
   double rz, pq, rr, bb, alpha, beta;
@@ -527,7 +490,7 @@ __global__ void k_sell_fill(const int64_t* __restrict__ rowptr, const int32_t* _
     b = rowptr[r];
     e = rowptr[r + 1];
   }
-  const int32_t pad = r < nrows ? (int32_t)r : 0;
+  const int32_t pad = (int32_t)(r < nrows ? r : nrows - 1);  // a column near the slice's own
   const int L = slen[sl];
   const int64_t o = sptr[sl] + lane;
   for (int k = 0; k < L; k++) {
@@ -1099,6 +1062,16 @@ static int pcg_reliable(Matrix* A, const V* val, const double* b, double* x, dou
   return status;
 }
 
+int sell_ready(Matrix* A, bool f64, bool f32, bool* ok) {
+  SellView<double> v64;
+  SellView<float> v32;
+  *ok = false;
+  if (f64) GT_TRY(sell_prepare(A, A->val64, &v64));
+  if (f32) GT_TRY(sell_prepare(A, A->val32, &v32));
+  *ok = (!f64 || v64.val) && (!f32 || v32.val);
+  return GT_OK;
+}
+
 int spmv64(Matrix* A, const double* x, double* y) {
   Ctx* ctx = A->space->mesh->ctx;
   if (!A->val64) return set_error(ctx, GT_ERR_INVALID, "matrix has no FP64 values");
@@ -1162,10 +1135,20 @@ int solve(Matrix* A, const double* b, double* x, double rtol, int maxit, int mod
   // the persistent kernel saves the per-phase launches and grid-wide
   // reduction tails that dominate small systems; large systems keep more
   // loads in flight with one launch per phase (measured crossover)
-  const bool persistent = ctx->pcg_path == 2 || (ctx->pcg_path == 0 && n <= kPersistentMaxRows);
+  bool persistent = ctx->pcg_path == 2 || (ctx->pcg_path == 0 && n <= kPersistentMaxRows);
+  int32_t it = 0, nupd = 0, it64 = 0;
   if (persistent) {
-    int32_t it = 0, nupd = 0, it64 = 0;
     status = pcg_persistent(A, mode, b, x, rtol, maxit, &it, &nupd, &it64, &inf.rel_residual);
+  } else if (ctx->pcg_path == 0 && A->bs == 1) {
+    // larger scalar systems: the persistent kernel on the sliced copy, as long
+    // as a CTA's local sets fit in shared memory.  Measured, us a solve, one
+    // launch per phase / sliced: P1 tetrahedra 79^3 rows FP64 22500 / 15670,
+    // mixed 15720 / 9570; 69^3 rows 16640 / 9890, 11610 / 6840
+    status = pcg_persistent(A, mode, b, x, rtol, maxit, &it, &nupd, &it64, &inf.rel_residual, true);
+    persistent = status != kPcgNoFit;
+    if (!persistent) status = GT_OK;
+  }
+  if (persistent) {
     if (status != GT_OK && status != GT_ERR_NOT_CONVERGED) return status;
     inf.iterations = it;
     inf.outer_iterations = mode == GT_SOLVE_FP32 ? 0 : nupd;

@@ -1,6 +1,6 @@
 """The persistent solver on CTA-local vectors (csrc/gt_pcg_local.cuh) at the
 edges of its placements: one row, fewer rows than CTAs, one cluster, a grid,
-block rows of 1, 2 and 3, and a numbering whose local sets do not fit in
+the sliced form, block rows of 1, 2 and 3, and a numbering whose local sets do not fit in
 shared memory (solved by the kernel on global vectors).
 
 The solver stops when its FP64 residual is at most rtol ||b||.  The same
@@ -51,6 +51,20 @@ def _check(A, b, x):
 ])
 def test_residual_at_the_edges(cell, order, ncomp, n, T, mode):
     A, b = _system(cell, order, ncomp, n, T)
+    x, info = GT.solve(A, b, rtol=RTOL, mode=mode)
+    assert info["converged"]
+    _check(A, b, x)
+    again, _ = GT.solve(A, b, rtol=RTOL, mode=mode)
+    assert np.array_equal(x, again)
+
+
+@pytest.mark.parametrize("T,mode", [(np.float64, "fp64"), ("mixed", "ir")])
+@pytest.mark.parametrize("cell,n", [("quad", 514), ("hex", 66), ("tet", 66)])
+def test_sliced_form(cell, n, T, mode):
+    """Scalar systems above 262,144 rows, streamed from the sliced copy; the
+    row counts (513^2, 65^3) leave one row in the last slice of 32."""
+    A, b = _system(cell, 1, 1, n, T)
+    assert A.shape[0] > 262144 and A.shape[0] % 32 == 1
     x, info = GT.solve(A, b, rtol=RTOL, mode=mode)
     assert info["converged"]
     _check(A, b, x)
