@@ -2588,8 +2588,10 @@ __global__ void k_kref(const double* __restrict__ gref, Tables1D tab, T lamf, T 
     for (int dd = 0; dd < BS; dd++) kref[(size_t)ab * BS * BS + cc * BS + dd] = blk[cc][dd];
 }
 
+// (Q2 elasticity 32^3 FP64: 945 us without the loads ahead, 799 with them; FP32
+// values need two CTAs of 512 threads on an SM, so at most 64 registers.)
 template <int D, int ORDER, int BS, int G, class T, bool LIFT>
-__global__ void k_scatter_uniform(const int64_t* __restrict__ rowptr, const int32_t* __restrict__ colind,
+__global__ void __launch_bounds__(512, sizeof(T) == sizeof(float) ? 2 : 1) k_scatter_uniform(const int64_t* __restrict__ rowptr, const int32_t* __restrict__ colind,
                                   const int64_t* __restrict__ inc_ptr, const int32_t* __restrict__ inc,
                                   const int32_t* __restrict__ cnd, int64_t nrows, int lmax,
                                   const T* __restrict__ kref, const double* __restrict__ gref,
@@ -2616,45 +2618,77 @@ __global__ void k_scatter_uniform(const int64_t* __restrict__ rowptr, const int3
   const unsigned gmask = (G == 32) ? 0xffffffffu : (((1u << G) - 1u) << (sub * G));
   const bool vec = be != nullptr && gl == 0;
   const int b = gl;
-  const int64_t nblk = (nrows + (int64_t)nw * RPW - 1) / ((int64_t)nw * RPW);
-  for (int64_t blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
-    const int64_t r = (blk * nw + w) * RPW + sub;
-    if (r >= nrows) continue;  // the group's lanes all skip together
-    const int64_t rb = rowptr[r];
-    const int L = (int)(rowptr[r + 1] - rb);
-    for (int i = gl; i < L; i += G) cols[i] = colind[rb + i];
+  // A row's inputs are a chain of dependent loads (row pointers, incidences,
+  // their cells' DOFs and scales), four latencies that the few warps beside
+  // the row slots cannot hide; the next row's are loaded a step at a time
+  // while the current row is summed.  (FP32 values: twice the warps fit, if they
+  // keep to 64 registers, and hide them better: 46 us on 15^3 Q2 elasticity,
+  // 53 with the loads ahead, which spill.)
+  constexpr bool AHEAD = sizeof(T) == sizeof(double);
+  // lane k < nin: incidence k and its scale |det J| coef_c (formed by one lane
+  // and handed to the group by shuffles: a conversion per lane would load the
+  // FP64 pipe, which also converts FP64 to FP32)
+  const int64_t stride = (int64_t)gridDim.x * nw * RPW;
+  int64_t r = ((int64_t)blockIdx.x * nw + w) * RPW + sub;
+  int64_t rb = 0, re = 0, ib = 0, ie = 0;
+  int32_t my_cb = 0, jk[PF];
+  double my_cf = 1.0;
+  auto load_ptrs = [&](int64_t q, int64_t& rb_, int64_t& re_, int64_t& ib_, int64_t& ie_) {
+    if (q < nrows) {
+      rb_ = __ldg(rowptr + q);
+      re_ = __ldg(rowptr + q + 1);
+      ib_ = __ldg(inc_ptr + q);
+      ie_ = __ldg(inc_ptr + q + 1);
+    } else {
+      rb_ = re_ = ib_ = ie_ = 0;
+    }
+  };
+  auto load_inc = [&](int64_t ib_, int64_t ie_) -> int32_t { return gl < ie_ - ib_ ? __ldg(inc + ib_ + gl) : 0; };
+  // the column DOFs of the first PF incidences' nodes b = gl and the scales;
+  // later incidences (a node in more than PF cells) load in the loop
+  auto load_cells = [&](int nin_, int32_t cb_, int32_t (&j_)[PF], double& cf_) {
+    cf_ = (coef && gl < nin_) ? __ldg(coef + cb_ / NN) : 1.0;
+#pragma unroll
+    for (int k = 0; k < PF; k++) {
+      const int32_t c = __shfl_sync(gmask, cb_, k, G) / NN;
+      j_[k] = (k < nin_ && b < NN) ? __ldg(cnd + (int64_t)c * NN + b) : 0;
+    }
+  };
+  load_ptrs(r, rb, re, ib, ie);
+  my_cb = load_inc(ib, ie);
+  load_cells((int)(ie - ib), my_cb, jk, my_cf);
+  while (r < nrows) {  // the group's lanes leave together
+    const int64_t rn = r + stride;
+    int64_t rbn, ren, ibn, ien;
+    if (AHEAD) load_ptrs(rn, rbn, ren, ibn, ien);
+    const int L = (int)(re - rb), nin = (int)(ie - ib);
+    for (int i = gl; i < L; i += G) cols[i] = __ldg(colind + rb + i);
     for (int i = gl; i < L * KB; i += G) acc[i] = (T)0;
     __syncwarp(gmask);
     double bsum[BS];
-    const int64_t ib = inc_ptr[r], ie = inc_ptr[r + 1];
     if (be != nullptr) {
       row_load_sum<BS, G>(ib, ie, inc, NN, be, gl, gmask, bsum);
     } else {
 #pragma unroll
       for (int cc = 0; cc < BS; cc++) bsum[cc] = 0.0;
     }
-    // the row's first PF incidences (at most 2^D on a structured mesh) are
-    // fetched up front: their cells, each lane's column DOF and the cells'
-    // scales are loads in flight together, and the column positions are
-    // independent searches, so the summation loop below waits on no global
-    // load; later incidences (a node in more than PF cells) load in the loop
-    const int nin = (int)(ie - ib);
-    const int32_t my_cb = gl < nin ? __ldg(inc + ib + gl) : 0;
-    // each incidence's scale |det J| coef_c computed by one lane and handed
-    // to the group by shuffles (a conversion per lane would load the FP64
-    // pipe, which also converts FP64 to FP32)
-    const T my_sc = (T)(adet * ((coef && gl < nin) ? __ldg(coef + my_cb / NN) : 1.0));
-    int32_t cbk[PF], jk[PF], pk[PF];
+    int32_t cbn;
+    if (AHEAD) cbn = load_inc(ibn, ien);
+    const T my_sc = (T)(adet * my_cf);
+    int32_t cbk[PF], pk[PF];
     T sck[PF];
 #pragma unroll
     for (int k = 0; k < PF; k++) {
       cbk[k] = __shfl_sync(gmask, my_cb, k, G);
-      const int32_t c = cbk[k] / NN;
-      jk[k] = (k < nin && b < NN) ? __ldg(cnd + (int64_t)c * NN + b) : 0;
       sck[k] = __shfl_sync(gmask, my_sc, k, G);
     }
+    // the column positions are independent searches: the summation loop
+    // below waits on no load
 #pragma unroll
     for (int k = 0; k < PF; k++) pk[k] = jk[k] > 0 ? find_col(cols, L, jk[k] - 1) : -1;
+    int32_t jkn[PF];
+    double cfn;
+    if (AHEAD) load_cells((int)(ien - ibn), cbn, jkn, cfn);
     // incidence cb's block: row node a, this lane's column node b (column
     // DOF j, position p), scale sc; then the group barrier that keeps the
     // summation order
@@ -2710,6 +2744,20 @@ __global__ void k_scatter_uniform(const int64_t* __restrict__ rowptr, const int3
 #pragma unroll
       for (int cc = 0; cc < BS; cc++) bvec[r * BS + cc] = bsum[cc];
     __syncwarp(gmask);  // the row slot is reused by the group's next row
+    if (!AHEAD) {
+      load_ptrs(rn, rbn, ren, ibn, ien);
+      cbn = load_inc(ibn, ien);
+      load_cells((int)(ien - ibn), cbn, jkn, cfn);
+    }
+    r = rn;
+    rb = rbn;
+    re = ren;
+    ib = ibn;
+    ie = ien;
+    my_cb = cbn;
+    my_cf = cfn;
+#pragma unroll
+    for (int k = 0; k < PF; k++) jk[k] = jkn[k];
   }
 }
 
@@ -2960,7 +3008,7 @@ __global__ void k_expand_rowptr(const int64_t* rowptr, int64_t nbrows, int bs, i
 // (BS x BS blocks in, BS scalar rows out), a lane copies component d of every
 // scalar row of a block, so each column and each input line is read once.
 // Bound by HBM (2 values + BS columns a block entry).  Measured, Q2
-// elasticity 32^3 (156M scalar entries FP64): 787 -> 716 us (4.2 TB/s), 15^3
+// elasticity 32^3 (156M scalar entries FP64): 787 -> 649 us (4.6 TB/s), 15^3
 // (16M): 71 -> 37 us.
 template <class V, int BS>
 __global__ void __launch_bounds__(256) k_expand_entries(const int64_t* __restrict__ rowptr,
@@ -2977,7 +3025,7 @@ __global__ void __launch_bounds__(256) k_expand_entries(const int64_t* __restric
     V v[BS];
     if (oval)
 #pragma unroll
-      for (int c = 0; c < BS; c++) v[c] = __ldcs(vals + o + (int64_t)k * (BS * BS) + c * BS + d);
+      for (int c = 0; c < BS; c++) v[c] = __ldg(vals + o + (int64_t)k * (BS * BS) + c * BS + d);
     const int32_t col = ocol ? __ldg(colind + b + k) * BS + d : 0;
 #pragma unroll
     for (int c = 0; c < BS; c++) {
