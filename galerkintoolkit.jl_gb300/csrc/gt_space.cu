@@ -222,14 +222,20 @@ struct HashBuf {
 // the instances that first met one, and the parents' count -- what the id of
 // any face follows from (slot_id)
 struct FaceNumbers {
+  Ctx* ctx = nullptr;
   HashBuf hb;
   int32_t* pos = nullptr;
   int32_t npar = 0;
   int64_t nd = 0;
-  void release(Ctx* ctx) {
+  void release() {
+    if (!ctx) return;
     hb.release(ctx);
     dfree(ctx, pos);
   }
+  FaceNumbers() = default;
+  FaceNumbers(const FaceNumbers&) = delete;
+  FaceNumbers& operator=(const FaceNumbers&) = delete;
+  ~FaceNumbers() { release(); }
 };
 
 // Numbers the d-faces of nf higher-dimensional faces (see file header).
@@ -238,6 +244,7 @@ struct FaceNumbers {
 static int number_faces(Ctx* ctx, const int32_t* fverts, int64_t nf, int nlv, int nld, int ndv, const LocalFaces& ld,
                         const int32_t* pverts, int64_t npar, int32_t* inst_ids, int32_t** dverts_out, FaceNumbers* F) {
   int64_t ninst = nf * nld;
+  F->ctx = ctx;
   int s = F->hb.alloc(ctx, npar + ninst);
   const Hash h = F->hb.h;
   F->npar = (int32_t)npar;
@@ -549,8 +556,8 @@ int number_dofs(Space* sp, int ngroups, const int32_t* groups_host) {
     dfree(ctx, keep);
     dfree(ctx, dgroups);
   }
-  FN.release(ctx);
-  EN.release(ctx);
+  FN.release();
+  EN.release();
   GT_TRY(dalloc(ctx, &dpos, nnodes_sp + 1));
   GT_TRY(exclusive_scan_i32(ctx, tag, dpos, nnodes_sp));
   k_renumber<<<GT_KC(ctx, grid_for(nc * t.nn, 256)), 256, 0, st>>>(sp->cell_ndofs, nc * t.nn, tag, dpos);
