@@ -587,8 +587,8 @@ __device__ __forceinline__ void thread_sort(int32_t* v) {
 
 // The count pass with one thread per block row, for rows of at most 32
 // incidences and 32 columns (P1 tetrahedra, Q1 quadrilaterals and hexahedra):
-// the thread sorts its incidences by insertion and builds its sorted column
-// list by binary search and insertion, both in shared memory interleaved
+// the thread sorts its incidences and builds its sorted column list by a hash
+// table (NN = 4) or by binary search and insertion, in shared memory interleaved
 // across the block's threads (element k of thread t at k * blockDim + t).
 // A row with more than 32 incidences or 32 columns sets *redo.  With bucket
 // the incidences are read from the row's bucket (k_inc_place) and the
@@ -600,7 +600,7 @@ __device__ __forceinline__ void thread_sort(int32_t* v) {
 // *redo the warp kernel recounts every row.
 // C16: the space's DOF spread is below 2^15, so every column differs from
 // its row by less than 2^15 and the list holds column - row in 16 bits:
-// 192 instead of 256 bytes of shared memory per thread, 9 instead of 6
+// 192 instead of 256 bytes of shared memory per thread, up to 9 instead of 6
 // blocks per SM (the pass is bound by shared-memory latency, not bandwidth).
 constexpr int kRowsMI = 32, kRowsS = 32;
 static_assert(kIncBucket == kRowsMI, "a bucket holds the incidences the row-per-thread pass takes");
@@ -617,6 +617,16 @@ __global__ void __launch_bounds__(128) k_pattern_rows(const int64_t* __restrict_
   CT* Cl = reinterpret_cast<CT*>(s_rows + kRowsMI * T) + tid;     // columns (- row with C16), Cl[k * T]
   const int64_t r = blockIdx.x * (int64_t)T + tid;
   const int32_t cbase = C16 ? (int32_t)r : 0;
+  // NN = 4: the columns in an open-addressing table of kRowsS entries, sorted
+  // in registers at the end -- a candidate then costs one or two dependent
+  // shared-memory accesses instead of a binary search and the shift of an
+  // insertion (96^3 x 6 P1 tetrahedra, 15 columns of 72 candidates: 256 us, 177
+  // here, at 7 blocks per SM; capped to the registers of 8 or 9, 212).  Q1
+  // hexahedron rows (27 columns) would fill it
+  constexpr bool HASH = NN == 4;
+  constexpr int32_t kEmpty = C16 ? -32768 : INT_MIN;  // no column: offsets are above -2^15, ids not negative
+  if constexpr (HASH)
+    for (int k = 0; k < kRowsS; k++) Cl[k * T] = (CT)kEmpty;
   if (r >= nrows) return;
   const int64_t ib = inc_ptr[r];
   const int ninc = (int)(inc_ptr[r + 1] - ib);
@@ -661,8 +671,11 @@ __global__ void __launch_bounds__(128) k_pattern_rows(const int64_t* __restrict_
   for (int k = 0; k < ninc; k++) inc[ib + k] = I[k * T];
   int n = 0;
   bool over = false;
+  auto slot_of = [](int32_t key) { return (int)(((unsigned)key * 2654435761u) >> 27); };
+  static_assert(kRowsS == 32, "five bits of the hash");
   if (ninc > 0) {
-    Cl[0] = (CT)((int32_t)r - cbase);  // the row's own DOF (block row r is node r + 1)
+    // the row's own DOF (block row r is node r + 1)
+    Cl[(HASH ? slot_of((int32_t)r - cbase) : 0) * T] = (CT)((int32_t)r - cbase);
     n = 1;
   }
   // the next incidence's node DOFs are loaded while the current ones are
@@ -706,6 +719,21 @@ __global__ void __launch_bounds__(128) k_pattern_rows(const int64_t* __restrict_
         for (int q = 0; q < NN; q++) known |= prev[u][q] == d[b];
       if (known) continue;
       const int32_t key = d[b] - 1 - cbase;
+      if constexpr (HASH) {
+        int h = slot_of(key), probe = 0;
+        int32_t at = Cl[h * T];
+        while (at != key && at != kEmpty && ++probe < kRowsS) {
+          h = (h + 1) & (kRowsS - 1);
+          at = Cl[h * T];
+        }
+        if (at == kEmpty) {
+          Cl[h * T] = (CT)key;
+          n++;
+        } else if (at != key) {
+          over = true;  // kRowsS other columns
+        }
+        continue;
+      }
       int lo = 0, hi = n;
       while (lo < hi) {
         const int mid = (lo + hi) >> 1;
@@ -738,7 +766,23 @@ __global__ void __launch_bounds__(128) k_pattern_rows(const int64_t* __restrict_
   }
   rowcnt[r] = n;
   small[r] = 1;
-  for (int k = 0; k < n; k++) slots[r * kRowsS + k] = (int32_t)Cl[k * T] + cbase;
+  if constexpr (HASH) {
+    int32_t v[kRowsS];
+#pragma unroll
+    for (int k = 0; k < kRowsS; k++) {
+      const int32_t at = Cl[k * T];
+      v[k] = at == kEmpty ? INT_MAX : at;
+    }
+    thread_sort<kRowsS>(v);
+    int4* out = reinterpret_cast<int4*>(slots + r * kRowsS);
+#pragma unroll
+    for (int q = 0; q < kRowsS / 4; q++)
+      if (4 * q < n)  // (entries past n are not read)
+        out[q] = make_int4((int)((unsigned)v[4 * q] + cbase), (int)((unsigned)v[4 * q + 1] + cbase),
+                           (int)((unsigned)v[4 * q + 2] + cbase), (int)((unsigned)v[4 * q + 3] + cbase));
+  } else {
+    for (int k = 0; k < n; k++) slots[r * kRowsS + k] = (int32_t)Cl[k * T] + cbase;
+  }
   if (n > __ldcg(maxrow)) atomicMax(maxrow, n);
 }
 

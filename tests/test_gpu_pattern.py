@@ -1,7 +1,8 @@
 """The warp-per-row sparsity pass at its edges, on fans of 2n P2 tetrahedra
 around one node: its row holds 5n + 5 columns of 20n candidates.  n = 5 .. 25
 cross the register sorts (32, 64, 128 columns, then shared memory and the fill
-pass), n = 13 the candidates the first launch has room for."""
+pass), n = 13 the candidates the first launch has room for.  The thread-per-row pass at its
+column limit, on P1 tetrahedra that share little more than one node."""
 import numpy as np
 import pytest
 
@@ -26,3 +27,30 @@ def test_fan_rows(n):
     orp, oci, ov = O.csc_to_csr(cp, rv, nz, ref["nfree"])
     assert np.array_equal(rp, orp) and np.array_equal(ci, oci)
     assert np.abs(v - ov).max() <= TOL64 * np.abs(ov).max()
+
+
+@pytest.mark.parametrize("disjoint,extra", [(1, 0), (5, 0), (9, 0), (10, 0), (10, 1), (10, 2), (11, 0)])
+def test_bouquet_rows(disjoint, extra):
+    """Tetrahedra around node 1: 3 new nodes each, 1 for each extra one (it
+    shares a face's edge with the first) -- 3 * disjoint + extra + 1 columns of
+    the 32 the row-per-thread pass holds; 33 and 34 are recounted."""
+    from gtgpu.mesh import Mesh
+    rng = np.random.default_rng(disjoint * 10 + extra)
+    n = 1 + 3 * disjoint + extra
+    coords = np.vstack([[0.0, 0.0, 0.0], rng.uniform(-1.0, 1.0, (n - 1, 3))])
+    cells = [[1, 2 + 3 * i, 3 + 3 * i, 4 + 3 * i] for i in range(disjoint)]
+    cells += [[1, 2, 3, 2 + 3 * disjoint + j] for j in range(extra)]
+    m = Mesh(D=3, cell_type=GT.api._lib.GT_TET4, coords=coords, cell_nodes=np.asarray(cells, np.int32),
+             corners=np.zeros(0, np.int32), bfaces=np.zeros((0, 3), np.int32), bface_group=np.zeros(0, np.int32),
+             bedges=np.zeros((0, 2), np.int32))
+    V = GT.lagrange_space(GT.interior(m), 1)
+    rp, ci, v = GT.assemble_matrix(GT.mass(), np.float64, V).csr()
+    dofs = V.face_dofs()
+    pairs = sorted({(a, b) for c in dofs for a in c for b in c})
+    assert np.array_equal(ci + 1, [b for _, b in pairs])
+    assert np.array_equal(np.diff(rp), np.bincount([a - 1 for a, _ in pairs], minlength=n))
+    assert np.diff(rp).max() == n
+    # the entries of the mass matrix add up to the volume (positive terms)
+    J = coords[np.asarray(cells) - 1][:, 1:] - coords[np.asarray(cells) - 1][:, :1]
+    vol = np.abs(np.linalg.det(J)).sum() / 6.0
+    assert abs(v.sum() - vol) <= 1e-12 * vol
