@@ -1,10 +1,11 @@
 """Batched assembly + solve of many independent problems.
 
 ``Batch`` wraps ``gt_batch_*`` (scalar matrices, or block size 3 for 3-D
-elasticity): the small instances (up to 32768 scalar rows) are
-solved by one persistent launch in which every CTA takes instances from a
-queue (largest first) and runs each one's whole Jacobi-PCG alone; the large
-instances run through the single-system solver.  Each instance keeps its own
+elasticity): of the small instances (up to 32768 scalar rows) those up to
+1024 rows are solved by one persistent launch in which every CTA takes
+instances from a queue (largest first) and runs each one's whole Jacobi-PCG
+alone, the others by one thread-block cluster each; the large instances run
+through the single-system solver.  Each instance keeps its own
 CG scalars and a summation order that depends only on the instance.
 ``run_batch`` drives a whole batch: HBM-budgeted waves, several worker
 contexts assembling instances concurrently and solving the large ones on
@@ -64,8 +65,8 @@ class Batch:
         check(self.ctx.h, self.ctx.lib.gt_batch_set_lanes(self.h, int(lanes)))
 
     def set_small_rows(self, rows: int):
-        """scalar rows up to which an instance is solved by one CTA (at most
-        32768); larger instances of the batch's own context, up to 262,144
+        """scalar rows up to which an instance belongs to the small tier (one
+        CTA up to 1024 rows, one cluster above; at most 32768); larger instances of the batch's own context, up to 262,144
         rows, share grouped persistent launches (FP64 and mixed modes)"""
         check(self.ctx.h, self.ctx.lib.gt_batch_set_small_rows(self.h, int(rows)))
 
@@ -239,8 +240,8 @@ def run_batch(specs, inputs, precision="mixed", rtol=1e-10, maxit=100000, worker
     single-system solver on the worker's stream, so several such solves and
     the other workers' assembly run on the device together; the smaller
     instances wait for the wave's small tier: one gt_batch over all of them,
-    solved by one persistent launch in which each CTA runs whole instances
-    from a largest-first queue.  Every instance's arithmetic depends only on
+    solved by one persistent launch in which each CTA (above 1024 rows each
+    cluster of CTAs) runs whole instances, largest first.  Every instance's arithmetic depends only on
     the instance, so its result is bitwise the same whatever the batch.
 
     inputs: {index: (mesh, kappa)} (instance_inputs).  precision "mixed"
@@ -323,8 +324,8 @@ def run_batch(specs, inputs, precision="mixed", rtol=1e-10, maxit=100000, worker
 def autotune_batch(specs, inputs, precision="mixed", rtol=1e-10, workers=(1, 2, 4, 8), sample=48, max_rows=2_000_000,
                    cache=None, use_cache=True, seed=0, small_rows=(4096, 16384, 32768)):
     """Pick run_batch's concurrency (worker contexts), the row limit of its
-    one-CTA-per-instance tier (the tile of the batched kernel: an instance
-    up to it is solved by one CTA, a larger one by the whole device) and
+    small tier (an instance up to it is solved by one CTA or one cluster, a
+    larger one by the whole device) and
     the small tier's SpMV lanes for a workload: run_batch is timed on a
     seeded sample of the instances (at most ``sample``, each under
     ``max_rows`` rows, spread over the size range) once per worker count,

@@ -27,11 +27,11 @@ Continuous batching: a slot that takes a request of at most ``batch_rows``
 scalar rows (Poisson or elasticity; by default 2,048) also takes the other
 such requests pending at that moment (up to ``batch_max``, within the
 budget) and solves them together with ``gt_batch``: those up to
-``small_rows`` rows one CTA each in one persistent launch per block size,
+``small_rows`` rows one CTA or one cluster each in shared launches per block size,
 larger ones (when ``batch_rows`` admits them) in shared grouped persistent
 launches, each on the CTAs its own solve would use.  So a stream of small
 requests is not served one grid-wide solve at a time, and a request's result
-never depends on its batch: the one-CTA tier's depends on the request alone,
+never depends on its batch: the small tier's depends on the request alone,
 the grouped tier's is bitwise that of the request's own solve.
 
 ``request_stream`` draws the seeded request mix of the serving benchmark:
@@ -263,8 +263,8 @@ def run_request(req: Request, ctx: Context, precision="mixed", rtol=1e-8, keep_s
 def run_batch_requests(reqs, ctx: Context, precision="mixed", rtol=1e-8, keep_solution=True, cache=None,
                        library=None, small_rows=2048):
     """Assemble (or refill) several requests on ctx and solve them together
-    (gt_batch): those up to small_rows scalar rows one CTA each in one
-    persistent launch per block size, the larger ones in grouped persistent
+    (gt_batch): those up to small_rows scalar rows one CTA or one cluster each
+    in shared launches per block size, the larger ones in grouped persistent
     launches (each on the CTAs its own solve would use)."""
     from .batch import Batch
     library = library or MeshLibrary()
@@ -296,7 +296,7 @@ class Server:
         # requests up to batch_rows scalar rows go through gt_batch (alone
         # or with others, up to batch_max); batching=False: one grid-wide
         # solve per request.  In a batch, requests up to small_rows are
-        # solved by one CTA each, so that tier lasts as long as its largest
+        # solved by one CTA or one cluster each, so that tier lasts as long as its largest
         # member: the limit keeps it short (on GB300, under the 2000 req/s
         # stream, 2048 scalar rows and batches of 16 completed 1.8x the
         # requests of 32768 and 64 at a p50 of 10 ms instead of 0.4 s); the
@@ -305,7 +305,7 @@ class Server:
         # 262,144: 588 requests/s at a p50 of 138 ms against 604 at 9.3 ms
         # (a batch then waits for its grouped launches, and requests of one
         # geometry in one batch each need their own resident instance), so
-        # by default only the one-CTA requests are batched
+        # by default only the small requests are batched
         self.batching = batching and runner is None
         self.batch_max = max(1, batch_max)
         self.batch_rows = batch_rows
