@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(256) k_elements_hex(const double* __restrict__
     const double det = J[0][0] * A[0][0] + J[0][1] * A[1][0] + J[0][2] * A[2][0];
     if (c < ncells && !(det != 0.0)) atomicOr(err, DEV_ERR_DEGENERATE);
     const double w = line.w[q1] * line.w[q2] * line.w[q3], adet = fabs(det);
-    s_dv[cl][q] = adet * w;
+    s_dv[cl][q] = (double)(T)(adet * w);  // |det J| w is held in T, also for the element vector
     const double cf = (coef && c < ncells ? coef[c] : 1.0) * w * recip_nr2(adet);
     auto dot = [&](int k, int l) { return cf * (A[k][0] * A[l][0] + A[k][1] * A[l][1] + A[k][2] * A[l][2]); };
     s_D[cl][0][q] = (T)dot(0, 0);
@@ -355,8 +355,21 @@ __global__ void __launch_bounds__(128) k_elements_p2(const double* __restrict__ 
     }
   }
   if (be && c < ncells) {
-    // integrals of the shape functions: -1/120 (vertex), 1/30 (edge)
-    const double s = adet * (scoef ? scoef[c] : 1.0) * fsrc[0] * (1.0 / 30.0), sv = -0.25 * s;
+    // integrals of the shape functions: -1/120 (vertex), 1/30 (edge).  FP32
+    // matrices hold |det J| w at the points of the 11-point rule in FP32, as
+    // k_elements does: with its three weights the sums over the points are
+    // those of the shape functions over the rule's three orbits
+    const double cf = (scoef ? scoef[c] : 1.0) * fsrc[0];
+    double s, sv;
+    if constexpr (sizeof(T) == 4) {
+      const double d0 = (double)(T)(adet * (-74.0 / 5625.0)), d1 = (double)(T)(adet * (343.0 / 45000.0)),
+                   d2 = (double)(T)(adet * (56.0 / 2250.0));
+      s = cf * (0.25 * d0 + (24.0 / 49.0) * d1 + (37.0 / 28.0) * d2);
+      sv = cf * (-0.125 * d0 + (13.0 / 49.0) * d1 - (27.0 / 56.0) * d2);
+    } else {
+      s = adet * cf * (1.0 / 30.0);
+      sv = -0.25 * s;
+    }
     double* b = be + c * 10;
 #pragma unroll
     for (int i = 0; i < 4; i++) b[V[i]] = sv;

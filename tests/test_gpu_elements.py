@@ -45,3 +45,45 @@ def test_laplacian_blocks(cells, simplex, order):
     M = sp.csr_matrix((v, ci, rp))
     assert np.abs(M @ np.ones(M.shape[0])).max() <= 2e-12 * scale
     assert abs(M - M.T).max() <= 2e-13 * scale
+
+
+def test_fp32_point_weights_of_the_load_vector_p2():
+    # |det J| w is held in the matrix's type.  The shape functions sum to one at
+    # every point, so the load vector of f = 1 sums to the cells' rounded point
+    # weights.  det J is the product of differences of rounded coordinates (a
+    # few eps off the cell volume; a point's rounding to FP32 changes for it
+    # with probability ~1e-8), the sum is exact to n eps: 1e-13 against the
+    # 1e-9 and more that the rounding to FP32 moves it.
+    cells = (3, 5, 7)
+    m = GT.cartesian_mesh((0.0, 1.0, 0.0, 1.0, 0.0, 1.0), cells, simplexify=True)
+    V = GT.lagrange_space(GT.interior(m), 2)
+    w = np.repeat([-74 / 5625, 343 / 45000, 56 / 2250], [1, 4, 6])
+    want = m.num_cells * (w / np.prod(cells)).astype(np.float32).astype(np.float64).sum()
+    assert abs(want - 1.0) > 1e-10
+    _, b = GT.assemble_matrix_and_vector(GT.laplacian(None), GT.source(1.0), np.float32, V)
+    assert abs(np.asarray(b, np.float64).sum() - want) <= 1e-13
+
+
+@pytest.mark.parametrize("order", [1, 2])
+def test_fp32_point_weights_of_the_load_vector_hex(order):
+    # the same on distorted hexahedra (parallel ones take the factored path,
+    # whose weights are FP64), det J from the trilinear map's gradients
+    m = GT.cartesian_mesh((0.0, 1.0, 0.0, 1.0, 0.0, 1.0), (3, 5, 7))
+    m.coords += np.random.default_rng(5).uniform(-0.02, 0.02, m.coords.shape)
+    V = GT.lagrange_space(GT.interior(m), order)
+    x1, w1 = np.polynomial.legendre.leggauss(order + 1)
+    x1, w1 = 0.5 + 0.5 * x1, 0.5 * w1
+    X = m.coords[m.cell_nodes.astype(np.int64) - 1]
+    want = exact = 0.0
+    for q in np.ndindex(order + 1, order + 1, order + 1):
+        g = np.empty((8, 3))
+        for v in range(8):
+            for d in range(3):
+                g[v, d] = np.prod([((1 if v >> t & 1 else -1) if t == d else (x1[q[t]] if v >> t & 1 else 1 - x1[q[t]]))
+                                   for t in range(3)])
+        dv = np.abs(np.linalg.det(np.einsum("cvi,vj->cij", X, g))) * w1[q[0]] * w1[q[1]] * w1[q[2]]
+        want += dv.astype(np.float32).astype(np.float64).sum()
+        exact += dv.sum()
+    assert abs(want - exact) > 1e-11
+    _, b = GT.assemble_matrix_and_vector(GT.laplacian(None), GT.source(1.0), np.float32, V)
+    assert abs(np.asarray(b, np.float64).sum() - want) <= 1e-13
