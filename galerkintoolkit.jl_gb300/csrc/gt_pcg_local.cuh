@@ -100,11 +100,14 @@ __device__ __forceinline__ Fx fx_norm(Fx f) {
 __device__ __forceinline__ double fx_double(Fx f) {  // of a normalised number
   if (f.e >= kFxNan) return __longlong_as_double(0x7ff8000000000000ll);
   if (f.m == 0) return 0.0;
-  const unsigned long long a = ((unsigned long long)(f.m < 0 ? -f.m : f.m) + 16) >> 5;  // 53 bits
+  const unsigned long long m = (unsigned long long)(f.m < 0 ? -f.m : f.m);
   const int x = f.e + 1080;  // biased exponent
   const long long sg = f.m < 0 ? (long long)(1ull << 63) : 0;
-  if (x <= 0) return __longlong_as_double(sg);
-  if (x >= 2046) return __longlong_as_double(sg | 0x7ff0000000000000ll);
+  // 53 bits, fewer below 2^-1022 (subnormal results, rounded once)
+  const int sh = x > 0 ? 5 : min(6 - x, 63);
+  const unsigned long long a = (m + (1ull << (sh - 1))) >> sh;
+  if (x <= 0) return __longlong_as_double(sg | (long long)a);
+  if (x > 2046) return __longlong_as_double(sg | 0x7ff0000000000000ll);
   return __longlong_as_double(sg | (long long)(((unsigned long long)(x - 1) << 52) + a));
 }
 // The sum over the warp of each lane's M numbers (normalised or from fx_from;

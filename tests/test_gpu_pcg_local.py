@@ -88,3 +88,17 @@ def test_zero_right_hand_side_and_iteration_limits():
     assert info["iterations"] == 0 and not np.any(x)
     with pytest.raises(Exception):
         GT.solve(A, b, rtol=RTOL, maxit=3, mode="fp64")
+
+
+@pytest.mark.parametrize("cell,n", [("quad", 33), ("quad", 130), ("tet", 66)])  # a cluster, a grid, the sliced form
+def test_squares_of_the_residual_below_the_normal_range(cell, n):
+    """b scaled by 2^-480: ||b||^2 lies near 2^-960, ||r||^2 at convergence at
+    2^-66 of it, below the smallest normal number.  The solve goes on there:
+    the scaled solution has the residual of the unscaled one."""
+    A, b = _system(cell, 1, 1, n, np.float64)
+    s = 2.0 ** -480
+    b = b / np.linalg.norm(b)
+    assert RTOL ** 2 * s ** 2 < np.finfo(float).tiny
+    x, info = GT.solve(A, b * s, rtol=RTOL, mode="fp64")
+    assert info["converged"] and 0.0 < info["rel_residual"] <= RTOL
+    _check(A, b, x / s)
