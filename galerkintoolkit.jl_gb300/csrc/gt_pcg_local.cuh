@@ -334,12 +334,20 @@ __device__ __forceinline__ A local_combine(A s, int j) {
   return s;
 }
 
+// local columns of a CTA's entries: the first n in shared memory, the others
+// in global memory
+struct LocalCols {
+  const uint16_t *sm, *gl;
+  int n;
+  __device__ __forceinline__ uint16_t operator[](int k) const { return k < n ? sm[k] : gl[k]; }
+};
+
 // out = A x over one group of the CTA's block rows [row0, re): BS * J lanes
 // per block row, lane (j, c) adds component c of the row's entries j, j + J,
 // ... in that order, then the J partial sums are combined; put(row, c, sum)
 // by lanes j = 0; get(k, d): component d of x at a column.
 template <int BS, int J, int U, class A, class V, class C, class GET, class PUT>
-__device__ __forceinline__ void local_group(int row0, int re, const int32_t* rp, const V* val, const C* lc, GET&& get,
+__device__ __forceinline__ void local_group(int row0, int re, const int32_t* rp, const V* val, const C& lc, GET&& get,
                                             PUT&& put) {
   constexpr int GL = BS * J, GPW = 32 / GL;
   const int lane = threadIdx.x & 31;
@@ -712,23 +720,17 @@ __device__ __forceinline__ void pcg_local_body(const PArgs& a, int nb, int blk, 
       if (tid == 0) S.next = LNW;
       for (int i = tid; i < nr; i += LT) put(i, 0, a.resid[r0 + i]);
     } else
-    // (a thread's rows follow the warp's number alone: the sums are reproducible)
+    // (a thread's rows follow its number alone, whatever part of the matrix is
+    // resident: the sums are the same at any size of shared memory)
     with_lanes<BS>(a.lanes, [&](auto jt) {
       constexpr int J = decltype(jt)::value, GPW = 32 / (BS * J), U = BS == 1 ? 8 : 4;
-      if constexpr (XL) {
-        const double* v64 = a.val64 + (size_t)k0 * BS * BS;
-        for (int row0 = wid * GPW; row0 < rsm; row0 += LNW * GPW)
-          local_group<BS, J, U, double>(row0, rsm, s_rp, v64, s_lc, getl, put);
-        for (int row0 = rsm + wid * GPW; row0 < nr; row0 += LNW * GPW)
-          local_group<BS, J, U, double>(row0, nr, s_rp, v64, glc, getl, put);
-      } else {
-        const auto* v64 = [&] {
-          if constexpr (RELIABLE) return a.val64 + (size_t)k0 * BS * BS;
-          else return gval;
-        }();
+      auto rows = [&](auto* v, auto&& lc, auto&& x) {
         for (int row0 = wid * GPW; row0 < nr; row0 += LNW * GPW)
-          local_group<BS, J, U, double>(row0, nr, s_rp, v64, gcol, get, put);
-      }
+          local_group<BS, J, U, double>(row0, nr, s_rp, v, lc, x, put);
+      };
+      if constexpr (XL) rows(a.val64 + (size_t)k0 * BS * BS, LocalCols{s_lc, glc, ksm}, getl);
+      else if constexpr (RELIABLE) rows(a.val64 + (size_t)k0 * BS * BS, gcol, get);
+      else rows(gval, gcol, get);
     });
   };
   auto finish_act = [&] {

@@ -161,3 +161,30 @@ def test_run_batch_concurrent_workers_bitwise_and_converged():
         for s in specs:
             assert three.infos[s.index]["rel_residual"] <= 1e-10
             assert np.array_equal(one.solutions[s.index], three.solutions[s.index])
+
+
+def test_grouped_result_with_a_partly_resident_matrix():
+    """Scattered numbering: the system's own launch keeps only part of its
+    matrix in shared memory, the shared launch beside a system of wider rows
+    all of it.  Solution, iterations and residual are bitwise the same."""
+    def system(order, n, scatter):
+        m = GT.cartesian_mesh((0, 1, 0, 1, 0, 1), (n, n, n))
+        if scatter:
+            new = np.random.default_rng(2).permutation(m.num_nodes)
+            coords = np.empty_like(m.coords)
+            coords[new] = m.coords
+            m.coords = coords
+            for name in ("cell_nodes", "corners", "bfaces", "bedges"):
+                setattr(m, name, np.ascontiguousarray((new[getattr(m, name) - 1] + 1).astype(np.int32)))
+        V = GT.lagrange_space(GT.interior(m), order, dirichlet_boundary=GT.boundary(m))
+        return GT.assemble_matrix_and_vector(GT.laplacian(GT.lognormal_cells(m.num_cells, 0.5, 31)), GT.source(1.0),
+                                             "mixed", V)
+
+    A, b = system(1, 18, True)
+    A2, b2 = system(2, 8, False)
+    B = GB.Batch([A, A2], small_rows=0)
+    for rtol in (1e-6, 1e-8, 1e-10):
+        x, infos = B.solve([b, b2], rtol=rtol, mode="ir")
+        xs, info = GT.solve(A, b, rtol=rtol, mode="ir")
+        assert np.array_equal(B.split(x)[0], xs)
+        assert infos[0]["iterations"] == info["iterations"] and infos[0]["rel_residual"] == info["rel_residual"]
