@@ -32,6 +32,21 @@ inline Line1D line_1d(int order) {
   return t;
 }
 
+// the contractions' arithmetic: FP64, FP32 or double-float
+template <class C>
+__device__ __forceinline__ C arith(double x) {
+  if constexpr (std::is_same<C, dfl>::value) return df_from_double(x);
+  else return (C)x;
+}
+__device__ __forceinline__ double mac(double a, double b, double c) { return fma(a, b, c); }
+__device__ __forceinline__ float mac(float a, float b, float c) { return fmaf(a, b, c); }
+__device__ __forceinline__ dfl mac(dfl a, dfl b, dfl c) { return df_add_sloppy(df_mul(a, b), c); }
+template <class T, class C>
+__device__ __forceinline__ T rounded(C x) {
+  if constexpr (std::is_same<C, dfl>::value) return x.hi;  // the nearest FP32 number: |lo| <= ulp(hi) / 2
+  else return (T)x;
+}
+
 // Scalar Laplacian on hexahedra with a trilinear map, order M - 1, CPB cells
 // per CTA.  With J the Jacobian at a point, the quadrature sum of the
 // reference (src/compiler.jl:1865-1917 with src/accessors.jl:1365-1373 and
@@ -60,7 +75,7 @@ template <int M>
 struct HexSize {
   static constexpr int NP = M * M, NN = M * M * M, NPAIR = NN * (NN + 1) / 2, XP = NP * (NP + 1) / 2;
 };
-template <int M, class T, int CPB>
+template <int M, class T, class C, int CPB>
 __global__ void __launch_bounds__(256) k_elements_hex(const double* __restrict__ coords,
                                                       const int32_t* __restrict__ cell_nodes,
                                                       const double* __restrict__ coef, Line1D line, int64_t ncells,
@@ -73,19 +88,19 @@ __global__ void __launch_bounds__(256) k_elements_hex(const double* __restrict__
   __shared__ double s_c[CPB][3][8];      // coefficients of the map: 1, x, y, xy, z, xz, yz, xyz
   __shared__ double s_dv[CPB][NN];       // |det J| w
   __shared__ double s_v[2][CPB][NN];     // partial contractions of the element vector
-  __shared__ T s_D[CPB][6][NN];          // 11, 22, 33, 12, 13, 23 at the points
-  __shared__ T s_U[CPB][6][NP][NP];      // [kl][q1 q2][a3 b3]
-  __shared__ T s_X[CPB][M][NP][NP], s_Y[CPB][M][NP][NP], s_Z[CPB][M][NP][NP];
-  __shared__ T s_LL[M][M][M], s_LD[M][M][M], s_DD[M][M][M];  // [q][a][b]
+  __shared__ C s_D[CPB][6][NN];          // 11, 22, 33, 12, 13, 23 at the points
+  __shared__ C s_U[CPB][6][NP][NP];      // [kl][q1 q2][a3 b3]
+  __shared__ C s_X[CPB][M][NP][NP], s_Y[CPB][M][NP][NP], s_Z[CPB][M][NP][NP];
+  __shared__ C s_LL[M][M][M], s_LD[M][M][M], s_DD[M][M][M];  // [q][a][b]
   __shared__ double s_L[M][M];           // [q][a]
   __shared__ uint16_t s_pair[NPAIR], s_xpair[XP];
   const int tid = threadIdx.x;
   const int64_t c0 = (int64_t)blockIdx.x * CPB;
   for (int i = tid; i < M * M * M; i += TH) {
     const int q = i / (M * M), a = i / M % M, b = i % M;
-    (&s_LL[0][0][0])[i] = (T)(line.L[q][a] * line.L[q][b]);
-    (&s_LD[0][0][0])[i] = (T)(line.L[q][a] * line.dL[q][b]);
-    (&s_DD[0][0][0])[i] = (T)(line.dL[q][a] * line.dL[q][b]);
+    (&s_LL[0][0][0])[i] = arith<C>(line.L[q][a] * line.L[q][b]);
+    (&s_LD[0][0][0])[i] = arith<C>(line.L[q][a] * line.dL[q][b]);
+    (&s_DD[0][0][0])[i] = arith<C>(line.dL[q][a] * line.dL[q][b]);
     if (b == 0) s_L[q][a] = line.L[q][a];
   }
   for (int n = tid; n < NN; n += TH) {
@@ -145,12 +160,12 @@ __global__ void __launch_bounds__(256) k_elements_hex(const double* __restrict__
     s_dv[cl][q] = (double)(T)(adet * w);  // |det J| w is held in T, also for the element vector
     const double cf = (coef && c < ncells ? coef[c] : 1.0) * w * recip_nr2(adet);
     auto dot = [&](int k, int l) { return cf * (A[k][0] * A[l][0] + A[k][1] * A[l][1] + A[k][2] * A[l][2]); };
-    s_D[cl][0][q] = (T)dot(0, 0);
-    s_D[cl][1][q] = (T)dot(1, 1);
-    s_D[cl][2][q] = (T)dot(2, 2);
-    s_D[cl][3][q] = (T)dot(0, 1);
-    s_D[cl][4][q] = (T)dot(0, 2);
-    s_D[cl][5][q] = (T)dot(1, 2);
+    s_D[cl][0][q] = arith<C>(dot(0, 0));
+    s_D[cl][1][q] = arith<C>(dot(1, 1));
+    s_D[cl][2][q] = arith<C>(dot(2, 2));
+    s_D[cl][3][q] = arith<C>(dot(0, 1));
+    s_D[cl][4][q] = arith<C>(dot(0, 2));
+    s_D[cl][5][q] = arith<C>(dot(1, 2));
   }
   __syncthreads();
   // contraction over q3 (with the element vector's: NN items a cell)
@@ -158,19 +173,19 @@ __global__ void __launch_bounds__(256) k_elements_hex(const double* __restrict__
   if (want_matrix)
     for (int it = tid; it < CPB * NP * NP; it += TH) {
       const int cl = it / (NP * NP), r = it - cl * (NP * NP), q12 = r / NP, ab = r - q12 * NP, a = ab / M, b = ab % M;
-      T u[6];
+      C u[6];
 #pragma unroll
-      for (int k = 0; k < 6; k++) u[k] = (T)0;
+      for (int k = 0; k < 6; k++) u[k] = C{};
 #pragma unroll
       for (int q = 0; q < M; q++) {
-        const T ll = s_LL[q][a][b], ld = s_LD[q][a][b], dd = s_DD[q][a][b];
+        const C ll = s_LL[q][a][b], ld = s_LD[q][a][b], dd = s_DD[q][a][b];
         const int p = q * NP + q12;
-        u[0] = fma(ll, s_D[cl][0][p], u[0]);
-        u[1] = fma(ll, s_D[cl][1][p], u[1]);
-        u[2] = fma(dd, s_D[cl][2][p], u[2]);
-        u[3] = fma(ll, s_D[cl][3][p], u[3]);
-        u[4] = fma(ld, s_D[cl][4][p], u[4]);
-        u[5] = fma(ld, s_D[cl][5][p], u[5]);
+        u[0] = mac(ll, s_D[cl][0][p], u[0]);
+        u[1] = mac(ll, s_D[cl][1][p], u[1]);
+        u[2] = mac(dd, s_D[cl][2][p], u[2]);
+        u[3] = mac(ll, s_D[cl][3][p], u[3]);
+        u[4] = mac(ld, s_D[cl][4][p], u[4]);
+        u[5] = mac(ld, s_D[cl][5][p], u[5]);
       }
 #pragma unroll
       for (int k = 0; k < 6; k++) s_U[cl][k][q12][ab] = u[k];
@@ -189,14 +204,14 @@ __global__ void __launch_bounds__(256) k_elements_hex(const double* __restrict__
       if (it < CPB * M * XP) {
         const int cl = it / (M * XP), r = it - cl * (M * XP), q1 = r / XP, p = s_xpair[r - q1 * XP];
         const int i = p >> 5, j = p & 31, a2 = i % M, a3 = i / M, b2 = j % M, b3 = j / M;
-        T s = (T)0;
+        C s{};
 #pragma unroll
         for (int q = 0; q < M; q++) {
           const int q12 = q * M + q1;
-          s = fma(s_LL[q][a2][b2], s_U[cl][2][q12][a3 * M + b3], s);
-          s = fma(s_DD[q][a2][b2], s_U[cl][1][q12][a3 * M + b3], s);
-          s = fma(s_LD[q][b2][a2], s_U[cl][5][q12][a3 * M + b3], s);  // k = 2, l = 3
-          s = fma(s_LD[q][a2][b2], s_U[cl][5][q12][b3 * M + a3], s);  // k = 3, l = 2
+          s = mac(s_LL[q][a2][b2], s_U[cl][2][q12][a3 * M + b3], s);
+          s = mac(s_DD[q][a2][b2], s_U[cl][1][q12][a3 * M + b3], s);
+          s = mac(s_LD[q][b2][a2], s_U[cl][5][q12][a3 * M + b3], s);  // k = 2, l = 3
+          s = mac(s_LD[q][a2][b2], s_U[cl][5][q12][b3 * M + a3], s);  // k = 3, l = 2
         }
         s_X[cl][q1][i][j] = s;
         s_X[cl][q1][j][i] = s;
@@ -204,14 +219,14 @@ __global__ void __launch_bounds__(256) k_elements_hex(const double* __restrict__
         const int t = it - CPB * M * XP;
         const int cl = t / (M * NP * NP), r = t - cl * (M * NP * NP), q1 = r / (NP * NP), ij = r - q1 * (NP * NP);
         const int i = ij / NP, j = ij - i * NP, a2 = i % M, a3 = i / M, b2 = j % M, b3 = j / M;
-        T y = (T)0, z = (T)0;
+        C y{}, z{};
 #pragma unroll
         for (int q = 0; q < M; q++) {
           const int q12 = q * M + q1;
-          const T ll = s_LL[q][a2][b2];
-          z = fma(ll, s_U[cl][0][q12][a3 * M + b3], z);
-          y = fma(s_LD[q][a2][b2], s_U[cl][3][q12][a3 * M + b3], y);
-          y = fma(ll, s_U[cl][4][q12][a3 * M + b3], y);
+          const C ll = s_LL[q][a2][b2];
+          z = mac(ll, s_U[cl][0][q12][a3 * M + b3], z);
+          y = mac(s_LD[q][a2][b2], s_U[cl][3][q12][a3 * M + b3], y);
+          y = mac(ll, s_U[cl][4][q12][a3 * M + b3], y);
         }
         s_Y[cl][q1][i][j] = y;
         s_Z[cl][q1][i][j] = z;
@@ -231,18 +246,17 @@ __global__ void __launch_bounds__(256) k_elements_hex(const double* __restrict__
       const int cl = it / NPAIR, p = s_pair[it - cl * NPAIR];
       const int64_t c = c0 + cl;
       const int n = p >> 5, m = p & 31, a1 = n % M, i = n / M, b1 = m % M, j = m / M;
-      T s = (T)0;
+      C s{};
 #pragma unroll
       for (int q = 0; q < M; q++) {
-        s = fma(s_LL[q][a1][b1], s_X[cl][q][i][j], s);
-        s = fma(s_DD[q][a1][b1], s_Z[cl][q][i][j], s);
-        s = fma(s_LD[q][b1][a1], s_Y[cl][q][i][j], s);
-        s = fma(s_LD[q][a1][b1], s_Y[cl][q][j][i], s);
+        s = mac(s_LL[q][a1][b1], s_X[cl][q][i][j], s);
+        s = mac(s_DD[q][a1][b1], s_Z[cl][q][i][j], s);
+        s = mac(s_LD[q][b1][a1], s_Y[cl][q][i][j], s);
+        s = mac(s_LD[q][a1][b1], s_Y[cl][q][j][i], s);
       }
       if (c < ncells) {
         T* K = Ke + c * (NN * NN);
-        K[n * NN + m] = s;
-        K[m * NN + n] = s;
+        K[n * NN + m] = K[m * NN + n] = rounded<T>(s);
       }
     }
   for (int it = tid; it < nv; it += TH) {

@@ -87,3 +87,18 @@ def test_fp32_point_weights_of_the_load_vector_hex(order):
     assert abs(want - exact) > 1e-11
     _, b = GT.assemble_matrix_and_vector(GT.laplacian(None), GT.source(1.0), np.float32, V)
     assert abs(np.asarray(b, np.float64).sum() - want) <= 1e-13
+
+
+@pytest.mark.parametrize("n", [2, 9, 17])
+def test_fp32_values_of_q1_hexahedra(n):
+    """FP32 values of distorted Q1 hexahedra are the element entries rounded
+    once and added in FP32.  With u = 2^-24, a rounding error of rms u / sqrt 3
+    of each of a diagonal entry's eight about equal terms (sqrt(1/8) of the
+    entry) and of its seven partial sums (sqrt(sum (j/8)^2, j = 2..8) = 1.78 of
+    the entry) gives at most 1.82 u / sqrt 3 = 6.3e-8 in the 2-norm."""
+    m = GT.cartesian_mesh((0.0, 1.0, 0.0, 1.0, 0.0, 1.0), (n, n, n))
+    m.coords += np.random.default_rng(3).uniform(-0.15, 0.15, m.coords.shape) / n
+    V = GT.lagrange_space(GT.interior(m), 1)
+    A = GT.assemble_matrix(GT.laplacian(GT.lognormal_cells(m.num_cells, 0.5, 17)), "mixed", V)
+    v = A.csr()[2]
+    assert np.linalg.norm(A.values32() - v) <= 6.3e-8 * np.linalg.norm(v)
