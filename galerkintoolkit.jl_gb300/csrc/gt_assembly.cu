@@ -425,6 +425,9 @@ __device__ __forceinline__ void warp_sort_regs(int32_t (&v)[NR], int lane) {
 // for rows of at most S columns, sorts them (in registers up to 128 keys,
 // bitonic in shared memory above) into the row's slot of S entries; the fill
 // pass copies those slots and runs the hash again only for longer rows.
+// rows (optional): only these nrows rows.  longs (optional, count pass): rows
+// with more candidates than fit go on this list, longest[0] is their longest
+// incidence list and longest[1] their number.
 // Bound by instruction issue: 65^2 x 64 Q2 hexahedron rows (64 columns on
 // average, up to 125) 511 -> 228 us, 41^3 P2 tetrahedron rows 62 -> 45 us.
 template <int NN, int S, bool FILL>
@@ -432,14 +435,17 @@ __global__ void __launch_bounds__(256) k_pattern(const int64_t* __restrict__ inc
                                                  const int32_t* __restrict__ cnd, int64_t nrows, int hcap, int icap,
                                                  int32_t* __restrict__ rowcnt, const int64_t* __restrict__ rowptr,
                                                  int32_t* __restrict__ colind, int32_t* __restrict__ slots,
-                                                 uint8_t* __restrict__ small, int32_t* maxrow, uint32_t* err) {
+                                                 uint8_t* __restrict__ small, int32_t* maxrow, uint32_t* err,
+                                                 const int32_t* __restrict__ rows, int32_t* longest,
+                                                 int32_t* __restrict__ longs) {
   extern __shared__ int32_t s_buf[];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   int32_t* tab = s_buf + (size_t)w * (hcap + 2 * icap);  // hash set
   int32_t* ibuf = tab + hcap;                            // sorted incidences of rows with more than 32
   int32_t* keys = ibuf + icap;                           // the row's distinct columns, insertion order
-  const int64_t r = (int64_t)blockIdx.x * (blockDim.x >> 5) + w;
-  if (r >= nrows) return;
+  const int64_t i0 = (int64_t)blockIdx.x * (blockDim.x >> 5) + w;
+  if (i0 >= nrows) return;
+  const int64_t r = rows ? rows[i0] : i0;
   if (FILL && small[r]) {
     // the count pass already wrote this row's sorted columns to its slot
     int64_t o = rowptr[r];
@@ -451,7 +457,15 @@ __global__ void __launch_bounds__(256) k_pattern(const int64_t* __restrict__ inc
   const int ninc = (int)(inc_ptr[r + 1] - ib);
   const int ncand = ninc * NN;
   if (ncand + (ncand >> 2) > hcap || ncand > icap) {
-    if (lane == 0) { atomicOr(err, DEV_ERR_ROW_CAP); if (!FILL) { rowcnt[r] = 0; small[r] = 1; } }
+    if (lane == 0) {
+      if (!FILL && longs) {
+        atomicMax(&longest[0], ninc);
+        longs[atomicAdd(&longest[1], 1)] = (int32_t)r;
+      } else {
+        atomicOr(err, DEV_ERR_ROW_CAP);
+      }
+      if (!FILL) { rowcnt[r] = 0; small[r] = 1; }
+    }
     return;
   }
   // load factor <= 0.8 even if every candidate were distinct
@@ -882,10 +896,12 @@ static int launch_pattern(Matrix* A, int32_t maxinc, const int32_t* bucket, bool
   int64_t nrows = A->nbrows;
   // hash table: load factor <= 0.8 even if every candidate were distinct;
   // ibuf holds the row's incidences, then the compacted keys (<= candidates)
-  // (the warp kernel's exact sizes need the longest incidence list, a host
-  // round trip; it first runs with room for kCandFirst candidates a row -- 8
-  // hexahedra, 25 tetrahedra -- and again with the exact sizes if a row has
-  // more)
+  // The warp kernel's exact sizes need the longest incidence list, a host
+  // round trip.  It first runs with room for kCandFirst candidates a row -- 9
+  // hexahedra, 25 tetrahedra -- and then, with room for the longest one, on
+  // the rows that have more.  (Assembly of P2 tetrahedra, some vertices with 48
+  // cells instead of 24, us: 15^3 x 6 cells 237, 291 with every row counted
+  // again; 21^3 x 6 283, 361.)
   constexpr int kCandFirst = 256;
   int hcap = 32, icap = 32, warps = 8;
   size_t smem = 0;
@@ -914,14 +930,17 @@ static int launch_pattern(Matrix* A, int32_t maxinc, const int32_t* bucket, bool
   // a row turned out longer than 32 incidences or columns) one warp per row
   bool rows_pass = NN <= 8 && S == kRowsS && ctx->pattern_rows, exact = false;
   if (!rows_pass) GT_TRY(setup_warp(false));
-  int32_t* dredo = nullptr;
-  GT_TRY(dalloc(ctx, &dredo, 1));
+  // rows pass: dredo[0] set when a row is too long for it; warp pass: the
+  // longest incidence list beyond kCandFirst candidates and such rows' number
+  int32_t *dredo = nullptr, *dlongs = nullptr;
+  GT_TRY(dalloc(ctx, &dredo, 2));
+  if (!rows_pass) GT_TRY(dalloc(ctx, &dlongs, nrows));
+  int64_t nlong = 0;
   int32_t* dlast = nullptr;
   GT_TRY(dalloc(ctx, &dlast, kRowChunks));
   for (int attempt = 0; attempt < 2; attempt++) {
-    const int grid = grid_for(nrows, warps);
-    GT_CUDA(ctx, cudaMemsetAsync(dmax, 0, sizeof(int32_t), st));
-    GT_CUDA(ctx, cudaMemsetAsync(dredo, 0, sizeof(int32_t), st));
+    if (nlong == 0) GT_CUDA(ctx, cudaMemsetAsync(dmax, 0, sizeof(int32_t), st));
+    GT_CUDA(ctx, cudaMemsetAsync(dredo, 0, 2 * sizeof(int32_t), st));
     if (nrows > 0 && rows_pass) {
       // 16-bit column offsets when every column is within 2^15 of its row
       const bool c16 = sp->dof_spread >= 0 && sp->dof_spread < 32768;
@@ -933,9 +952,10 @@ static int launch_pattern(Matrix* A, int32_t maxinc, const int32_t* bucket, bool
         k_pattern_rows<NN, false><<<GT_KC(ctx, grid_for(nrows, 128)), 128, rsm, st>>>(
             A->inc_ptr, A->inc, sp->cell_ndofs, nrows, rowcnt, slots, small, dmax, dredo, bucket);
     } else if (nrows > 0) {
-      k_pattern<NN, S, false><<<GT_KC(ctx, grid), warps * 32, smem, st>>>(A->inc_ptr, A->inc, sp->cell_ndofs, nrows,
-                                                                          hcap, icap, rowcnt, nullptr, nullptr, slots,
-                                                                          small, dmax, ctx->d_err);
+      const int64_t n = nlong ? nlong : nrows;
+      k_pattern<NN, S, false><<<GT_KC(ctx, grid_for(n, warps)), warps * 32, smem, st>>>(
+          A->inc_ptr, A->inc, sp->cell_ndofs, n, hcap, icap, rowcnt, nullptr, nullptr, slots, small, dmax, ctx->d_err,
+          nlong ? dlongs : nullptr, dredo, exact ? nullptr : dlongs);
     }
     GT_LAUNCH(ctx, "k_pattern<count>");
     GT_TRY(exclusive_scan_i64(ctx, rowcnt, A->rowptr, nrows));
@@ -949,20 +969,20 @@ static int launch_pattern(Matrix* A, int32_t maxinc, const int32_t* bucket, bool
     mark(ctx, "pattern_count");
     GT_CUDA(ctx, cudaMemcpyAsync(&ctx->h_scratch[0], A->rowptr + nrows, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
     GT_CUDA(ctx, cudaMemcpyAsync(&ctx->h_scratch[1], dmax, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-    GT_CUDA(ctx, cudaMemcpyAsync(&ctx->h_scratch[2], dredo, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+    GT_CUDA(ctx, cudaMemcpyAsync(&ctx->h_scratch[2], dredo, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
     uint32_t bits = 0;
     GT_TRY(take_device_error(ctx, &bits));  // synchronises
     // bits of kernels on other streams (element checks) go back for the next take
     const uint32_t own = DEV_ERR_ROW_CAP | DEV_ERR_HASH_FULL;
     ctx->held_err |= bits & ~own;
-    const bool cap = bits & DEV_ERR_ROW_CAP;
-    if ((bits & DEV_ERR_HASH_FULL) || (cap && (rows_pass || exact)))
-      return set_error(ctx, GT_ERR_INVALID, "sparsity: row capacity exceeded");
-    int32_t redo = 0;
-    memcpy(&redo, &ctx->h_scratch[2], sizeof(int32_t));
-    if (!(rows_pass ? redo != 0 : cap)) break;
+    if (bits & own) return set_error(ctx, GT_ERR_INVALID, "sparsity: row capacity exceeded");
+    int32_t redo[2];
+    memcpy(redo, &ctx->h_scratch[2], sizeof(redo));
+    if (redo[0] == 0) break;
     exact = true;
-    if (!rows_pass) {  // a row beyond kCandFirst candidates
+    if (!rows_pass) {  // rows beyond kCandFirst candidates
+      maxinc = redo[0];
+      nlong = redo[1];
       GT_TRY(setup_warp(true));
       continue;
     }
@@ -977,6 +997,7 @@ static int launch_pattern(Matrix* A, int32_t maxinc, const int32_t* bucket, bool
     GT_TRY(setup_warp(true));
   }
   dfree(ctx, dredo);
+  dfree(ctx, dlongs);
   dfree(ctx, dlast);
   if (want_last) {
     memcpy(A->chunk_last, &ctx->h_scratch[16], sizeof(int32_t) * kRowChunks);
@@ -996,7 +1017,8 @@ static int launch_pattern(Matrix* A, int32_t maxinc, const int32_t* bucket, bool
     const int grid = grid_for(nrows, warps);
     k_pattern<NN, S, true><<<GT_KC(ctx, grid), warps * 32, smem, st>>>(A->inc_ptr, A->inc, sp->cell_ndofs, nrows,
                                                                        hcap, icap, nullptr, A->rowptr, A->colind,
-                                                                       slots, small, dmax, ctx->d_err);
+                                                                       slots, small, dmax, ctx->d_err, nullptr, nullptr,
+                                                                       nullptr);
     GT_LAUNCH(ctx, "k_pattern<fill>");
   }
   mark(ctx, "pattern_fill");

@@ -54,3 +54,49 @@ def test_bouquet_rows(disjoint, extra):
     J = coords[np.asarray(cells) - 1][:, 1:] - coords[np.asarray(cells) - 1][:, :1]
     vol = np.abs(np.linalg.det(J)).sum() / 6.0
     assert abs(v.sum() - vol) <= 1e-12 * vol
+
+
+def _with_split_cells(n, nodes):
+    """A grid of P2 tetrahedra whose cells around the first `nodes` interior
+    nodes are split at their centroids: 48 cells at such a node."""
+    m = GT.cartesian_mesh((0.0, 1.0, 0.0, 1.0, 0.0, 1.0), (n, n, n), simplexify=True)
+    cn = m.cell_nodes
+    inner = np.nonzero(((m.coords > 0.0) & (m.coords < 1.0)).all(axis=1))[0] + 1
+    split = np.isin(cn, inner[:nodes]).any(axis=1)
+    new = m.num_nodes + 1 + np.arange(split.sum())
+    cells = [cn[~split]]
+    for j in range(4):
+        t = cn[split].copy()
+        t[:, j] = new
+        cells.append(t)
+    m.coords = np.ascontiguousarray(np.vstack([m.coords, m.coords[cn[split] - 1].mean(axis=1)]))
+    m.cell_nodes = np.ascontiguousarray(np.vstack(cells).astype(np.int32))
+    return m
+
+
+@pytest.mark.parametrize("n,nodes", [(3, 1), (4, 3), (5, 64)])
+def test_few_rows_beyond_the_first_launch(n, nodes):
+    """A few rows with more candidates than the first launch has room for: they
+    alone are counted again (one launch and a scan more)."""
+    m = _with_split_cells(n, nodes)
+    V = GT.lagrange_space(GT.interior(m), 2)
+    A = GT.assemble_matrix(GT.laplacian(), np.float64, V)
+    rp, ci, v = A.csr()
+    om = dict(D=3, ctype=m.cell_type, coords=m.coords, cell_nodes=m.cell_nodes, pf0=m.corners, pf1=m.bedges,
+              pf1g=None, pf2=m.bfaces, pf2g=m.bface_group, cells=(), box=())
+    ref = O.lagrange_space(om, 2)
+    cp, rv, nz = O.assemble_matrix(ref, O.LAPLACE, 4)
+    orp, oci, ov = O.csc_to_csr(cp, rv, nz, ref["nfree"])
+    assert np.array_equal(rp, orp) and np.array_equal(ci, oci)
+    assert np.abs(v - ov).max() <= TOL64 * np.abs(ov).max()
+    ctx = V.ctx
+    if n == 3:  # a scan of one launch in both
+        plain = GT.cartesian_mesh((0.0, 1.0, 0.0, 1.0, 0.0, 1.0), (n, n, n), simplexify=True)
+        count = []
+        for mesh in (plain, m):
+            W = GT.lagrange_space(GT.interior(mesh), 2)
+            GT.assemble_matrix(GT.laplacian(), np.float64, W)
+            l0 = ctx.launches()
+            GT.assemble_matrix(GT.laplacian(), np.float64, W)
+            count.append(ctx.launches() - l0)
+        assert count[1] == count[0] + 2
