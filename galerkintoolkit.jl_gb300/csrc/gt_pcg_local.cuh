@@ -103,12 +103,12 @@ __device__ __forceinline__ double fx_double(Fx f) {  // of a normalised number
   const unsigned long long m = (unsigned long long)(f.m < 0 ? -f.m : f.m);
   const int x = f.e + 1080;  // biased exponent
   const long long sg = f.m < 0 ? (long long)(1ull << 63) : 0;
-  // 53 bits, fewer below 2^-1022 (subnormal results, rounded once)
-  const int sh = x > 0 ? 5 : min(6 - x, 63);
-  const unsigned long long a = (m + (1ull << (sh - 1))) >> sh;
-  if (x <= 0) return __longlong_as_double(sg | (long long)a);
+  if (__builtin_expect(x <= 0, 0)) {  // below 2^-1022: fewer than 53 bits
+    const int sh = min(6 - x, 63);
+    return __longlong_as_double(sg | (long long)((m + (1ull << (sh - 1))) >> sh));
+  }
   if (x > 2046) return __longlong_as_double(sg | 0x7ff0000000000000ll);
-  return __longlong_as_double(sg | (long long)(((unsigned long long)(x - 1) << 52) + a));
+  return __longlong_as_double(sg | (long long)(((unsigned long long)(x - 1) << 52) + ((m + 16) >> 5)));
 }
 // The sum over the warp of each lane's M numbers (normalised or from fx_from;
 // at most 256 in all), in every lane, normalised: aligned to the largest
@@ -334,20 +334,12 @@ __device__ __forceinline__ A local_combine(A s, int j) {
   return s;
 }
 
-// local columns of a CTA's entries: the first n in shared memory, the others
-// in global memory
-struct LocalCols {
-  const uint16_t *sm, *gl;
-  int n;
-  __device__ __forceinline__ uint16_t operator[](int k) const { return k < n ? sm[k] : gl[k]; }
-};
-
 // out = A x over one group of the CTA's block rows [row0, re): BS * J lanes
 // per block row, lane (j, c) adds component c of the row's entries j, j + J,
 // ... in that order, then the J partial sums are combined; put(row, c, sum)
 // by lanes j = 0; get(k, d): component d of x at a column.
 template <int BS, int J, int U, class A, class V, class C, class GET, class PUT>
-__device__ __forceinline__ void local_group(int row0, int re, const int32_t* rp, const V* val, const C& lc, GET&& get,
+__device__ __forceinline__ void local_group(int row0, int re, const int32_t* rp, const V* val, const C* lc, GET&& get,
                                             PUT&& put) {
   constexpr int GL = BS * J, GPW = 32 / GL;
   const int lane = threadIdx.x & 31;
@@ -655,6 +647,8 @@ __device__ __forceinline__ void pcg_local_body(const PArgs& a, int nb, int blk, 
       if (s_rp[mid] <= cap) lo = mid;
       else hi = mid - 1;
     }
+    // whole groups of rows (local_group), unless all fit
+    if (lo < nr) with_lanes<BS>(a.lanes, [&](auto jt) { lo -= lo % (32 / (BS * decltype(jt)::value)); });
     S.rsm = lo;
   }
   __syncthreads();
@@ -724,13 +718,21 @@ __device__ __forceinline__ void pcg_local_body(const PArgs& a, int nb, int blk, 
     // resident: the sums are the same at any size of shared memory)
     with_lanes<BS>(a.lanes, [&](auto jt) {
       constexpr int J = decltype(jt)::value, GPW = 32 / (BS * J), U = BS == 1 ? 8 : 4;
-      auto rows = [&](auto* v, auto&& lc, auto&& x) {
+      if constexpr (XL) {
+        // (resident rows end between two of a warp's groups, or with the rows;
+        // two loops: the compiler then reads s_lc as shared memory)
+        const double* v64 = a.val64 + (size_t)k0 * BS * BS;
+        int row0 = wid * GPW;
+        for (; row0 < rsm; row0 += LNW * GPW) local_group<BS, J, U, double>(row0, rsm, s_rp, v64, s_lc, getl, put);
+        for (; row0 < nr; row0 += LNW * GPW) local_group<BS, J, U, double>(row0, nr, s_rp, v64, glc, getl, put);
+      } else {
+        const auto* v64 = [&] {
+          if constexpr (RELIABLE) return a.val64 + (size_t)k0 * BS * BS;
+          else return gval;
+        }();
         for (int row0 = wid * GPW; row0 < nr; row0 += LNW * GPW)
-          local_group<BS, J, U, double>(row0, nr, s_rp, v, lc, x, put);
-      };
-      if constexpr (XL) rows(a.val64 + (size_t)k0 * BS * BS, LocalCols{s_lc, glc, ksm}, getl);
-      else if constexpr (RELIABLE) rows(a.val64 + (size_t)k0 * BS * BS, gcol, get);
-      else rows(gval, gcol, get);
+          local_group<BS, J, U, double>(row0, nr, s_rp, v64, gcol, get, put);
+      }
     });
   };
   auto finish_act = [&] {
