@@ -8,8 +8,11 @@
 //    (largest first) and runs its whole Jacobi-PCG alone -- SpMV with G lanes
 //    per row, CTA reductions through shared memory, no inter-CTA
 //    synchronisation -- then takes the next one, so the device stays full
-//    however uneven the sizes; the others by one thread-block cluster each
-//    (gt_pcg_local.cuh), largest first, in one launch per lane count;
+//    however uneven the sizes;
+//  * larger small instances with the arithmetic of one thread-block cluster
+//    each (gt_pcg_local.cuh): on clusters, in one launch per block size, or --
+//    when there are more of them than the clusters get done in the same time --
+//    the smaller ones on one CTA each, from a queue (k_bpcg_cluster);
 //  * medium instances (up to the persistent solver's 262,144 rows, matrices
 //    of the batch's own context, FP64 or mixed mode) share cooperative
 //    launches of the persistent solver: each one on the CTAs its own solve
@@ -18,9 +21,9 @@
 //    the other through the single-system solver of gt_solve.cu.
 //
 // Either way an instance's arithmetic and summation order depend only on
-// the instance (one CTA in a fixed order, or the grid layout of the
-// instance's own solve), so its result is bitwise the same alone and in any
-// mix.  The precision modes match gt_solve: FP64 CG, FP32 CG with FP64
+// the instance (one CTA in a fixed order, a cluster's, or the grid layout of
+// the instance's own solve), so its result is bitwise the same alone and in
+// any mix.  The precision modes match gt_solve: FP64 CG, FP32 CG with FP64
 // reliable updates (an FP32 run that stalls or loses its rate continues in
 // FP64), and FP32 CG.
 #include <algorithm>
@@ -29,6 +32,7 @@
 #include <vector>
 
 #include "gt_internal.cuh"
+#include "gt_pcg_impl.cuh"
 #include "gt_rowdot.cuh"
 
 namespace gt {
@@ -36,10 +40,11 @@ namespace gt {
 constexpr int BT = 256;                 // threads per CTA of the batched kernel
 constexpr int BNW = BT / 32;
 constexpr int64_t kSmallRows = 32768;   // largest instance of the small tier
-// Small instances up to this size run one per CTA, the others one per
-// cluster.  Measured on 16 uneven Poisson problems of 256 to 4,096 cells
-// (225 to 30,000 rows; assembly and mixed solves to 1e-10): 9.8 ms, 114 ms
-// with every one on one CTA, whose SM then holds the largest alone.
+// Small instances up to this size are solved by k_bpcg, one per CTA, the
+// others with a cluster's arithmetic.  Measured on 16 uneven Poisson problems
+// of 256 to 4,096 cells (225 to 30,000 rows; assembly and mixed solves to
+// 1e-10): 9.1 ms, 119 ms with every one on one CTA, whose SM then holds the
+// largest alone.
 constexpr int64_t kOneCtaRows = 1024;
 
 struct BInst {
@@ -64,16 +69,16 @@ struct BRes {
 struct BatchImpl {
   Ctx* ctx = nullptr;
   int n = 0;
-  int G = 0;  // lanes per row of the one-CTA solves; 0: each instance's own (row_lanes of its mean row)
+  int G = 0;  // lanes per row of k_bpcg; 0: each instance's own (row_lanes of its mean row)
   int64_t ntot = 0;
   std::vector<Matrix*> mats;
   std::vector<BInst> h_inst;
   BInst* d_inst = nullptr;
-  int64_t small_rows = kSmallRows;  // scalar rows up to which an instance runs on one CTA
+  int64_t small_rows = kSmallRows;  // scalar rows up to which an instance is of the small tier
   std::vector<int> small, large;   // instance ids by class (small: largest first)
 };
 
-// the one-CTA tier: instances up to B->small_rows scalar rows, largest first
+// the small tier: instances up to B->small_rows scalar rows, largest first
 static void classify(BatchImpl* B) {
   B->small.clear();
   B->large.clear();
@@ -114,7 +119,7 @@ __device__ __forceinline__ const V* inst_vals(const BInst& in) {
   else return (const V*)in.v32;
 }
 
-// One CTA per instance, instances from a queue.  BS: block size of the
+// One CTA per instance (up to kOneCtaRows rows), instances from a queue.  BS: block size of the
 // instances of the launch (G lanes per block row); V: values of the
 // iteration, X: vector type; REL: FP64 reliable updates (needs v64).
 // from_x: start from the given x (else x = 0).  Jacobi on the scalar
@@ -328,6 +333,246 @@ __global__ void __launch_bounds__(BT) k_bpcg(const BInst* __restrict__ insts, co
   }
 }
 
+// A cluster's arithmetic on one CTA (gt_pcg_local.cuh, CL), bitwise: the rows
+// are split among LCLUSTER shares as among a cluster's CTAs, every sum is taken
+// by (share, warp of its CTA) -- a warp here takes one after the other -- and
+// the vector updates and the scalars are the cluster's own functions.  One
+// instance per CTA from a queue (its entry lanes beside it); row pointers and
+// vectors in shared memory as far as they fit, else in global memory.
+// cont: continuations of FP32 runs in FP64, from x and st.
+constexpr int VW = pcg::LCLUSTER * pcg::LNW;  // warps of a cluster
+struct VShared {
+  pcg::Fx part[3][VW];
+  pcg::PState st;
+  double alpha;
+  int first[pcg::LCLUSTER + 1];
+  int act, next;
+  int nw;  // warps of a share that hold values in some sum
+};
+// threads per CTA (scalar rows: two CTAs on an SM; block rows, whose products
+// load more per lane: one of twice the warps -- 64 elasticity instances of 1,944
+// rows FP64 11.3 ms, 12.5 with 512 threads)
+constexpr int vthreads(int bs) { return bs == 1 ? 512 : 1024; }
+template <int BS, class V, class X, bool REL>
+__global__ void __launch_bounds__(vthreads(BS), BS == 1 ? 2 : 1) k_bpcg_cluster(
+    const BInst* __restrict__ insts, const int2* __restrict__ queue, int nq, int32_t* head,
+    const double* __restrict__ b, double* x, X* xs, X* r, X* p, X* q, X* dinv, pcg::PState* st, pcg::PRule rule,
+    int cont, int smem_bytes) {
+  using namespace pcg;
+  extern __shared__ __align__(16) unsigned char s_dyn[];
+  __shared__ VShared S;
+  constexpr int VT = vthreads(BS), VNW = VT / 32;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  while (true) {
+    __syncthreads();
+    if (tid == 0) S.next = atomicAdd(head, 1);
+    __syncthreads();
+    if (S.next >= nq) return;
+    const int2 job = queue[S.next];
+    const BInst in = insts[job.x];
+    const int nb = (int)in.nrows, n = nb * BS;
+    const V* val = inst_vals<V>(in);
+    const double* bi = b + in.off;
+    double* xi = x + in.off;
+    X *xsi = xs + in.off, *ri = r + in.off, *pi = p + in.off, *qi = q + in.off, *di = dinv + in.off;
+    int room = smem_bytes;
+    auto place = [&](auto*& v, int cnt) {
+      const int bytes = (cnt * (int)sizeof(*v) + 15) & ~15;
+      if (bytes > room) return false;
+      v = reinterpret_cast<std::remove_reference_t<decltype(v)>>(s_dyn + (smem_bytes - room));
+      room -= bytes;
+      return true;
+    };
+    place(pi, n);
+    int32_t* rp = nullptr;
+    const bool rps = place(rp, nb + 1);
+    place(ri, n);
+    place(qi, n);
+    place(di, n);
+    place(xsi, n);
+    for (int i = wid; i <= LCLUSTER; i += VNW) {
+      const int64_t f = local_first_row(in.rowptr, nb, LCLUSTER, i, BS * BS, BS * row_cost(BS));
+      if (lane == 0) S.first[i] = (int)f;
+    }
+    if (rps)
+      for (int i = tid; i <= nb; i += VT) rp[i] = (int32_t)in.rowptr[i];
+    for (int i = tid; i < n; i += VT) {
+      const int br = i / BS, c = i - br * BS;
+      const int64_t pos = (in.rowptr[br] + in.diag[br]) * BS * BS + c * BS + c;
+      di[i] = (X)(1.0 / (in.v64 ? in.v64[pos] : (double)in.v32[pos]));
+      if (!cont) xi[i] = 0.0;
+      xsi[i] = (X)0;
+      pi[i] = (X)0;
+    }
+    if (tid == 0) {
+      S.st = cont ? st[job.x] : PState{};
+      S.st.done = 0;
+    }
+    __syncthreads();
+    if (tid == 0) {
+      int most = 0;
+      for (int s = 0; s < LCLUSTER; s++) most = max(most, S.first[s + 1] - S.first[s]);
+      const int gpw = BS == 3 ? 2 : 32 / job.y;  // block rows of a warp in the residual's sums
+      S.nw = min(LNW, max((most * BS + 31) / 32, (most + gpw - 1) / gpw));
+    }
+    for (int i = tid; i < 3 * VW; i += VT) (&S.part[0][0])[i] = Fx{0, kFxZero};
+    __syncthreads();
+    // out = A x over block rows [row0, re), a warp
+    auto product = [&](auto jt, auto ut, auto zero, int row0, int re, auto* v, auto&& get, auto&& put) {
+      constexpr int J = decltype(jt)::value, U = decltype(ut)::value;
+      if (rps) local_group<BS, J, U, decltype(zero)>(row0, re, rp, v, in.colind, get, put);
+      else local_group<BS, J, U, decltype(zero)>(row0, re, in.rowptr, v, in.colind, get, put);
+    };
+    // Sum of K values over the cluster's threads, then ctl(totals) by thread 0.
+    // each(share, lo, hi, w, v): adds the values of this lane as lane of warp w
+    // of the share with entries [lo, hi)
+    auto total = [&](auto kt, auto zero, auto&& each, auto&& ctl) {
+      constexpr int K = decltype(kt)::value;
+      for (int t = wid; t < LCLUSTER * S.nw; t += VNW) {
+        const int s = t % LCLUSTER, w = t / LCLUSTER;
+        const int lo = S.first[s] * BS, hi = S.first[s + 1] * BS;
+        Fx f[K];
+#pragma unroll
+        for (int k = 0; k < K; k++) f[k] = Fx{0, kFxZero};
+        if (lo + w * (K == 3 ? 1 : 32) < hi) {  // (else no value: zero)
+          decltype(zero) v[K];
+#pragma unroll
+          for (int k = 0; k < K; k++) v[k] = zero;
+          each(lo, hi, w, v);
+#pragma unroll
+          for (int k = 0; k < K; k++) {
+            const Fx u[1] = {fx_from(v[k])};
+            f[k] = fx_warp_sum<1>(u);
+          }
+        }
+        if (lane == 0)
+#pragma unroll
+          for (int k = 0; k < K; k++) S.part[k][s * LNW + w] = f[k];
+      }
+      __syncthreads();
+      if (wid == 0) {
+        double tot[K];
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+          Fx u[VW / 32];
+#pragma unroll
+          for (int i = 0; i < VW / 32; i++) u[i] = S.part[k][lane + i * 32];
+          tot[k] = fx_double(fx_warp_sum<VW / 32>(u));
+        }
+        if (lane == 0) ctl(tot);
+      }
+      __syncthreads();
+    };
+    auto finish_act = [&] { S.act = (S.st.done || S.st.iters >= rule.maxit) ? 2 : 0; };
+    // FP64 residual -> r, with its sums
+    auto residual = [&](auto&& ctl) {
+      total(std::integral_constant<int, 3>(), 0.0,
+            [&](int lo, int hi, int w, double (&v)[3]) {
+              with_lanes<BS>(job.y, [&](auto jt) {
+                constexpr int J = decltype(jt)::value, GPW = 32 / (BS * J);
+                const std::integral_constant<int, 4> ut;
+                auto put = [&](int row, int c, double o) {
+                  const int i = row * BS + c;
+                  cg_residual(bi[i], o, di[i], ri[i], v);
+                };
+                auto get = [&](int c, int d) { return xi[c * BS + d]; };
+                for (int row0 = lo / BS + w * GPW; row0 < hi / BS; row0 += LNW * GPW) {
+                  if constexpr (REL) product(jt, ut, 0.0, row0, hi / BS, in.v64, get, put);
+                  else product(jt, ut, 0.0, row0, hi / BS, val, get, put);
+                }
+              });
+            },
+            ctl);
+    };
+    residual([&](const double* tot) {
+      ctl_start(S.st, tot, rule, cont);
+      finish_act();
+    });
+    while (!(S.act & 2)) {
+      const X beta = (X)S.st.beta;
+      for (int i = tid; i < n; i += VT) pi[i] = fma(beta, pi[i], times(di[i], ri[i]));
+      __syncthreads();
+      with_lanes<BS>(job.y, [&](auto jt) {
+        constexpr int J = decltype(jt)::value, GPW = 32 / (BS * J);
+        auto get = [&](int c, int d) { return pi[c * BS + d]; };
+        auto put = [&](int row, int c, X o) { qi[row * BS + c] = o; };
+        const std::integral_constant<int, BS == 3 ? 2 : (sizeof(X) == 4 ? 8 : 4)> ut;
+        for (int row0 = wid * GPW; row0 < nb; row0 += VNW * GPW) product(jt, ut, (X)0, row0, nb, val, get, put);
+      });
+      __syncthreads();
+      total(std::integral_constant<int, 1>(), (X)0,
+            [&](int lo, int hi, int w, X (&v)[1]) {
+              for (int i = lo + w * 32 + lane; i < hi; i += LT) v[0] = fma(qi[i], pi[i], v[0]);
+            },
+            [&](const double* tot) { S.alpha = quick_div(S.st.rz, tot[0]); });
+      const X alpha = (X)S.alpha;
+      total(std::integral_constant<int, 2>(), (X)0,
+            [&](int lo, int hi, int w, X (&v)[2]) {
+              for (int i = lo + w * 32 + lane; i < hi; i += LT) cg_step(alpha, qi[i], pi[i], di[i], ri[i], xsi[i], v);
+            },
+            [&](const double* tot) {
+              const int upd = ctl_step<X, REL>(S.st, tot, rule);
+              finish_act();
+              if (upd) S.act = upd;
+            });
+      if constexpr (REL) {
+        if (S.act & 1) {
+          const bool slow = S.act & 4;
+          for (int i = tid; i < n; i += VT) {
+            xi[i] += (double)xsi[i];
+            xsi[i] = (X)0;
+          }
+          __syncthreads();
+          residual([&](const double* tot) {
+            ctl_update<X>(S.st, tot, rule, slow);
+            finish_act();
+          });
+        }
+      }
+    }
+    if (!REL && S.st.done)
+      for (int i = tid; i < n; i += VT) xi[i] += (double)xsi[i];
+    if (tid == 0) st[job.x] = S.st;
+  }
+}
+
+// fits[j]: the local sets of instance ids[j] fit the CTAs of a cluster, given
+// room64 / room32 bytes in the FP64 / FP32 iteration (0: not asked; xl: with
+// FP64 residuals) -- the cluster kernel's own test, which sends an instance
+// that fails it to a grid.  A CTA per instance, a warp per share of rows.
+template <int BS>
+__global__ void __launch_bounds__(BT) k_cluster_fits(const BInst* __restrict__ insts, const int32_t* __restrict__ ids,
+                                                     int room64, int room32, int xl, int32_t* __restrict__ fits) {
+  using namespace pcg;
+  __shared__ uint32_t bits[BNW][kSmallRows / 32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const BInst in = insts[ids[blockIdx.x]];
+  const int nwords = (int)((in.nrows + 31) / 32), tail = bitmap_bytes(nwords);
+  uint32_t* bit = bits[wid];
+  bool ok = true;
+  for (int s = wid; s < LCLUSTER; s += BNW) {
+    const int64_t r0 = local_first_row(in.rowptr, in.nrows, LCLUSTER, s, BS * BS, BS * row_cost(BS));
+    const int64_t r1 = local_first_row(in.rowptr, in.nrows, LCLUSTER, s + 1, BS * BS, BS * row_cost(BS));
+    for (int i = lane; i < nwords; i += 32) bit[i] = 0;
+    __syncwarp();
+    for (int64_t k = in.rowptr[r0] + lane; k < in.rowptr[r1]; k += 32) atomicOr(&bit[in.colind[k] >> 5], 1u << (in.colind[k] & 31));
+    for (int64_t i = r0 + lane; i < r1; i += 32) atomicOr(&bit[i >> 5], 1u << (i & 31));
+    __syncwarp();
+    int nloc = 0;
+    for (int i = lane; i < nwords; i += 32) nloc += __popc(bit[i]);
+    nloc = __reduce_add_sync(0xffffffffu, nloc);
+    const int nr = (int)(r1 - r0), n = nr * BS;
+    ok &= nloc < 65535;
+    if (room64) ok &= local_bytes<BS, double, false, true, false>(n, nloc, nr) + tail <= (size_t)room64;
+    if (room32)
+      ok &= (xl ? local_bytes<BS, float, true, true, false>(n, nloc, nr)
+                : local_bytes<BS, float, false, true, false>(n, nloc, nr)) + tail <= (size_t)room32;
+    __syncwarp();
+  }
+  ok = __syncthreads_and(ok);
+  if (threadIdx.x == 0) fits[blockIdx.x] = ok;
+}
+
 }  // namespace gt
 
 struct gt_batch : gt::BatchImpl {};
@@ -396,7 +641,7 @@ static int launch_small_g(gt_batch* B, int bs, int G, const std::vector<int>& id
   return st;
 }
 
-// lanes of instance i in the one-CTA solves: fixed by set_lanes, else from
+// lanes of instance i in k_bpcg: fixed by set_lanes, else from
 // the instance's own mean row length (so the result depends on nothing
 // else); block rows of 3 take 2 or 4
 static int inst_lanes(const gt_batch* B, int i) {
@@ -418,6 +663,166 @@ static int launch_small(gt_batch* B, const std::vector<int>& ids, const double* 
         if (B->mats[i]->bs == bs && inst_lanes(B, i) == g) sub.push_back(i);
       if (!sub.empty()) GT_TRY((launch_small_g<V, X, REL>(B, bs, g, sub, b, x, rtol, maxit, delta, from_x, hres)));
     }
+  return GT_OK;
+}
+
+// Device blocks of one call, given back when it ends
+struct Blocks {
+  Ctx* ctx;
+  std::vector<void*> held;
+  explicit Blocks(Ctx* c) : ctx(c) {}
+  Blocks(const Blocks&) = delete;
+  Blocks& operator=(const Blocks&) = delete;
+  ~Blocks() {
+    for (void* p : held) pool_free(ctx, p);
+  }
+  template <class T>
+  int get(T** p, int64_t n) {
+    GT_TRY(dalloc(ctx, (unsigned char**)p, (int64_t)sizeof(T) * n));
+    held.push_back(*p);
+    return GT_OK;
+  }
+};
+
+// The instances ids, of block size BS, by k_bpcg_cluster; from (optional): the
+// states of FP32 runs that these continue, by instance
+template <int BS, class V, class X, bool REL>
+static int launch_shared(gt_batch* B, const std::vector<int>& ids, const double* b, double* x, double rtol, int maxit,
+                         double delta, const std::vector<pcg::PState>* from, std::vector<pcg::PState>& st) {
+  Ctx* ctx = B->ctx;
+  cudaStream_t s = ctx->stream;
+  if (ids.empty()) return GT_OK;
+  Blocks mem(ctx);
+  const int64_t n = B->ntot;
+  X *xs, *r, *p, *q, *dinv;
+  int2* queue;
+  int32_t* head;
+  pcg::PState* dst;
+  GT_TRY(mem.get(&xs, n));
+  GT_TRY(mem.get(&r, n));
+  GT_TRY(mem.get(&p, n));
+  GT_TRY(mem.get(&q, n));
+  GT_TRY(mem.get(&dinv, n));
+  GT_TRY(mem.get(&queue, (int64_t)ids.size()));
+  GT_TRY(mem.get(&head, 1));
+  GT_TRY(mem.get(&dst, B->n));
+  std::vector<int2> jobs;
+  for (int i : ids) jobs.push_back(make_int2(i, pcg::entry_lanes(B->mats[i], sizeof(X) == sizeof(double))));
+  GT_TRY(copy_in(ctx, queue, jobs.data(), (int64_t)jobs.size()));
+  if (from) GT_TRY(copy_in(ctx, dst, from->data(), B->n));
+  GT_CUDA(ctx, cudaMemsetAsync(head, 0, sizeof(int32_t), s));
+  auto kern = k_bpcg_cluster<BS, V, X, REL>;
+  // as much shared memory as the largest instance needs, up to 64 KB: beyond,
+  // the L1 left for the matrix is worth more (256 instances of 4,096 rows of
+  // 24 entries 6.4 ms at 64 KB, 6.9 with none, 9.7 at 100 KB; of 3,969 rows of 9
+  // entries 10.0, 11.9 and 9.6)
+  constexpr int kMost = 64 * 1024;
+  int64_t need = 0;
+  for (int i : ids) need = std::max(need, (5 * (int64_t)sizeof(X) * BS + 4) * (B->mats[i]->nbrows + 1) + 128);
+  const int smem = (int)std::min<int64_t>(kMost, need) & ~15;
+  GT_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost));
+  int per_sm = 0;
+  GT_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, vthreads(BS), smem));
+  const int grid = (int)std::min<int64_t>((int64_t)std::max(per_sm, 1) * ctx->num_sms, (int64_t)ids.size());
+  const pcg::PRule rule{rtol * rtol, delta * delta, maxit, ctx->ir_stall_ratio, ctx->ir_stall_count};
+  kern<<<GT_KC(ctx, grid), vthreads(BS), smem, s>>>(B->d_inst, queue, (int)ids.size(), head, b, x, xs, r, p, q, dinv, dst, rule,
+                                          from != nullptr, smem);
+  GT_LAUNCH(ctx, "k_bpcg_cluster");
+  std::vector<pcg::PState> all(B->n);
+  GT_CUDA(ctx, cudaMemcpyAsync(all.data(), dst, sizeof(pcg::PState) * B->n, cudaMemcpyDeviceToHost, s));
+  GT_CUDA(ctx, cudaStreamSynchronize(s));
+  for (int i : ids) st[i] = all[i];
+  return GT_OK;
+}
+template <class V, class X, bool REL>
+static int launch_shared(gt_batch* B, const std::vector<int>& ids, const double* b, double* x, double rtol, int maxit,
+                         double delta, const std::vector<pcg::PState>* from, std::vector<pcg::PState>& st) {
+  std::vector<int> sub[2];
+  for (int i : ids) sub[B->mats[i]->bs == 3].push_back(i);
+  GT_TRY((launch_shared<1, V, X, REL>(B, sub[0], b, x, rtol, maxit, delta, from, st)));
+  return launch_shared<3, V, X, REL>(B, sub[1], b, x, rtol, maxit, delta, from, st);
+}
+
+// operations of an iteration: entries and row costs
+static int64_t cg_work(const Matrix* A) {
+  return A->bnnz * A->bs * A->bs + pcg::row_cost(A->bs) * A->nbrows * A->bs;
+}
+
+// Which of the instances ids (largest first) k_bpcg_cluster takes, the others
+// being left to the clusters.  Both give the same result, so the choice may
+// look at the whole batch: the smallest ones go to single CTAs as long as that
+// shortens the estimated time of the clusters (at_once of them side by side)
+// and then the CTAs.  An iteration of an instance of w operations takes
+// about 5.5 + w / 55,000 us on a cluster and 4 + w / 2,600 us (block
+// rows 3,600) on a CTA alone on its SM, SMs gain 15% by a second one, and iterations go
+// roughly with rows^0.4.  Measured, mixed solves to 1e-10, ms, cluster / CTA: 1
+// instance of 3,969 rows 1.2 / 6.3, 16 3.7 / 6.3, 64 12.3 / 6.8, 256 46 / 10.0; 64
+// of 16,129 rows 33 / 62, 256 125 / 86; 512 of 1,225 rows 54 / 4.7.
+static void pick_shared(const gt_batch* B, const std::vector<int>& ids, int at_once, std::vector<int>* shared) {
+  const int m = (int)ids.size();
+  std::vector<double> cl(m), one(m), rest(m + 1, 0.0);
+  for (int k = 0; k < m; k++) {
+    const Matrix* A = B->mats[ids[k]];
+    const double rows = (double)A->nbrows * A->bs, its = pow(rows, 0.4);
+    const double w = (double)cg_work(A);
+    cl[k] = its * (5.5 + w / 55000.0);
+    one[k] = its * (4.0 + w / (A->bs == 1 ? 2600.0 : 3600.0));
+  }
+  for (int k = m - 1; k >= 0; k--) rest[k] = rest[k + 1] + one[k];
+  std::vector<double> slot(std::max(at_once, 1), 0.0);
+  double most = 0.0, best = 0.0;
+  int first = 0;  // instances from here on go to single CTAs
+  for (int k = 0; k <= m; k++) {
+    const double t = most + (k < m ? std::max(one[k], rest[k] / (1.15 * B->ctx->num_sms)) : 0.0);
+    if (k == 0 || t <= best) {
+      best = t;
+      first = k;
+    }
+    if (k < m) {
+      double& s = *std::min_element(slot.begin(), slot.end());
+      s += cl[k];
+      most = std::max(most, s);
+    }
+  }
+  shared->assign(ids.begin() + first, ids.end());
+}
+
+// Moves the instances that k_bpcg_cluster solves from clustered to shared: of
+// those pick_shared names, the ones that the cluster kernel would not pass on
+// to a grid
+static int split_clustered(gt_batch* B, std::vector<int>& clustered, int mode, std::vector<int>* shared) {
+  Ctx* ctx = B->ctx;
+  std::vector<int> passed;
+  for (int bs : {1, 3}) {
+    std::vector<int> ids, sub;
+    for (int i : clustered)
+      if (B->mats[i]->bs == bs) ids.push_back(i);
+    if (ids.empty()) continue;
+    std::stable_sort(ids.begin(), ids.end(), [&](int i, int j) { return cg_work(B->mats[i]) > cg_work(B->mats[j]); });
+    pcg::ClusterRoom r64, r32;
+    if (mode != GT_SOLVE_FP32) GT_TRY((pcg::cluster_room<double, double, true>(ctx, bs, &r64)));
+    if (mode == GT_SOLVE_FP32) GT_TRY((pcg::cluster_room<float, float, false>(ctx, bs, &r32)));
+    if (mode == GT_SOLVE_IR) GT_TRY((pcg::cluster_room<float, float, true>(ctx, bs, &r32)));
+    const int at_once = mode == GT_SOLVE_FP64 ? r64.at_once : r32.at_once;
+    if (at_once >= 1) pick_shared(B, ids, at_once, &sub);
+    std::vector<int32_t> fits(sub.size());
+    if (!sub.empty()) {
+      Blocks mem(ctx);
+      int32_t *dids, *dfits;
+      GT_TRY(mem.get(&dids, (int64_t)sub.size()));
+      GT_TRY(mem.get(&dfits, (int64_t)sub.size()));
+      GT_TRY(copy_in(ctx, dids, sub.data(), (int64_t)sub.size()));
+      auto kern = bs == 1 ? k_cluster_fits<1> : k_cluster_fits<3>;
+      kern<<<GT_KC(ctx, (unsigned)sub.size()), BT, 0, ctx->stream>>>(B->d_inst, dids, r64.smem, r32.smem,
+                                                                    mode == GT_SOLVE_IR, dfits);
+      GT_LAUNCH(ctx, "k_cluster_fits");
+      GT_CUDA(ctx, cudaMemcpyAsync(fits.data(), dfits, sizeof(int32_t) * sub.size(), cudaMemcpyDeviceToHost, ctx->stream));
+      GT_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    }
+    const size_t head = ids.size() - sub.size();
+    for (size_t k = 0; k < ids.size(); k++) (k >= head && fits[k - head] ? *shared : passed).push_back(ids[k]);
+  }
+  clustered = passed;
   return GT_OK;
 }
 
@@ -459,7 +864,7 @@ static int batch_solve(gt_batch* B, const double* b, double* x, double rtol, int
     }
     return GT_OK;
   };
-  // small instances: one persistent launch, and one of clusters
+  // small instances: one persistent launch ...
   std::vector<int> one, clustered;
   for (int i : B->small) {
     const int64_t rows = B->h_inst[i].nrows * B->h_inst[i].bs;
@@ -493,6 +898,34 @@ static int batch_solve(gt_batch* B, const double* b, double* x, double rtol, int
     info[i].rel_residual = hres[i].bb > 0 ? sqrt(hres[i].rr / hres[i].bb) : 0.0;
     if (mode == GT_SOLVE_FP64) info[i].fp64_iterations = hres[i].iters;
     if (hres[i].status != 0) status = GT_ERR_NOT_CONVERGED;
+  }
+  // ... then single CTAs with a cluster's arithmetic, then clusters
+  std::vector<int> shared;
+  GT_TRY(split_clustered(B, clustered, mode, &shared));
+  if (!shared.empty()) {
+    std::vector<pcg::PState> st(ni), st2(ni);
+    if (mode == GT_SOLVE_FP64) {
+      GT_TRY((launch_shared<double, double, true>(B, shared, b, x, rtol, maxit, 0.0, nullptr, st)));
+      for (int i : shared) info[i].fp64_iterations = st[i].iters;
+    } else if (mode == GT_SOLVE_FP32) {
+      GT_TRY((launch_shared<float, float, false>(B, shared, b, x, rtol, maxit, 0.0, nullptr, st)));
+    } else {
+      GT_TRY((launch_shared<float, float, true>(B, shared, b, x, rtol, maxit, ctx->ir_delta, nullptr, st)));
+      std::vector<int> stalled;
+      for (int i : shared)
+        if (st[i].done == 2) stalled.push_back(i);
+      GT_TRY((launch_shared<double, double, true>(B, stalled, b, x, rtol, maxit, 0.0, &st, st2)));
+      for (int i : stalled) {
+        info[i].fp64_iterations = st2[i].iters - st[i].iters;
+        st[i] = st2[i];
+      }
+    }
+    for (int i : shared) {
+      info[i].iterations = st[i].iters;
+      info[i].outer_iterations = mode == GT_SOLVE_FP32 ? 0 : st[i].nupd;
+      info[i].rel_residual = st[i].bb > 0 ? sqrt(st[i].rr / st[i].bb) : 0.0;
+      if (!(st[i].rr <= st[i].tol2)) status = GT_ERR_NOT_CONVERGED;
+    }
   }
   GT_TRY(groups(clustered, true));
   mark(ctx, "batch_small");

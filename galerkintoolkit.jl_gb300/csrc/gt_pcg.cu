@@ -5,6 +5,7 @@
 namespace gt {
 namespace pcg {
 
+template int cluster_room<double, double, true>(Ctx*, int, ClusterRoom*);
 template int run_sliced<double, double, true>(Ctx*, Matrix*, const double*, const double*, double*, double, int, double,
                                     const PRun*, PRun*, int);
 template int run_groups_dispatch<double, double, true>(

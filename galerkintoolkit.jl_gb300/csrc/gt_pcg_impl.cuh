@@ -67,7 +67,15 @@ struct PState {
   int32_t max_cyc;  // longest cycle between reliable updates so far
 };
 
-struct PArgs {
+// when an iteration ends, updates its residual or goes on in FP64
+struct PRule {
+  double rtol2, delta2;
+  int maxit;
+  double stall_ratio;  // hand-over rule (Ctx::ir_stall_ratio / ir_stall_count)
+  int stall_count;
+};
+
+struct PArgs : PRule {
   const int64_t* rowptr;
   const int32_t* colind;
   const void* val;       // iteration values (V)
@@ -86,10 +94,6 @@ struct PArgs {
   uint32_t* bar;         // barrier counter, zero at launch
   int32_t* err;          // set to 1 when a barrier timed out
   PState* st;
-  double rtol2, delta2;
-  int maxit;
-  double stall_ratio;  // hand-over rule (Ctx::ir_stall_ratio / ir_stall_count)
-  int stall_count;
 };
 
 __device__ __forceinline__ uint64_t global_ns() {
@@ -548,13 +552,18 @@ struct LPlan {
 enum class Place { Auto, Cluster, Grid };
 
 template <class K>
-static int local_plan(Ctx* ctx, const Matrix* A, K kern, bool cluster, size_t xsize, size_t vsize, LPlan* L) {
-  const int64_t lsize = xsize == sizeof(float) ? sizeof(float) + sizeof(double) : xsize;  // local set, a component
+static int cta_room(Ctx* ctx, K kern, int* most) {
   cudaFuncAttributes fa{};
   GT_CUDA(ctx, cudaFuncGetAttributes(&fa, (const void*)kern));
   int optin = 0;
   GT_CUDA(ctx, cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
-  L->most = (optin - (int)fa.sharedSizeBytes) & ~1023;
+  *most = (optin - (int)fa.sharedSizeBytes) & ~1023;
+  return GT_OK;
+}
+template <class K>
+static int local_plan(Ctx* ctx, const Matrix* A, K kern, bool cluster, size_t xsize, size_t vsize, LPlan* L) {
+  const int64_t lsize = xsize == sizeof(float) ? sizeof(float) + sizeof(double) : xsize;  // local set, a component
+  GT_TRY(cta_room(ctx, kern, &L->most));
   const int64_t n = A->nbrows * A->bs;
   const int64_t want = (n + kLocalRows - 1) / kLocalRows;
   const int64_t cap = std::min<int64_t>(ctx->num_sms, LMAXCTA);
@@ -582,6 +591,12 @@ static bool cluster_place(const Matrix* A, bool fp64, Place place) {
   if (place != Place::Auto) return place == Place::Cluster;
   const int64_t work = A->bnnz * A->bs * A->bs + row_cost(A->bs) * A->nbrows * A->bs;
   return (fp64 ? work : work * 5 / 8) <= kClusterWork;
+}
+
+// entry lanes of a scalar row (with_lanes)
+inline int entry_lanes(const Matrix* A, bool fp64) {
+  const double avg = A->nbrows > 0 ? (double)A->bnnz / (double)A->nbrows : 1.0;
+  return fp64 && avg <= 20 ? 1 : (avg <= 40 ? 2 : 4);
 }
 
 // buffers, the start state (zero, or a continuation's) and the Jacobi
@@ -665,8 +680,7 @@ static int pcg_prepare(Ctx* ctx, PSolve<BS, G, V, X, REL>& P, Matrix* A, const V
   args.lcol = P.lcol;
   args.resid = P.resid;
   args.init = from ? 2 : 1;
-  const double avg = A->nbrows > 0 ? (double)A->bnnz / (double)A->nbrows : 1.0;
-  args.lanes = sizeof(X) == sizeof(double) && avg <= 20 ? 1 : (avg <= 40 ? 2 : 4);
+  args.lanes = entry_lanes(A, sizeof(X) == sizeof(double));
   args.bar = P.bar;
   args.err = P.err;
   args.st = P.st;
@@ -841,6 +855,39 @@ int run_sliced(Ctx* ctx, Matrix* A, const V* val, const double* b, double* x, do
   return pcg_finish<1, 2, V, X, REL>(P, h, e != 0, out);
 }
 
+// The clusters of the cluster form: the shared memory a CTA is given, and how
+// many clusters the device holds at once (0: none)
+struct ClusterRoom {
+  int smem = 0, at_once = 0;
+};
+template <int BS, class V, class X, bool REL>
+static int cluster_room_typed(Ctx* ctx, ClusterRoom* room, cudaLaunchConfig_t* cfg, cudaLaunchAttribute* at) {
+  auto kern = k_pcg_cluster<BS, V, X, REL>;
+  GT_TRY(cta_room(ctx, kern, &room->smem));
+  GT_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  GT_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, room->smem));
+  at->id = cudaLaunchAttributeClusterDimension;
+  at->val.clusterDim.x = LCLUSTER;
+  at->val.clusterDim.y = at->val.clusterDim.z = 1;
+  cfg->gridDim = dim3(LCLUSTER);
+  cfg->blockDim = dim3(LT);
+  cfg->dynamicSmemBytes = (size_t)room->smem;
+  cfg->stream = ctx->stream;
+  cfg->attrs = at;
+  cfg->numAttrs = 1;
+  if (cudaOccupancyMaxActiveClusters(&room->at_once, kern, cfg) != cudaSuccess) {
+    cudaGetLastError();
+    room->at_once = 0;
+  }
+  return GT_OK;
+}
+template <class V, class X, bool REL>
+int cluster_room(Ctx* ctx, int bs, ClusterRoom* room) {
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute at[1];
+  return bs == 1 ? cluster_room_typed<1, V, X, REL>(ctx, room, &cfg, at) : cluster_room_typed<3, V, X, REL>(ctx, room, &cfg, at);
+}
+
 // Systems of one block size, each on the CTAs its stand-alone
 // solve would use (so its partition, its sums and its result are bitwise that
 // solve's).  Those placed on a cluster share launches of one cluster per
@@ -875,20 +922,9 @@ static int run_groups_typed(Ctx* ctx, Place place, const std::vector<Matrix*>& A
   cudaLaunchConfig_t cfg{};
   cudaLaunchAttribute at[1];
   if (!cl.empty()) {
-    GT_CUDA(ctx, cudaFuncSetAttribute(ckern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    GT_CUDA(ctx, cudaFuncSetAttribute(ckern, cudaFuncAttributeMaxDynamicSharedMemorySize, cplan.most));
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = LCLUSTER;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    cfg.gridDim = dim3((unsigned)(LCLUSTER * cl.size()));
-    cfg.blockDim = dim3(LT);
-    cfg.dynamicSmemBytes = (size_t)cplan.most;
-    cfg.stream = s;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    int fit = 0;
-    if (cudaOccupancyMaxActiveClusters(&fit, ckern, &cfg) != cudaSuccess || fit < 1) {
-      cudaGetLastError();
+    ClusterRoom room;
+    GT_TRY((cluster_room_typed<BS, V, X, REL>(ctx, &room, &cfg, at)));
+    if (room.at_once < 1) {
       grid.insert(grid.end(), cl.begin(), cl.end());
       cl.clear();
     }
@@ -1024,6 +1060,9 @@ int run_groups_dispatch(Ctx* ctx, Place place, int bs, const std::vector<Matrix*
   return set_error(ctx, GT_ERR_UNSUPPORTED, "persistent PCG: unsupported block size");
 }
 
+extern template int cluster_room<double, double, true>(Ctx*, int, ClusterRoom*);
+extern template int cluster_room<float, float, true>(Ctx*, int, ClusterRoom*);
+extern template int cluster_room<float, float, false>(Ctx*, int, ClusterRoom*);
 extern template int run_groups_dispatch<double, double, true>(
     Ctx*, Place, int, const std::vector<Matrix*>&, const std::vector<const double*>&,
     const std::vector<const double*>&, const std::vector<double*>&, double, int, double, const std::vector<const PRun*>&,

@@ -4,6 +4,7 @@
 namespace gt {
 namespace pcg {
 
+template int cluster_room<float, float, true>(Ctx*, int, ClusterRoom*);
 template int run_sliced<float, float, true>(Ctx*, Matrix*, const float*, const double*, double*, double, int, double,
                                     const PRun*, PRun*, int);
 template int run_groups_dispatch<float, float, true>(

@@ -338,15 +338,15 @@ __device__ __forceinline__ A local_combine(A s, int j) {
 // per block row, lane (j, c) adds component c of the row's entries j, j + J,
 // ... in that order, then the J partial sums are combined; put(row, c, sum)
 // by lanes j = 0; get(k, d): component d of x at a column.
-template <int BS, int J, int U, class A, class V, class C, class GET, class PUT>
-__device__ __forceinline__ void local_group(int row0, int re, const int32_t* rp, const V* val, const C* lc, GET&& get,
+template <int BS, int J, int U, class A, class R, class V, class C, class GET, class PUT>
+__device__ __forceinline__ void local_group(int row0, int re, const R* rp, const V* val, const C* lc, GET&& get,
                                             PUT&& put) {
   constexpr int GL = BS * J, GPW = 32 / GL;
   const int lane = threadIdx.x & 31;
   const int g = lane / GL, l = lane - g * GL, j = l / BS, c = l - j * BS;
   const int row = row0 + g;
   const bool ok = g < GPW && row < re;
-  const int k0 = ok ? rp[row] + j : 0, e = ok ? rp[row + 1] : 0;
+  const int k0 = ok ? (int)rp[row] + j : 0, e = ok ? (int)rp[row + 1] : 0;
   const int n = __reduce_max_sync(0xffffffffu, ok && e > k0 ? (e - k0 + J - 1) / J : 0);  // the warp's steps
   A s = (A)0;
   for (int t = 0; t < n; t += U) {
@@ -453,6 +453,131 @@ __device__ __forceinline__ int64_t local_first_row(const int64_t* __restrict__ r
   return hi;
 }
 
+// --- the vector updates and the iteration's scalars ---------------------------
+// (shared with the kernel that does a cluster's arithmetic on one CTA: products
+// and sums are contracted as written here)
+template <class X>
+__device__ __forceinline__ X times(X a, X b) {
+  if constexpr (sizeof(X) == sizeof(double)) return __dmul_rn(a, b);
+  else return __fmul_rn(a, b);
+}
+// r -= alpha q, xs += alpha p, z = Dinv r; v: r.z, r.r.  Returns z
+template <class X>
+__device__ __forceinline__ X cg_step(X alpha, X q, X p, X di, X& r, X& xs, X (&v)[2]) {
+  r = fma(-alpha, q, r);
+  const X z = times(di, r);
+  xs = fma(alpha, p, xs);
+  v[0] = fma(r, z, v[0]);
+  v[1] = fma(r, r, v[1]);
+  return z;
+}
+// a row's FP64 residual b - o -> r; v: r.z, ||r||^2, ||b||^2.  Returns z
+template <class X>
+__device__ __forceinline__ X cg_residual(double b, double o, X di, X& r, double (&v)[3]) {
+  const double ri = b - o;
+  const X rx = (X)ri, z = times(di, rx);
+  r = rx;
+  v[0] = fma((double)rx, (double)z, v[0]);
+  v[1] = fma(ri, ri, v[1]);
+  v[2] = fma(b, b, v[2]);
+  return z;
+}
+
+// The iteration's scalars, by one thread, from the sums' totals.
+// After the residual of the start's x (cont: the continuation of an FP32 run)
+__device__ __forceinline__ void ctl_start(PState& T, const double* tot, const PRule& u, bool cont) {
+  T.started = 1;
+  T.rz = tot[0];
+  T.rr = tot[1];
+  T.rmax2 = T.rr;
+  T.thr = u.delta2 * T.rmax2;
+  T.beta = 0.0;
+  if (cont) {
+    T.it_upd = T.iters;
+    T.max_cyc = 0;
+    T.stall = 0;
+  } else {
+    T.bb = tot[2];
+    T.tol2 = u.rtol2 * T.bb;
+    T.rzold = 0.0;
+    T.iters = 0;
+    T.nupd = 0;
+  }
+  T.done = le_pos(T.rr, T.tol2);
+}
+// After a step: 1 when a reliable update is due, 5 when after a slow cycle
+template <class X, bool RELIABLE>
+__device__ __forceinline__ int ctl_step(PState& T, const double* tot, const PRule& u) {
+  const double rr = tot[1];
+  T.iters += 1;
+  T.beta = quick_div(tot[0], T.rz);
+  T.rzold = T.rz;
+  T.rz = tot[0];
+  T.rr = rr;
+  const bool stop = le_pos(rr, T.tol2) || T.iters >= u.maxit || is_nan(rr);
+  if constexpr (RELIABLE) {
+    // an FP32 cycle (recurrence residual down by delta) that runs past 2.5x
+    // the longest earlier cycle: the FP32 iteration has lost the rate of the
+    // exact iteration (eps32 * cond(A) too large); hand over to FP64
+    const int cyc = T.iters - T.it_upd;
+    const bool slow =
+        sizeof(X) < sizeof(double) && (cyc > kSlowCycle || (T.max_cyc > 0 && cyc > (5 * T.max_cyc) / 2 + 16));
+    const bool upd = stop || slow || (sizeof(X) < sizeof(double) && le_pos(rr, T.thr));
+    return upd ? (slow ? 5 : 1) : 0;
+  } else {
+    T.done = stop;
+    return 0;
+  }
+}
+// After a reliable update's residual
+template <class X>
+__device__ __forceinline__ void ctl_update(PState& T, const double* tot, const PRule& u, bool slow) {
+  const double rzn = tot[0], rrn = tot[1];
+  double beta = T.rzold != 0.0 ? rzn / T.rzold : 0.0;
+  // the recurrence lost track of the true residual (an FP64 run past its
+  // attainable accuracy, or FP32 drift): the next direction restarts from the
+  // true residual instead of scaling the old one by the true/recurrence
+  // mismatch
+  if (rzn > (sizeof(X) == sizeof(double) ? kRestartRatio64 : kRestartRatio) * T.rz) beta = 0.0;
+  const double prev = T.rmax2;
+  const int cyc = T.iters - T.it_upd;
+  T.rz = rzn;
+  T.rr = rrn;
+  T.rmax2 = rrn;
+  T.thr = u.delta2 * rrn;
+  T.nupd += 1;
+  T.done = rrn <= T.tol2 || T.iters >= u.maxit || !(rrn == rrn);
+  if (sizeof(X) == sizeof(double) && !T.done) {
+    // FP64: true-residual checks that do not halve ||r||, kStagnation times
+    // running -- the tolerance lies below the attainable accuracy
+    // (eps64 * cond(A)); the solve ends, not converged
+    T.stall = rrn > 0.25 * prev ? T.stall + 1 : 0;
+    if (T.stall >= kStagnation) T.done = 1;
+  }
+  if (sizeof(X) < sizeof(double) && !T.done) {
+    // the recurrence fell by delta but the true residual did not halve: the
+    // FP32 operator no longer resolves the error (eps32 * cond ~ 1)
+    T.stall = rrn > u.stall_ratio * prev ? T.stall + 1 : 0;
+    if (T.stall >= u.stall_count || slow) T.done = 2;
+  }
+  if (cyc > T.max_cyc) T.max_cyc = cyc;
+  T.it_upd = T.iters;
+  T.beta = beta;
+}
+
+// Shared memory of a CTA's local set: its own vectors (n_own entries), p at its
+// nloc local columns, their numbers (XL: and FP64 x at them) and nptr row (or
+// slice) pointers; the bitmap and the resident part of the matrix come on top.
+template <int BS, class X, bool XL, bool CL, bool SL>
+__host__ __device__ inline size_t local_bytes(int n_own, int nloc, int nptr) {
+  size_t off = ((size_t)n_own * (2 + CL + 2 * !SL) + (size_t)nloc * BS) * sizeof(X);
+  off = (off + 7) & ~size_t(7);
+  off += (size_t)nloc * ((XL ? BS * sizeof(double) : 0) + sizeof(int32_t) * (XL && CL ? 2 : 1));
+  off += ((size_t)nptr + 1) * sizeof(int32_t);
+  return (off + 15) & ~size_t(15);
+}
+__host__ __device__ inline int bitmap_bytes(int nwords) { return (nwords * 6 + 15) & ~15; }  // words + 16-bit prefixes
+
 // The solve of one system by nb CTAs, this CTA being number blk of them;
 // smem_bytes: the dynamic shared memory of the launch.
 // Entry lanes per block row: every lane of a row costs a step of the
@@ -538,7 +663,7 @@ __device__ __forceinline__ void pcg_local_body(const PArgs& a, int nb, int blk, 
     w0 = nr > 0 ? lo >> 5 : 0;
     nwords = nr > 0 ? (hi >> 5) - w0 + 1 : 0;
   }
-  const int tail = ((nwords * 6 + 15) & ~15);  // 32-bit bitmap words + 16-bit prefix
+  const int tail = bitmap_bytes(nwords);
   // (a window beyond the shared memory: no columns are marked, and the local
   // set counts as not fitting below)
   const bool window = !SL || tail + 4096 <= smem_bytes;
@@ -598,8 +723,7 @@ __device__ __forceinline__ void pcg_local_body(const PArgs& a, int nb, int blk, 
   int32_t* s_g = reinterpret_cast<int32_t*>(s_x + (XL ? (size_t)nloc * BS : 0));
   int32_t* s_gc = XL && CL ? s_g + nloc : s_g;
   int32_t* s_rp = s_gc + nloc;
-  size_t used = reinterpret_cast<unsigned char*>(s_rp + (int)(f1 - f0) + 1) - smem;
-  used = (used + 15) & ~size_t(15);
+  const size_t used = local_bytes<BS, X, XL, CL, SL>(n_own, nloc, (int)(f1 - f0));
   {
     const bool fits = window && nloc < 65535 && used + tail <= (size_t)smem_bytes;
     const float v[1] = {fits ? 0.0f : 1.0f};
@@ -695,14 +819,11 @@ __device__ __forceinline__ void pcg_local_body(const PArgs& a, int nb, int blk, 
     auto getl = [&](int c, int d) { return s_x[c * BS + d]; };
     auto put = [&](int row, int c, double o) {
       const int i = row * BS + c;
-      const double bi = a.b[e0 + i], ri = bi - o;
-      const X rx = (X)ri, zx = w_di[i] * rx;
+      X rx;
+      const X zx = cg_residual(a.b[e0 + i], o, w_di[i], rx, v);
       s_r[i] = rx;
       if constexpr (CL) s_z[i] = zx;
       else __stcg(z + e0 + i, zx);
-      v[0] += (double)rx * (double)zx;
-      v[1] += ri * ri;
-      v[2] += bi * bi;
     };
     if constexpr (SL) {
       // (the rows' sums first: a thread's own rows follow its number alone)
@@ -751,25 +872,7 @@ __device__ __forceinline__ void pcg_local_body(const PArgs& a, int nb, int blk, 
     for (int i = tid; i < n_own; i += LT) w_xs[i] = (X)0;
     for (int i = tid; i < nl; i += LT) s_p[i] = (X)0;
     if (!local_total<3, CL>(v, LT, nb, blk, a.part, epoch, a.err, S, C, [&](const double* tot) {
-          PState& T = S.st;
-          T.started = 1;
-          T.rz = tot[0];
-          T.rr = tot[1];
-          T.rmax2 = T.rr;
-          T.thr = a.delta2 * T.rmax2;
-          T.beta = 0.0;
-          if (init == 2) {
-            T.it_upd = T.iters;
-            T.max_cyc = 0;
-            T.stall = 0;
-          } else {
-            T.bb = tot[2];
-            T.tol2 = a.rtol2 * T.bb;
-            T.rzold = 0.0;
-            T.iters = 0;
-            T.nupd = 0;
-          }
-          T.done = le_pos(T.rr, T.tol2);
+          ctl_start(S.st, tot, a, init == 2);
           S.beta = 0.0;
           finish_act();
         }))
@@ -818,7 +921,7 @@ __device__ __forceinline__ void pcg_local_body(const PArgs& a, int nb, int blk, 
 #pragma unroll
         for (int u = 0; u < U; u++) {
           const int i = i0 + u * LT;
-          if (i < nl) s_p[i] = zv[u] + bx * s_p[i];
+          if (i < nl) s_p[i] = fma(bx, s_p[i], zv[u]);
         }
       }
     }
@@ -835,7 +938,7 @@ __device__ __forceinline__ void pcg_local_body(const PArgs& a, int nb, int blk, 
       });
       __syncthreads();
       X acc[1] = {(X)0};
-      for (int i = tid; i < n_own; i += LT) acc[0] += s_q[i] * s_po[i];
+      for (int i = tid; i < n_own; i += LT) acc[0] = fma(s_q[i], s_po[i], acc[0]);
       if (!local_total<1, CL>(acc, n_own, nb, blk, a.part, epoch, a.err, S, C, [&](const double* tot) {
             S.alpha = quick_div(S.st.rz, tot[0]);
             S.next = LNW;
@@ -859,41 +962,20 @@ __device__ __forceinline__ void pcg_local_body(const PArgs& a, int nb, int blk, 
         for (int u = 0; u < U; u++) {
           const int i = i0 + u * LT;
           if (i < n_own) {
-            const X ri = s_r[i] - alpha * s_q[i];
-            const X zi = dv[u] * ri;
-            w_xs[i] = xv[u] + alpha * s_po[i];
+            X ri = s_r[i];
+            const X zi = cg_step(alpha, s_q[i], s_po[i], dv[u], ri, xv[u], v);
+            w_xs[i] = xv[u];
             s_r[i] = ri;
             if constexpr (CL) s_z[i] = zi;
             else __stcg(z + e0 + i, zi);
-            v[0] += ri * zi;
-            v[1] += ri * ri;
           }
         }
       }
       if (!local_total<2, CL>(v, n_own, nb, blk, a.part, epoch, a.err, S, C, [&](const double* tot) {
-            PState& T = S.st;
-            const double rr = tot[1];
-            T.iters += 1;
-            T.beta = S.beta = quick_div(tot[0], T.rz);
-            T.rzold = T.rz;
-            T.rz = tot[0];
-            T.rr = rr;
-            const bool stop = le_pos(rr, T.tol2) || T.iters >= a.maxit || is_nan(rr);
-            if constexpr (RELIABLE) {
-              // an FP32 cycle (recurrence residual down by delta) that runs
-              // past 2.5x the longest earlier cycle: the FP32 iteration has
-              // lost the rate of the exact iteration (eps32 * cond(A) too
-              // large); hand over to FP64
-              const int cyc = T.iters - T.it_upd;
-              const bool slow = sizeof(X) < sizeof(double) &&
-                                (cyc > kSlowCycle || (T.max_cyc > 0 && cyc > (5 * T.max_cyc) / 2 + 16));
-              const bool upd = stop || slow || (sizeof(X) < sizeof(double) && le_pos(rr, T.thr));
-              finish_act();
-              if (upd) S.act = 1 | (slow ? 4 : 0);
-            } else {
-              T.done = stop;
-              finish_act();
-            }
+            const int upd = ctl_step<X, RELIABLE>(S.st, tot, a);
+            S.beta = S.st.beta;
+            finish_act();
+            if (upd) S.act = upd;
           }))
         return;
     }
@@ -910,40 +992,8 @@ __device__ __forceinline__ void pcg_local_body(const PArgs& a, int nb, int blk, 
         double v[3] = {0.0, 0.0, 0.0};
         residual(v);
         if (!local_total<3, CL>(v, LT, nb, blk, a.part, epoch, a.err, S, C, [&](const double* tot) {
-              PState& T = S.st;
-              const double rzn = tot[0], rrn = tot[1];
-              double beta = T.rzold != 0.0 ? rzn / T.rzold : 0.0;
-              // the recurrence lost track of the true residual (an FP64 run
-              // past its attainable accuracy, or FP32 drift): the next
-              // direction restarts from the true residual instead of scaling
-              // the old one by the true/recurrence mismatch
-              if (rzn > (sizeof(X) == sizeof(double) ? kRestartRatio64 : kRestartRatio) * T.rz) beta = 0.0;
-              const double prev = T.rmax2;
-              const int cyc = T.iters - T.it_upd;
-              T.rz = rzn;
-              T.rr = rrn;
-              T.rmax2 = rrn;
-              T.thr = a.delta2 * rrn;
-              T.nupd += 1;
-              T.done = rrn <= T.tol2 || T.iters >= a.maxit || !(rrn == rrn);
-              if (sizeof(X) == sizeof(double) && !T.done) {
-                // FP64: true-residual checks that do not halve ||r||,
-                // kStagnation times running -- the tolerance lies below the
-                // attainable accuracy (eps64 * cond(A)); the solve ends, not
-                // converged
-                T.stall = rrn > 0.25 * prev ? T.stall + 1 : 0;
-                if (T.stall >= kStagnation) T.done = 1;
-              }
-              if (sizeof(X) < sizeof(double) && !T.done) {
-                // the recurrence fell by delta but the true residual did not
-                // halve: the FP32 operator no longer resolves the error
-                // (eps32 * cond ~ 1)
-                T.stall = rrn > a.stall_ratio * prev ? T.stall + 1 : 0;
-                if (T.stall >= a.stall_count || slow) T.done = 2;
-              }
-              if (cyc > T.max_cyc) T.max_cyc = cyc;
-              T.it_upd = T.iters;
-              T.beta = S.beta = beta;
+              ctl_update<X>(S.st, tot, a, slow);
+              S.beta = S.st.beta;
               finish_act();
             }))
           return;

@@ -4,14 +4,15 @@
 elasticity): of the small instances (up to 32768 scalar rows) those up to
 1024 rows are solved by one persistent launch in which every CTA takes
 instances from a queue (largest first) and runs each one's whole Jacobi-PCG
-alone, the others by one thread-block cluster each; the large instances run
-through the single-system solver.  Each instance keeps its own
+alone, the others by one thread-block cluster each or, where there are many,
+the smaller ones by a CTA each with a cluster's arithmetic; the large
+instances run through the single-system solver.  Each instance keeps its own
 CG scalars and a summation order that depends only on the instance.
 ``run_batch`` drives a whole batch: HBM-budgeted waves, several worker
 contexts assembling instances concurrently and solving the large ones on
 their own streams while the small ones gather for the one-launch tier.
-``autotune_lanes`` picks the lanes per matrix row of the per-CTA SpMV by
-timing the candidates on the batch itself, ``autotune_batch`` the number of
+``autotune_lanes`` picks the lanes per matrix row of the per-CTA SpMV
+(instances up to 1024 rows) by timing the candidates on the batch itself, ``autotune_batch`` the number of
 worker contexts (and the lanes) on a sample of a workload; both cache the
 choice in a JSON file keyed by the batch's shape.
 
@@ -65,8 +66,8 @@ class Batch:
         check(self.ctx.h, self.ctx.lib.gt_batch_set_lanes(self.h, int(lanes)))
 
     def set_small_rows(self, rows: int):
-        """scalar rows up to which an instance belongs to the small tier (one
-        CTA up to 1024 rows, one cluster above; at most 32768); larger instances of the batch's own context, up to 262,144
+        """scalar rows up to which an instance belongs to the small tier (at
+        most 32768); larger instances of the batch's own context, up to 262,144
         rows, share grouped persistent launches (FP64 and mixed modes)"""
         check(self.ctx.h, self.ctx.lib.gt_batch_set_small_rows(self.h, int(rows)))
 
@@ -240,8 +241,8 @@ def run_batch(specs, inputs, precision="mixed", rtol=1e-10, maxit=100000, worker
     single-system solver on the worker's stream, so several such solves and
     the other workers' assembly run on the device together; the smaller
     instances wait for the wave's small tier: one gt_batch over all of them,
-    solved by one persistent launch in which each CTA (above 1024 rows each
-    cluster of CTAs) runs whole instances, largest first.  Every instance's arithmetic depends only on
+    solved by persistent launches in which each CTA or cluster of CTAs runs
+    whole instances, largest first.  Every instance's arithmetic depends only on
     the instance, so its result is bitwise the same whatever the batch.
 
     inputs: {index: (mesh, kappa)} (instance_inputs).  precision "mixed"

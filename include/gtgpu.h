@@ -275,20 +275,23 @@ int gt_spmv(gt_matrix* matrix, const double* x, double* y);
  * A batch of n assembled matrices of block size 1 (scalar problems) or 3
  * (3-D elasticity) on the device of ctx (they may come from other contexts
  * of that device, e.g. assembled concurrently on several streams), solved
- * together on ctx's stream: instances of up to 32768 scalar rows (see
- * gt_batch_set_small_rows) up to 1024 rows in one persistent launch per block
- * size in which each CTA takes instances from a queue (largest first) and runs
- * each one's whole Jacobi-PCG alone, above that one thread-block cluster each; medium ones in grouped persistent launches (below);
- * larger ones one after the other through the single-system solver.  An
+ * together on ctx's stream: small instances (up to 32768 scalar rows, see
+ * gt_batch_set_small_rows) in persistent launches in which a CTA or a
+ * thread-block cluster runs an instance's whole Jacobi-PCG (up to 1024 rows
+ * a CTA; above, the larger ones a cluster and -- with many of them -- the
+ * smaller ones a CTA with the cluster's arithmetic); medium ones in grouped
+ * persistent launches (below); larger ones one after the other through the
+ * single-system solver.  An
  * instance's result does not depend on the rest of the batch.  b and x are
  * the instances' vectors concatenated in batch order (num_free_dofs each,
  * FP64); x is the output (every solve starts from 0).  infos: n entries.
  * GT_SOLVE_IR needs GT_MIXED matrices.  Other block sizes: GT_ERR_INVALID. */
 typedef struct gt_batch gt_batch;
 int gt_batch_create(gt_ctx* ctx, int n, gt_matrix* const* matrices, gt_batch** batch);
-/* lanes per matrix row in the SpMV of the one-CTA-per-instance solves (1, 2,
+/* lanes per matrix row in the SpMV of the instances of up to 1024 rows (1, 2,
  * 4 or 8; 0, the default: each instance's own, from its mean row length;
- * block rows of 3 take 2 or 4: 1 -> 2, 8 -> 4) */
+ * block rows of 3 take 2 or 4: 1 -> 2, 8 -> 4).  Larger instances have lanes
+ * of their own, whatever is set here. */
 int gt_batch_set_lanes(gt_batch* batch, int lanes);
 /* scalar rows up to which an instance is of the small tier (0 .. 32768; the
  * default 32768); larger ones up to 262,144 rows, of ctx's own matrices,

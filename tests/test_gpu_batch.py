@@ -188,3 +188,70 @@ def test_grouped_result_with_a_partly_resident_matrix():
         xs, info = GT.solve(A, b, rtol=rtol, mode="ir")
         assert np.array_equal(B.split(x)[0], xs)
         assert infos[0]["iterations"] == info["iterations"] and infos[0]["rel_residual"] == info["rel_residual"]
+
+
+def _scattered(m, seed=2):
+    """m with its nodes renumbered at random"""
+    new = np.random.default_rng(seed).permutation(m.num_nodes)
+    coords = np.empty_like(m.coords)
+    coords[new] = m.coords
+    m.coords = coords
+    for name in ("cell_nodes", "corners", "bfaces", "bedges"):
+        a = getattr(m, name)
+        setattr(m, name, np.ascontiguousarray((new[a - 1] + 1).astype(np.int32)) if a.size else a)
+    return m
+
+
+def _problem(cell, order, ncomp, n, scatter=False):
+    D = 2 if cell == "quad" else 3
+    m = GT.cartesian_mesh((0.0, 1.0) * D, (n,) * D, simplexify=cell == "tet")
+    if scatter:
+        m = _scattered(m)
+    V = GT.lagrange_space(GT.interior(m), order, tensor_size=(ncomp,) if ncomp > 1 else None,
+                          dirichlet_boundary=GT.boundary(m))
+    k = GT.lognormal_cells(m.num_cells, 0.5, 31)
+    a = GT.laplacian(k) if ncomp == 1 else GT.elasticity(k, 0.3)
+    return GT.assemble_matrix_and_vector(a, GT.source(1.0 if ncomp == 1 else [0.5, 0.5, -1.0]), "mixed", V)
+
+
+@pytest.mark.parametrize("mode,rtol,maxit", [("fp64", 1e-10, 20000), ("ir", 1e-10, 20000), ("fp32", 1e-5, 20000),
+                                             ("ir", 1e-17, 4000), ("fp64", 1e-17, 4000), ("ir", 1e-10, 7)])
+@pytest.mark.parametrize("cell,order,ncomp,n,scatter", [
+    ("quad", 1, 1, 36, False), ("quad", 2, 1, 20, True), ("hex", 1, 1, 12, True), ("hex", 2, 1, 6, False),
+    ("tet", 1, 1, 14, False), ("tet", 2, 1, 7, True), ("hex", 1, 3, 9, False), ("hex", 2, 3, 4, True)])
+def test_many_instances_above_the_one_cta_rows(cell, order, ncomp, n, scatter, mode, rtol, maxit):
+    """Many instances of more than 1,024 rows share SMs, one CTA each; a single
+    one is solved by a cluster.  The results are bitwise the same, with their
+    iterations and residuals (also of solves that stall, miss the tolerance or
+    reach maxit), and the launches do not grow with the batch."""
+    A, b = _problem(cell, order, ncomp, n, scatter)
+    assert A.shape[0] > 1024
+    count = 100
+    B = GB.Batch([A] * count)
+    kw = dict(rtol=rtol, maxit=maxit, mode=mode, raise_on_fail=False)
+    scale = 1.0 + np.arange(count) / count
+    l0 = A.ctx.launches()
+    x, infos = B.solve([b * s for s in scale], **kw)
+    assert A.ctx.launches() - l0 < count
+    parts = B.split(x)
+    for k in (0, 17, 99):
+        alone, one = GB.Batch([A]).solve([b * scale[k]], **kw)
+        assert np.array_equal(alone, parts[k]) and infos[k] == one[0]
+
+
+@pytest.mark.parametrize("mode", ["fp64", "ir"])
+def test_uneven_batch_is_independent_of_its_mix(mode):
+    """Clusters, shared SMs, grids (a scattered numbering whose local sets do
+    not fit a cluster) and the one-CTA tier in one batch: every instance's
+    result is bitwise that of the instance alone."""
+    probs = [_problem("hex", 1, 1, 30, True), _problem("quad", 1, 1, 150), _problem("hex", 2, 1, 6),
+             _problem("hex", 1, 3, 8), _problem("quad", 1, 1, 9)]
+    small = _problem("quad", 1, 1, 34)
+    mats = [A for A, _ in probs] + [small[0]] * 60
+    bs = [b for _, b in probs] + [small[1]] * 60
+    x, infos = GB.Batch(mats).solve(bs, rtol=1e-10, mode=mode)
+    parts = GB.Batch(mats).split(x)
+    for k in (0, 1, 2, 3, 4, 5, 64):
+        alone, one = GB.Batch([mats[k]]).solve([bs[k]], rtol=1e-10, mode=mode)
+        assert infos[k]["rel_residual"] <= 1e-10
+        assert np.array_equal(alone, parts[k]) and infos[k] == one[0], k
