@@ -931,10 +931,11 @@ static int launch_pattern(Matrix* A, int32_t maxinc, const int32_t* bucket, bool
   bool rows_pass = NN <= 8 && S == kRowsS && ctx->pattern_rows, exact = false;
   if (!rows_pass) GT_TRY(setup_warp(false));
   // rows pass: dredo[0] set when a row is too long for it; warp pass: the
-  // longest incidence list beyond kCandFirst candidates and such rows' number
-  int32_t *dredo = nullptr, *dlongs = nullptr;
-  GT_TRY(dalloc(ctx, &dredo, 2));
-  if (!rows_pass) GT_TRY(dalloc(ctx, &dlongs, nrows));
+  // longest incidence list beyond kCandFirst candidates, such rows' number and
+  // the rows
+  int32_t* dredo = nullptr;
+  GT_TRY(dalloc(ctx, &dredo, 2 + (rows_pass ? 0 : nrows)));
+  int32_t* const dlongs = dredo + 2;
   int64_t nlong = 0;
   int32_t* dlast = nullptr;
   GT_TRY(dalloc(ctx, &dlast, kRowChunks));
@@ -997,7 +998,6 @@ static int launch_pattern(Matrix* A, int32_t maxinc, const int32_t* bucket, bool
     GT_TRY(setup_warp(true));
   }
   dfree(ctx, dredo);
-  dfree(ctx, dlongs);
   dfree(ctx, dlast);
   if (want_last) {
     memcpy(A->chunk_last, &ctx->h_scratch[16], sizeof(int32_t) * kRowChunks);
