@@ -666,24 +666,6 @@ static int launch_small(gt_batch* B, const std::vector<int>& ids, const double* 
   return GT_OK;
 }
 
-// Device blocks of one call, given back when it ends
-struct Blocks {
-  Ctx* ctx;
-  std::vector<void*> held;
-  explicit Blocks(Ctx* c) : ctx(c) {}
-  Blocks(const Blocks&) = delete;
-  Blocks& operator=(const Blocks&) = delete;
-  ~Blocks() {
-    for (void* p : held) pool_free(ctx, p);
-  }
-  template <class T>
-  int get(T** p, int64_t n) {
-    GT_TRY(dalloc(ctx, (unsigned char**)p, (int64_t)sizeof(T) * n));
-    held.push_back(*p);
-    return GT_OK;
-  }
-};
-
 // The instances ids, of block size BS, by k_bpcg_cluster; from (optional): the
 // states of FP32 runs that these continue, by instance
 template <int BS, class V, class X, bool REL>

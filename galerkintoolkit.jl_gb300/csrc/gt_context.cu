@@ -229,8 +229,9 @@ static int scan_impl(Ctx* ctx, const Tin* in, Tout* out, int64_t n) {
   }
   Tout* sums = nullptr;
   Tout* soff = nullptr;
-  GT_TRY(dalloc(ctx, &sums, nb));
-  GT_TRY(dalloc(ctx, &soff, nb + 1));
+  Blocks mem(ctx);
+  GT_TRY(mem.get(&sums, nb));
+  GT_TRY(mem.get(&soff, nb + 1));
   k_block_sums<Tin, Tout><<<GT_KC(ctx, (unsigned)nb), SCAN_T, 0, ctx->stream>>>(in, sums, n);
   GT_LAUNCH(ctx, "k_block_sums");
   const int raw = nb <= SCAN_RAW;
@@ -240,8 +241,6 @@ static int scan_impl(Ctx* ctx, const Tin* in, Tout* out, int64_t n) {
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) s = check_cuda(ctx, e, "k_block_scan");
   }
-  dfree(ctx, sums);
-  dfree(ctx, soff);
   return s;
 }
 

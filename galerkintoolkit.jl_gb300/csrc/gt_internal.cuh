@@ -163,6 +163,24 @@ void dfree(Ctx* ctx, T*& p) {
   p = nullptr;
 }
 
+// Device blocks of one call, given back when it ends (also by an error)
+struct Blocks {
+  Ctx* ctx;
+  std::vector<void*> held;
+  explicit Blocks(Ctx* c) : ctx(c) {}
+  Blocks(const Blocks&) = delete;
+  Blocks& operator=(const Blocks&) = delete;
+  ~Blocks() {
+    for (void* p : held) pool_free(ctx, p);
+  }
+  template <class T>
+  int get(T** p, int64_t n) {
+    GT_TRY(dalloc(ctx, (unsigned char**)p, (int64_t)sizeof(T) * n));
+    held.push_back(*p);
+    return GT_OK;
+  }
+};
+
 // reads the device error word (synchronises the stream) and clears it
 int take_device_error(Ctx* ctx, uint32_t* bits);
 
@@ -263,6 +281,8 @@ inline void matrix_values_changed(Matrix* A) {
 }
 // frees the sliced-ELL copy
 void sell_release(Matrix* A);
+// frees its FP64 values
+void sell_release_values64(Matrix* A);
 // makes the sliced-ELL copies of the named values current; *ok: they exist
 int sell_ready(Matrix* A, bool f64, bool f32, bool* ok);
 

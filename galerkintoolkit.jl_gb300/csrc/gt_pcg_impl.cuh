@@ -507,7 +507,8 @@ struct PRun {
 
 // One system's persistent solve: its CTA count (as many as give two row
 // passes per CTA, at most the co-resident CTAs of k_pcg), its buffers and
-// its kernel arguments.
+// its kernel arguments.  What it still holds when it ends goes back to the
+// pool, after the work queued on it.
 template <int BS, int G, class V, class X, bool REL>
 struct PSolve {
   Ctx* ctx = nullptr;       // owns the buffers (a batch may hold matrices of other contexts)
@@ -521,7 +522,34 @@ struct PSolve {
   int32_t* err = nullptr;
   PState* st = nullptr;
   bool own_sync = true;     // bar, err and st allocated here
+  PArgs* dargs = nullptr;   // args on the device (stand-alone local kernel)
   PArgs args{};
+  PSolve() = default;
+  PSolve(const PSolve&) = delete;
+  PSolve& operator=(const PSolve&) = delete;
+  ~PSolve() {
+    if (!ctx) return;
+    cudaStreamSynchronize(ctx->stream);
+    release();
+  }
+  void release() {
+    dfree(ctx, xs);
+    dfree(ctx, r);
+    dfree(ctx, z);
+    dfree(ctx, p);
+    dfree(ctx, q);
+    dfree(ctx, dinv);
+    dfree(ctx, part);
+    dfree(ctx, lcol);
+    dfree(ctx, resid);
+    dfree(ctx, dargs);
+    if (own_sync) {
+      dfree(ctx, bar);
+      dfree(ctx, err);
+      dfree(ctx, st);
+    }
+    ctx = nullptr;
+  }
 };
 
 template <int BS, int G, class V, class X, bool REL>
@@ -610,6 +638,7 @@ static int pcg_prepare(Ctx* ctx, PSolve<BS, G, V, X, REL>& P, Matrix* A, const V
   P.ctx = ctx;
   P.A = A;
   P.nb = nb;
+  P.own_sync = bar == nullptr;
   GT_TRY(dalloc(ctx, &P.xs, n));
   GT_TRY(dalloc(ctx, &P.r, n));
   GT_TRY(dalloc(ctx, &P.z, n));
@@ -624,7 +653,6 @@ static int pcg_prepare(Ctx* ctx, PSolve<BS, G, V, X, REL>& P, Matrix* A, const V
     GT_TRY(dalloc(ctx, &P.q, n));
     GT_TRY(dalloc(ctx, &P.part, (int64_t)3 * P.nb * PSLOT));
   }
-  P.own_sync = bar == nullptr;
   if (P.own_sync) {
     GT_TRY(dalloc(ctx, &P.bar, 2));
     GT_TRY(dalloc(ctx, &P.err, 2));
@@ -692,26 +720,6 @@ static int pcg_prepare(Ctx* ctx, PSolve<BS, G, V, X, REL>& P, Matrix* A, const V
   return GT_OK;
 }
 
-template <int BS, int G, class V, class X, bool REL>
-static void pcg_release(PSolve<BS, G, V, X, REL>& P) {
-  Ctx* ctx = P.ctx;
-  dfree(ctx, P.xs);
-  dfree(ctx, P.r);
-  dfree(ctx, P.z);
-  dfree(ctx, P.p);
-  dfree(ctx, P.q);
-  dfree(ctx, P.dinv);
-  dfree(ctx, P.part);
-  dfree(ctx, P.lcol);
-  dfree(ctx, P.resid);
-  if (P.own_sync) {
-    dfree(ctx, P.bar);
-    dfree(ctx, P.err);
-    pool_free(ctx, P.st);
-    P.st = nullptr;
-  }
-}
-
 // the outcome of a finished system (h: its final state; err: a barrier timed
 // out) and the release of its buffers
 template <int BS, int G, class V, class X, bool REL>
@@ -726,7 +734,7 @@ static int pcg_finish(PSolve<BS, G, V, X, REL>& P, const PState& h, bool err, PR
   } else if (status == GT_OK && !(h.rr <= h.tol2)) {
     status = GT_ERR_NOT_CONVERGED;
   }
-  pcg_release(P);
+  P.release();
   return status;
 }
 
@@ -754,11 +762,10 @@ int run_typed(Ctx* ctx, Matrix* A, const V* val, const double* b, double* x, dou
     PState h{};
     bool err = false;
     int chunk = local ? 512 : 32, done_iters = from ? from->st.iters : 0;
-    PArgs* dargs = nullptr;
     const int2* dmap = nullptr;
     if (local) {
-      GT_TRY(dalloc(ctx, (unsigned char**)&dargs, (int64_t)sizeof(PArgs)));
-      GT_TRY(copy_in(ctx, (unsigned char*)dargs, (const unsigned char*)&args, (int64_t)sizeof(PArgs)));
+      GT_TRY(dalloc(ctx, &P.dargs, 1));
+      GT_TRY(copy_in(ctx, P.dargs, (const PArgs*)&args, 1));
     }
     for (int launch = 0;; launch++) {
       int init = launch == 0 ? (from ? 2 : 1) : 0;
@@ -766,7 +773,7 @@ int run_typed(Ctx* ctx, Matrix* A, const V* val, const double* b, double* x, dou
       if (it_end > maxit || it_end < 0) it_end = maxit;
       ctx->launches++;
       if (local) {
-        void* kargs[] = {&dargs, &dmap, &init, &chunk, &smem};
+        void* kargs[] = {&P.dargs, &dmap, &init, &chunk, &smem};
         GT_CUDA(ctx, cudaLaunchCooperativeKernel((const void*)lkern, dim3(P.nb), dim3(LT), kargs, smem, s));
       } else {
         GT_CUDA(ctx, cudaMemsetAsync(P.bar, 0, sizeof(uint32_t), s));
@@ -787,10 +794,9 @@ int run_typed(Ctx* ctx, Matrix* A, const V* val, const double* b, double* x, dou
       if (h.done || h.iters >= maxit) break;
       if (chunk < 2048) chunk *= 2;
     }
-    if (dargs) pool_free(ctx, dargs);
     if (local && !err && h.done == LOVERFLOW) {
       // nothing was computed: more shared memory, or the global vectors
-      pcg_release(P);
+      P.release();
       if (smem < L.most) smem = L.most;
       else local = false;
       continue;
@@ -800,7 +806,8 @@ int run_typed(Ctx* ctx, Matrix* A, const V* val, const double* b, double* x, dou
 }
 
 // A scalar system in its sliced form; PCG_NOFIT, with nothing done, when it has
-// no sliced copy or its local sets do not fit in shared memory.  smem: a CTA's
+// no sliced copy, its local sets do not fit in shared memory or there is no
+// memory left for what this form holds beside the other's vectors.  smem: a CTA's
 // shared memory (0: the expected need)
 template <class V, class X, bool REL>
 int run_sliced(Ctx* ctx, Matrix* A, const V* val, const double* b, double* x, double rtol, int maxit, double delta,
@@ -817,23 +824,35 @@ int run_sliced(Ctx* ctx, Matrix* A, const V* val, const double* b, double* x, do
   if (spread >= 0) local = std::min<int64_t>(local, rows + 2 * spread);
   const int64_t need = rows * 5 / 4 * 2 * (int64_t)sizeof(X) + local * (int64_t)(sizeof(X) + 4 + (REL && sizeof(X) == 4 ? 8 : 0)) + 8192;
   if (need > L.most + 8192) return PCG_NOFIT;
+  // out of memory: the copies that only this form takes go back too
+  auto without = [&](int s) -> int {
+    if (s != GT_ERR_OOM) return s;
+    if (A->sell_state != 1) sell_release(A);
+    else if (sizeof(V) == 4) sell_release_values64(A);
+    return PCG_NOFIT;
+  };
   bool ready = false;
-  GT_TRY(sell_ready(A, REL, sizeof(V) == 4, &ready));
+  const int rs = sell_ready(A, REL, sizeof(V) == 4, &ready);
+  if (rs != GT_OK) return without(rs);
   if (!ready) return PCG_NOFIT;
   if (smem == 0) smem = (int)std::min<int64_t>(L.most, (need + 1023) & ~int64_t(1023));
   GT_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L.most));
   PSolve<1, 2, V, X, REL> P;
-  GT_TRY((pcg_prepare<1, 2, V, X, REL>(ctx, P, A, val, b, x, rtol, maxit, delta, from, L.nb, true, true)));
-  PArgs* dargs = nullptr;
-  GT_TRY(dalloc(ctx, (unsigned char**)&dargs, (int64_t)sizeof(PArgs)));
-  GT_TRY(copy_in(ctx, (unsigned char*)dargs, (const unsigned char*)&P.args, (int64_t)sizeof(PArgs)));
+  int ps = pcg_prepare<1, 2, V, X, REL>(ctx, P, A, val, b, x, rtol, maxit, delta, from, L.nb, true, true);
+  if (ps == GT_OK) ps = dalloc(ctx, &P.dargs, 1);
+  if (ps != GT_OK) {
+    cudaStreamSynchronize(s);
+    P.release();
+    return without(ps);
+  }
+  GT_TRY(copy_in(ctx, P.dargs, (const PArgs*)&P.args, 1));
   PState h{};
   int32_t e = 0;
   int chunk = 512;
   ChunkGraph graph;
   auto body = [&]() -> int {
     ctx->launches++;
-    void* kargs[] = {&dargs, &chunk, &smem};
+    void* kargs[] = {&P.dargs, &chunk, &smem};
     GT_CUDA(ctx, cudaLaunchCooperativeKernel((const void*)kern, dim3(P.nb), dim3(LT), kargs, smem, s));
     GT_CUDA(ctx, cudaMemcpyAsync(ctx->h_dscratch, P.st, sizeof(PState), cudaMemcpyDeviceToHost, s));
     GT_CUDA(ctx, cudaMemcpyAsync(ctx->h_scratch, P.err, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
@@ -846,9 +865,8 @@ int run_sliced(Ctx* ctx, Matrix* A, const V* val, const double* b, double* x, do
     memcpy(&e, ctx->h_scratch, sizeof(int32_t));
     if (e || h.done || h.iters >= maxit) break;
   }
-  pool_free(ctx, dargs);
   if (!e && h.done == LOVERFLOW) {
-    pcg_release(P);
+    P.release();
     if (smem < L.most) return run_sliced<V, X, REL>(ctx, A, val, b, x, rtol, maxit, delta, from, out, L.most);
     return PCG_NOFIT;
   }
@@ -995,7 +1013,7 @@ static int run_groups_typed(Ctx* ctx, Place place, const std::vector<Matrix*>& A
     for (int k = 0; k < prepared; k++) {
       const int i = ids[k];
       if (ws == GT_OK && !err && h[k].done == LOVERFLOW) {
-        pcg_release(P[k]);
+        P[k].release();
         overflow.push_back(i);
         continue;
       }

@@ -574,6 +574,11 @@ void sell_release(Matrix* A) {
   A->sell_cur64 = A->sell_cur32 = false;
 }
 
+void sell_release_values64(Matrix* A) {
+  dfree(A->ctx, A->sell_v64);
+  A->sell_cur64 = false;
+}
+
 // The sliced copy of a scalar matrix with values val (A->val64 or A->val32),
 // built on first use and refilled after value updates; view->val stays null
 // when the copy does not apply (block rows, the opt-in tiled kernel, or a
@@ -586,15 +591,15 @@ static int sell_prepare(Matrix* A, const V* val, SellView<V>* view) {
   const int64_t nrows = A->nbrows, ns = (nrows + SELL_C - 1) / SELL_C;
   const unsigned g = (unsigned)((ns * 32 + 255) / 256);
   if (A->sell_state == 0) {
+    sell_release(A);  // what an attempt without the memory for all of it left
     int32_t* len32 = nullptr;
     GT_TRY(dalloc(ctx, &A->sell_len, ns));
     GT_TRY(dalloc(ctx, &A->sell_ptr, ns + 1));
-    GT_TRY(dalloc(ctx, &len32, ns));
+    Blocks mem(ctx);
+    GT_TRY(mem.get(&len32, ns));
     k_sell_len<<<GT_KC(ctx, g), 256, 0, ctx->stream>>>(A->rowptr, nrows, ns, A->sell_len, len32);
     GT_LAUNCH(ctx, "k_sell_len");
-    int st = exclusive_scan_i64(ctx, len32, A->sell_ptr, ns);
-    dfree(ctx, len32);
-    GT_TRY(st);
+    GT_TRY(exclusive_scan_i64(ctx, len32, A->sell_ptr, ns));
     GT_CUDA(ctx, cudaMemcpyAsync(&ctx->h_scratch[4], A->sell_ptr + ns, sizeof(int64_t), cudaMemcpyDeviceToHost,
                                  ctx->stream));
     GT_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
@@ -744,13 +749,14 @@ static int pcg(Matrix* A, const V* val, const X* b, X* x, double rtol, int maxit
   CGState* st = nullptr;
   unsigned gs = cg_spmv_grid(A), gv = vec_grid(n), gi = ipt_grid(n);
   Scratch sc;
+  Blocks mem(ctx);
   GT_TRY(sc.alloc(ctx, gs > gv ? gs : gv));
-  GT_TRY(dalloc(ctx, &r, n));
-  GT_TRY(dalloc(ctx, &z, n));
-  GT_TRY(dalloc(ctx, &p, n));
-  GT_TRY(dalloc(ctx, &q, n));
-  GT_TRY(dalloc(ctx, &dinv, n));
-  GT_TRY(dalloc(ctx, (unsigned char**)&st, sizeof(CGState)));
+  GT_TRY(mem.get(&r, n));
+  GT_TRY(mem.get(&z, n));
+  GT_TRY(mem.get(&p, n));
+  GT_TRY(mem.get(&q, n));
+  GT_TRY(mem.get(&dinv, n));
+  GT_TRY(mem.get(&st, 1));
   CGState h0{};
   h0.maxit = maxit;
   GT_CUDA(ctx, cudaMemcpyAsync(st, &h0, sizeof(CGState), cudaMemcpyHostToDevice, s));
@@ -792,14 +798,7 @@ static int pcg(Matrix* A, const V* val, const X* b, X* x, double rtol, int maxit
   *iters_out = h.iters;
   *rr_out = h.rr;
   *bb_out = h.bb;
-  int status = (h.rr <= h.tol2) ? GT_OK : GT_ERR_NOT_CONVERGED;
-  dfree(ctx, r);
-  dfree(ctx, z);
-  dfree(ctx, p);
-  dfree(ctx, q);
-  dfree(ctx, dinv);
-  pool_free(ctx, st);
-  return status;
+  return h.rr <= h.tol2 ? GT_OK : GT_ERR_NOT_CONVERGED;
 }
 
 // ---------------------------------------------------------------------------
@@ -989,15 +988,16 @@ static int pcg_reliable(Matrix* A, const V* val, const double* b, double* x, dou
   unsigned gmax = gs > gv ? gs : gv;
   if (gr > gmax) gmax = gr;
   Scratch sc;
+  Blocks mem(ctx);
   GT_TRY(sc.alloc(ctx, gmax));
-  GT_TRY(dalloc(ctx, &xs, n));
-  GT_TRY(dalloc(ctx, &r, n));
-  GT_TRY(dalloc(ctx, &z, n));
-  GT_TRY(dalloc(ctx, &p, n));
-  GT_TRY(dalloc(ctx, &q, n));
-  GT_TRY(dalloc(ctx, &dinv, n));
-  GT_TRY(dalloc(ctx, &bb, 1));
-  GT_TRY(dalloc(ctx, (unsigned char**)&st, sizeof(CGState)));
+  GT_TRY(mem.get(&xs, n));
+  GT_TRY(mem.get(&r, n));
+  GT_TRY(mem.get(&z, n));
+  GT_TRY(mem.get(&p, n));
+  GT_TRY(mem.get(&q, n));
+  GT_TRY(mem.get(&dinv, n));
+  GT_TRY(mem.get(&bb, 1));
+  GT_TRY(mem.get(&st, 1));
   GT_CUDA(ctx, cudaMemsetAsync(st, 0, sizeof(CGState), s));
   GT_CUDA(ctx, cudaMemsetAsync(xs, 0, sizeof(X) * n, s));
   GT_TRY(find_diag(A));
@@ -1050,16 +1050,7 @@ static int pcg_reliable(Matrix* A, const V* val, const double* b, double* x, dou
   *iters_out = h.iters;
   *nupd_out = h.nupd;
   *relres_out = h.bb > 0 ? sqrt(h.rr / h.bb) : 0.0;
-  int status = h.done == 2 ? CG_STALLED : (h.rr <= h.tol2) ? GT_OK : GT_ERR_NOT_CONVERGED;
-  dfree(ctx, xs);
-  dfree(ctx, r);
-  dfree(ctx, z);
-  dfree(ctx, p);
-  dfree(ctx, q);
-  dfree(ctx, dinv);
-  dfree(ctx, bb);
-  pool_free(ctx, st);
-  return status;
+  return h.done == 2 ? CG_STALLED : (h.rr <= h.tol2) ? GT_OK : GT_ERR_NOT_CONVERGED;
 }
 
 int sell_ready(Matrix* A, bool f64, bool f32, bool* ok) {
@@ -1099,8 +1090,9 @@ static int true_residual(Matrix* A, const double* b, const double* x, double* re
   double *r = nullptr, *scal = nullptr;
   Scratch sc;
   GT_TRY(sc.alloc(ctx, vec_grid(n)));
-  GT_TRY(dalloc(ctx, &r, n));
-  GT_TRY(dalloc(ctx, &scal, 2));
+  Blocks mem(ctx);
+  GT_TRY(mem.get(&r, n));
+  GT_TRY(mem.get(&scal, 2));
   GT_TRY((Ops<double, double>::spmv(ctx, A, A->val64, x, b, r)));
   GT_TRY(norm2(ctx, (const double*)r, n, scal, sc.rb));
   GT_TRY(norm2(ctx, b, n, scal + 1, sc.rb));
@@ -1108,8 +1100,6 @@ static int true_residual(Matrix* A, const double* b, const double* x, double* re
   GT_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   double rn2 = ctx->h_dscratch[0], bn2 = ctx->h_dscratch[1];
   *relres = bn2 > 0 ? sqrt(rn2 / bn2) : 0.0;
-  dfree(ctx, r);
-  dfree(ctx, scal);
   return GT_OK;
 }
 
@@ -1170,8 +1160,9 @@ int solve(Matrix* A, const double* b, double* x, double rtol, int maxit, int mod
   } else if (mode == GT_SOLVE_FP32) {
     if (!A->val32) return set_error(ctx, GT_ERR_INVALID, "GT_SOLVE_FP32 needs FP32 values (GT_FP32 or GT_MIXED)");
     float *bf = nullptr, *xf = nullptr;
-    GT_TRY(dalloc(ctx, &bf, n));
-    GT_TRY(dalloc(ctx, &xf, n));
+    Blocks mem(ctx);
+    GT_TRY(mem.get(&bf, n));
+    GT_TRY(mem.get(&xf, n));
     k_copy_f64_to_f32<<<GT_KC(ctx, gv), RED_T, 0, s>>>(b, n, bf);
     k_copy_f64_to_f32<<<GT_KC(ctx, gv), RED_T, 0, s>>>(x, n, xf);
     GT_LAUNCH(ctx, "k_copy_f64_to_f32");
@@ -1183,8 +1174,6 @@ int solve(Matrix* A, const double* b, double* x, double rtol, int maxit, int mod
     inf.iterations = it;
     inf.rel_residual = bb > 0 ? sqrt(rr / bb) : 0.0;
     if (A->val64) GT_TRY(true_residual(A, b, x, &inf.rel_residual));
-    dfree(ctx, bf);
-    dfree(ctx, xf);
   } else if (mode == GT_SOLVE_IR) {
     if (!A->val64 || !A->val32) return set_error(ctx, GT_ERR_INVALID, "GT_SOLVE_IR needs GT_MIXED values");
     // FP32 CG (FP32 values, vectors and inner sums) with an FP64 true
@@ -1229,12 +1218,13 @@ int gt_solve(gt_matrix* A, const double* b, double* x, double rtol, int maxit, i
   bool xdev = cudaPointerGetAttributes(&ax, x) == cudaSuccess && ax.type == cudaMemoryTypeDevice;
   cudaGetLastError();
   double *bd = (double*)b, *xd = x;
+  Blocks mem(ctx);
   if (!bdev) {
-    GT_TRY(dalloc(ctx, &bd, n));
+    GT_TRY(mem.get(&bd, n));
     GT_TRY(copy_in(ctx, bd, b, n));
   }
   if (!xdev) {
-    GT_TRY(dalloc(ctx, &xd, n));
+    GT_TRY(mem.get(&xd, n));
     GT_TRY(copy_in(ctx, xd, (const double*)x, n));
   }
   int s = solve(A, bd, xd, rtol, maxit, mode, info);
@@ -1242,9 +1232,7 @@ int gt_solve(gt_matrix* A, const double* b, double* x, double rtol, int maxit, i
     int s2 = copy_out(ctx, x, xd, n);
     cudaStreamSynchronize(ctx->stream);
     if (s == GT_OK) s = s2;
-    dfree(ctx, xd);
   }
-  if (!bdev) dfree(ctx, bd);
   return s;
 }
 

@@ -145,3 +145,53 @@ def test_unattainable_tolerance_stops_without_diverging(n):
     if B is not None:
         xb, infos = B.solve([b], rtol=1e-19, maxit=200000, mode="fp64", raise_on_fail=False)
         assert infos[0]["iterations"] < 20 * ok["iterations"] + 200 and infos[0]["rel_residual"] < 1e-12
+
+
+@pytest.mark.parametrize("mode", ["fp64", "ir", "fp32"])
+def test_solve_with_little_memory_left(mode, monkeypatch):
+    """Scalar systems above 262,144 rows with less and less device memory
+    free: a solve fails with GT_ERR_OOM or succeeds, it succeeds wherever the
+    solver with one launch per phase does, and with the matrices gone the
+    context holds nothing more than before."""
+    torch = pytest.importorskip("torch")
+    left = (400, 200, 160, 130, 110, 90, 75, 60, 50, 40, 30, 20, 10, 4)  # MB
+    monkeypatch.setenv("GTGPU_PCG", "launches")
+    phases = GT.Context(0)
+    monkeypatch.delenv("GTGPU_PCG")
+    ctxs = {"phases": phases, "default": GT.Context(0)}
+    m = GT.cartesian_mesh((0, 1, 0, 1, 0, 1), (66, 66, 66))
+    runs, held, spaces = {}, {}, {}
+    for name, ctx in ctxs.items():
+        V = spaces[name] = GT.lagrange_space(GT.interior(m), 1, dirichlet_boundary=GT.boundary(m), ctx=ctx)
+        A, b = GT.assemble_matrix_and_vector(GT.laplacian(), GT.source(1.0), "mixed", V)
+        GT.solve(A, b, rtol=1e-4, mode=mode)  # every kernel has run
+        del A
+        held[name] = ctx.memory()[0]
+        runs[name] = [GT.assemble_matrix_and_vector(GT.laplacian(), GT.source(1.0), "mixed", V)[0] for _ in left]
+        ctx.trim()
+    ok = {name: [] for name in ctxs}
+    for k, mb in enumerate(left):
+        for name, ctx in ctxs.items():
+            hog = torch.empty(torch.cuda.mem_get_info()[0] - (mb << 20), dtype=torch.uint8, device="cuda")
+            try:
+                x, info = GT.solve(runs[name][k], b, rtol=1e-4, mode=mode)
+                ok[name].append(True)
+                assert info["converged"]
+            except GT.GTError as e:
+                ok[name].append(False)
+                assert e.code == _lib.GT_ERR_OOM
+            del hog
+            torch.cuda.empty_cache()
+            ctx.trim()
+    assert any(ok["phases"]) and not all(ok["phases"])
+    assert all(d or not p for d, p in zip(ok["default"], ok["phases"])), ok
+    for name, ctx in ctxs.items():
+        runs[name].clear()
+        ctx.synchronize()
+        assert ctx.memory()[0] == held[name]
+        x, info = GT.solve(GT.assemble_matrix(GT.laplacian(), "mixed", spaces[name]), b, rtol=1e-4, mode=mode)
+        assert info["converged"]
+    del V, spaces
+    m._device.clear()
+    for ctx in ctxs.values():
+        ctx.close()
