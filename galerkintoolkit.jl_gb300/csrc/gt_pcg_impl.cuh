@@ -439,8 +439,16 @@ __device__ __forceinline__ void pcg_body(const PArgs& a, int nb, int blk, int in
   if (blk == 0 && tid == 0) *a.st = S;
 }
 
+// CTAs an SM (0: the compiler's choice): four, three of block rows of 3, where
+// the compiler would spill.  Measured, ms: Q2 hexahedra 30^3 FP64 22.5 (25.3
+// by its choice), Q2 elasticity on scattered numberings 16^3 FP64 27.3 (32.6),
+// 19^3 FP32 15.0 (20.4); the FP32 iteration with updates is faster by its choice
+// (P2 tetrahedra 31^3 21.6, 22.9 with four).
+constexpr int pcg_per_sm(int bs, bool fp64, bool reliable) {
+  return fp64 ? (bs == 3 ? 3 : 4) : (bs == 3 && !reliable ? 3 : 0);
+}
 template <int BS, int G, class V, class X, bool RELIABLE>
-__global__ void __launch_bounds__(PT) k_pcg(PArgs a, int init, int it_end) {
+__global__ void __launch_bounds__(PT, pcg_per_sm(BS, sizeof(X) == sizeof(double), RELIABLE)) k_pcg(PArgs a, int init, int it_end) {
   __shared__ double s_red[3 * NW];
   __shared__ double s_tot[4];
   __shared__ int s_abort;
@@ -509,7 +517,7 @@ struct PRun {
 // passes per CTA, at most the co-resident CTAs of k_pcg), its buffers and
 // its kernel arguments.  What it still holds when it ends goes back to the
 // pool, after the work queued on it.
-template <int BS, int G, class V, class X, bool REL>
+template <int BS, class V, class X, bool REL>
 struct PSolve {
   Ctx* ctx = nullptr;       // owns the buffers (a batch may hold matrices of other contexts)
   Matrix* A = nullptr;
@@ -552,12 +560,21 @@ struct PSolve {
   }
 };
 
-template <int BS, int G, class V, class X, bool REL>
-static int pcg_ctas(Ctx* ctx, const Matrix* A, int* nb) {
+// k_pcg of a matrix: lanes per row by its mean row length (row_lanes; block rows
+// of 2 are short), and the CTAs that solve it
+template <int BS, class V, class X, bool REL>
+static int pcg_kernel(Ctx* ctx, const Matrix* A, const void** kern, int* nb) {
+  int G = 2;
+  *kern = (const void*)k_pcg<BS, 2, V, X, REL>;
+  if constexpr (BS != 2)
+    if (A->nbrows > 0 && row_lanes((double)A->bnnz / (double)A->nbrows) > 2) {
+      G = 4;
+      *kern = (const void*)k_pcg<BS, 4, V, X, REL>;
+    }
   int per_sm = 0;
-  GT_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pcg<BS, G, V, X, REL>, PT, 0));
+  GT_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, *kern, PT, 0));
   if (per_sm < 1) return set_error(ctx, GT_ERR_CUDA, "persistent PCG kernel does not fit on an SM");
-  constexpr int NG = PT / G;
+  const int NG = PT / G;
   int64_t want = (A->nbrows + 2 * NG - 1) / (2 * NG);  // at least two row passes per CTA
   int64_t cap = (int64_t)per_sm * ctx->num_sms;
   *nb = (int)(want < cap ? (want > 0 ? want : 1) : cap);
@@ -629,8 +646,8 @@ inline int entry_lanes(const Matrix* A, bool fp64) {
 
 // buffers, the start state (zero, or a continuation's) and the Jacobi
 // diagonal of one system; bar / err / st come from the caller when given
-template <int BS, int G, class V, class X, bool REL>
-static int pcg_prepare(Ctx* ctx, PSolve<BS, G, V, X, REL>& P, Matrix* A, const V* val, const double* b, double* x,
+template <int BS, class V, class X, bool REL>
+static int pcg_prepare(Ctx* ctx, PSolve<BS, V, X, REL>& P, Matrix* A, const V* val, const double* b, double* x,
                        double rtol, int maxit, double delta, const PRun* from, int nb, bool local, bool sliced = false,
                        uint32_t* bar = nullptr, int32_t* err = nullptr, PState* st = nullptr) {
   cudaStream_t s = ctx->stream;
@@ -722,8 +739,8 @@ static int pcg_prepare(Ctx* ctx, PSolve<BS, G, V, X, REL>& P, Matrix* A, const V
 
 // the outcome of a finished system (h: its final state; err: a barrier timed
 // out) and the release of its buffers
-template <int BS, int G, class V, class X, bool REL>
-static int pcg_finish(PSolve<BS, G, V, X, REL>& P, const PState& h, bool err, PRun* out) {
+template <int BS, class V, class X, bool REL>
+static int pcg_finish(PSolve<BS, V, X, REL>& P, const PState& h, bool err, PRun* out) {
   Ctx* ctx = P.ctx;
   int status = GT_OK;
   if (err) status = set_error(ctx, GT_ERR_TIMEOUT, "persistent PCG: a grid barrier timed out");
@@ -744,7 +761,7 @@ static int pcg_finish(PSolve<BS, G, V, X, REL>& P, const PState& h, bool err, PR
 // vectors does.  Measured, us a solve, local / global vectors: 2-D Q1 64 x 64
 // FP64 1630 / 2790, 3-D Q1 25^3 mixed 889 / 1370, Q2 elasticity 11^3 FP64
 // 15200 / 42200.
-template <int BS, int G, class V, class X, bool REL>
+template <int BS, class V, class X, bool REL>
 int run_typed(Ctx* ctx, Matrix* A, const V* val, const double* b, double* x, double rtol, int maxit, double delta,
               const PRun* from, PRun* out) {
   cudaStream_t s = ctx->stream;
@@ -754,10 +771,11 @@ int run_typed(Ctx* ctx, Matrix* A, const V* val, const double* b, double* x, dou
   int smem = L.est;
   for (bool local = L.ok;;) {
     int nb = L.nb;
-    if (!local) GT_TRY((pcg_ctas<BS, G, V, X, REL>(ctx, A, &nb)));
+    const void* gkern = nullptr;
+    if (!local) GT_TRY((pcg_kernel<BS, V, X, REL>(ctx, A, &gkern, &nb)));
     else GT_CUDA(ctx, cudaFuncSetAttribute(lkern, cudaFuncAttributeMaxDynamicSharedMemorySize, L.most));
-    PSolve<BS, G, V, X, REL> P;
-    GT_TRY((pcg_prepare<BS, G, V, X, REL>(ctx, P, A, val, b, x, rtol, maxit, delta, from, nb, local)));
+    PSolve<BS, V, X, REL> P;
+    GT_TRY((pcg_prepare<BS, V, X, REL>(ctx, P, A, val, b, x, rtol, maxit, delta, from, nb, local)));
     PArgs& args = P.args;
     PState h{};
     bool err = false;
@@ -778,7 +796,7 @@ int run_typed(Ctx* ctx, Matrix* A, const V* val, const double* b, double* x, dou
       } else {
         GT_CUDA(ctx, cudaMemsetAsync(P.bar, 0, sizeof(uint32_t), s));
         void* kargs[] = {&args, &init, &it_end};
-        GT_CUDA(ctx, cudaLaunchCooperativeKernel((const void*)k_pcg<BS, G, V, X, REL>, dim3(P.nb), dim3(PT), kargs, 0, s));
+        GT_CUDA(ctx, cudaLaunchCooperativeKernel(gkern, dim3(P.nb), dim3(PT), kargs, 0, s));
       }
       GT_CUDA(ctx, cudaMemcpyAsync(ctx->h_dscratch, P.st, sizeof(PState), cudaMemcpyDeviceToHost, s));
       GT_CUDA(ctx, cudaMemcpyAsync(ctx->h_scratch, P.err, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
@@ -801,7 +819,7 @@ int run_typed(Ctx* ctx, Matrix* A, const V* val, const double* b, double* x, dou
       else local = false;
       continue;
     }
-    return pcg_finish<BS, G, V, X, REL>(P, h, err, out);
+    return pcg_finish<BS, V, X, REL>(P, h, err, out);
   }
 }
 
@@ -837,8 +855,8 @@ int run_sliced(Ctx* ctx, Matrix* A, const V* val, const double* b, double* x, do
   if (!ready) return PCG_NOFIT;
   if (smem == 0) smem = (int)std::min<int64_t>(L.most, (need + 1023) & ~int64_t(1023));
   GT_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L.most));
-  PSolve<1, 2, V, X, REL> P;
-  int ps = pcg_prepare<1, 2, V, X, REL>(ctx, P, A, val, b, x, rtol, maxit, delta, from, L.nb, true, true);
+  PSolve<1, V, X, REL> P;
+  int ps = pcg_prepare<1, V, X, REL>(ctx, P, A, val, b, x, rtol, maxit, delta, from, L.nb, true, true);
   if (ps == GT_OK) ps = dalloc(ctx, &P.dargs, 1);
   if (ps != GT_OK) {
     cudaStreamSynchronize(s);
@@ -870,7 +888,7 @@ int run_sliced(Ctx* ctx, Matrix* A, const V* val, const double* b, double* x, do
     if (smem < L.most) return run_sliced<V, X, REL>(ctx, A, val, b, x, rtol, maxit, delta, from, out, L.most);
     return PCG_NOFIT;
   }
-  return pcg_finish<1, 2, V, X, REL>(P, h, e != 0, out);
+  return pcg_finish<1, V, X, REL>(P, h, e != 0, out);
 }
 
 // The clusters of the cluster form: the shared memory a CTA is given, and how
@@ -915,7 +933,7 @@ int cluster_room(Ctx* ctx, int bs, ClusterRoom* room) {
 // bounded sums.  All systems of one call start alike (froms all null, or all
 // continuations).  A system whose local sets do not fit goes from a cluster to
 // a grid, and from a shared grid to one of its own.
-template <int BS, int G, class V, class X, bool REL>
+template <int BS, class V, class X, bool REL>
 static int run_groups_typed(Ctx* ctx, Place place, const std::vector<Matrix*>& As, const std::vector<const V*>& vals,
                             const std::vector<const double*>& bs, const std::vector<double*>& xs, double rtol,
                             int maxit, double delta, const std::vector<const PRun*>& froms, std::vector<PRun>& outs,
@@ -956,7 +974,7 @@ static int run_groups_typed(Ctx* ctx, Place place, const std::vector<Matrix*>& A
     PState* sts = nullptr;
     PArgs* dargs = nullptr;
     int2* dmap = nullptr;
-    std::vector<PSolve<BS, G, V, X, REL>> P(m);
+    std::vector<PSolve<BS, V, X, REL>> P(m);
     int prepared = 0;
     std::vector<PState> h(m);
     std::vector<PArgs> hargs(m);
@@ -973,7 +991,7 @@ static int run_groups_typed(Ctx* ctx, Place place, const std::vector<Matrix*>& A
       for (int k = 0; k < m; k++) {
         const int i = ids[k];
         prepared++;
-        GT_TRY((pcg_prepare<BS, G, V, X, REL>(ctx, P[k], As[i], vals[i], bs[i], xs[i], rtol, maxit, delta, froms[i],
+        GT_TRY((pcg_prepare<BS, V, X, REL>(ctx, P[k], As[i], vals[i], bs[i], xs[i], rtol, maxit, delta, froms[i],
                                               cluster ? LCLUSTER : plan[i].nb, true, false, bars + 2 * k, errs + 2 * k,
                                               sts + k)));
         hargs[k] = P[k].args;
@@ -1017,7 +1035,7 @@ static int run_groups_typed(Ctx* ctx, Place place, const std::vector<Matrix*>& A
         overflow.push_back(i);
         continue;
       }
-      const int st = pcg_finish<BS, G, V, X, REL>(P[k], h[k], err, &outs[i]);
+      const int st = pcg_finish<BS, V, X, REL>(P[k], h[k], err, &outs[i]);
       status[i] = ws == GT_OK ? st : ws;
     }
     dfree(ctx, bars);
@@ -1056,12 +1074,11 @@ static int run_groups_typed(Ctx* ctx, Place place, const std::vector<Matrix*>& A
   }
   for (int i : alone)
     status[i] =
-        run_typed<BS, G, V, X, REL>(ctx, As[i], vals[i], bs[i], xs[i], rtol, maxit, delta, froms[i], &outs[i]);
+        run_typed<BS, V, X, REL>(ctx, As[i], vals[i], bs[i], xs[i], rtol, maxit, delta, froms[i], &outs[i]);
   return GT_OK;
 }
 
-// kernel instances by block size (G: lanes per row of the kernel on global
-// vectors)
+// kernel instances by block size
 template <class V, class X, bool REL>
 int run_groups_dispatch(Ctx* ctx, Place place, int bs, const std::vector<Matrix*>& As, const std::vector<const V*>& vals,
                         const std::vector<const double*>& b, const std::vector<double*>& x, double rtol, int maxit,
@@ -1069,11 +1086,11 @@ int run_groups_dispatch(Ctx* ctx, Place place, int bs, const std::vector<Matrix*
                         std::vector<int>& status) {
   switch (bs) {
     case 1:
-      return run_groups_typed<1, 2, V, X, REL>(ctx, place, As, vals, b, x, rtol, maxit, delta, froms, outs, status);
+      return run_groups_typed<1, V, X, REL>(ctx, place, As, vals, b, x, rtol, maxit, delta, froms, outs, status);
     case 2:
-      return run_groups_typed<2, 2, V, X, REL>(ctx, place, As, vals, b, x, rtol, maxit, delta, froms, outs, status);
+      return run_groups_typed<2, V, X, REL>(ctx, place, As, vals, b, x, rtol, maxit, delta, froms, outs, status);
     case 3:
-      return run_groups_typed<3, 4, V, X, REL>(ctx, place, As, vals, b, x, rtol, maxit, delta, froms, outs, status);
+      return run_groups_typed<3, V, X, REL>(ctx, place, As, vals, b, x, rtol, maxit, delta, froms, outs, status);
   }
   return set_error(ctx, GT_ERR_UNSUPPORTED, "persistent PCG: unsupported block size");
 }

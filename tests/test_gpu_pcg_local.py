@@ -102,3 +102,57 @@ def test_squares_of_the_residual_below_the_normal_range(cell, n):
     x, info = GT.solve(A, b * s, rtol=RTOL, mode="fp64")
     assert info["converged"] and 0.0 < info["rel_residual"] <= RTOL
     _check(A, b, x / s)
+
+
+def _scattered(cell, order, ncomp, n, T):
+    """nodes numbered at random"""
+    D = 2 if cell == "quad" else 3
+    m = GT.cartesian_mesh((0.0, 1.0) * D, (n,) * D, simplexify=cell == "tet")
+    new = np.random.default_rng(5).permutation(m.num_nodes)
+    coords = np.empty_like(m.coords)
+    coords[new] = m.coords
+    m.coords = coords
+    for name in ("cell_nodes", "corners", "bfaces", "bedges"):
+        a = getattr(m, name)
+        setattr(m, name, np.ascontiguousarray((new[a - 1] + 1).astype(np.int32)) if a.size else a)
+    m.cell_nodes = np.ascontiguousarray(m.cell_nodes[np.random.default_rng(6).permutation(m.num_cells)])
+    V = GT.lagrange_space(GT.interior(m), order, tensor_size=(ncomp,) if ncomp > 1 else None,
+                          dirichlet_boundary=GT.boundary(m))
+    k = GT.lognormal_cells(m.num_cells, 0.5, 31)
+    a = GT.laplacian(k) if ncomp == 1 else GT.elasticity(k, 0.3)
+    return GT.assemble_matrix_and_vector(a, GT.source(1.0 if ncomp == 1 else [0.5] * ncomp), T, V)
+
+
+@pytest.mark.parametrize("mode", ["fp64", "ir"])
+@pytest.mark.parametrize("cell,order,ncomp,n", [
+    ("hex", 2, 1, 25), ("quad", 2, 1, 250), ("quad", 2, 2, 170), ("hex", 1, 3, 41), ("hex", 2, 3, 17)])
+def test_kernel_on_global_vectors(cell, order, ncomp, n, mode):
+    """its lane counts: mean rows up to and above 40 entries, block rows"""
+    A, b = _scattered(cell, order, ncomp, n, "mixed")
+    x, info = GT.solve(A, b, rtol=RTOL, mode=mode)
+    assert info["converged"] and info["rel_residual"] <= RTOL
+    _check(A, b, x)
+
+
+@pytest.mark.parametrize("cell,order,ncomp,n", [
+    ("quad", 1, 1, 2), ("quad", 1, 1, 4), ("quad", 2, 1, 17), ("hex", 1, 1, 9), ("tet", 1, 1, 13),  # one cluster
+    ("quad", 1, 1, 130), ("hex", 2, 1, 13), ("tet", 2, 1, 9),  # a grid
+    ("quad", 1, 2, 2), ("quad", 2, 2, 11), ("hex", 1, 3, 2), ("hex", 2, 3, 6),  # block rows
+    ("quad", 1, 1, 514), ("hex", 1, 1, 66),  # the sliced form
+])
+def test_fp32_mode(cell, order, ncomp, n):
+    """The FP32 iteration without residual updates stops by its recurrence
+    residual, which drifts from the true one by the rounding of the k updates
+    of x and r: at most (row length + 4) u sum |a_ij| |x_j| each."""
+    A, b = _system(cell, order, ncomp, n, "mixed")
+    x, info = GT.solve(A, b, rtol=1e-4, mode="fp32")
+    assert info["converged"]
+    rp, ci, v = A.csr()
+    M = sp.csr_matrix((v, ci, rp), shape=(len(b), len(b)))
+    u, k = 2.0 ** -24, info["iterations"]
+    slack = (k + 1) * (np.diff(rp).max() + 4) * u * np.linalg.norm(abs(M) @ np.abs(x))
+    r = np.linalg.norm(b - M @ x)
+    assert r <= 1e-4 * np.linalg.norm(b) + slack
+    assert abs(info["rel_residual"] - r / np.linalg.norm(b)) <= 1e-6 * info["rel_residual"]
+    again, _ = GT.solve(A, b, rtol=1e-4, mode="fp32")
+    assert np.array_equal(x, again)
