@@ -267,6 +267,10 @@ struct Matrix {
   double* sell_v64 = nullptr;
   float* sell_v32 = nullptr;
   bool sell_cur64 = false, sell_cur32 = false;  // values match val64 / val32
+  // what solves found of this sparsity's local sets, by form of the persistent
+  // solver (gt_pcg_impl.cuh): 1 the expected shared memory was too small, 2 all
+  // of it
+  uint8_t local_sets[6] = {};
   // the last cell among the incidences of each row chunk (rows nbrows*k/K ..
   // nbrows*(k+1)/K, K = kRowChunks; -1: no incidence), from the count pass:
   // the scatter of a chunk waits only for the element chunks up to that cell

@@ -755,6 +755,13 @@ static int pcg_finish(PSolve<BS, V, X, REL>& P, const PState& h, bool err, PRun*
   return status;
 }
 
+// place in Matrix::local_sets of a form: iteration type and residuals, sliced
+// or not
+template <class X, bool REL>
+constexpr int local_form(bool sliced) {
+  return (sizeof(X) == sizeof(double) ? 0 : REL ? 1 : 2) + 3 * sliced;
+}
+
 // One system on the whole device.  The local kernel (gt_pcg_local.cuh) takes
 // it unless its local sets do not fit in shared memory -- a numbering that
 // scatters a CTA's columns over the whole system; then the kernel on global
@@ -768,8 +775,9 @@ int run_typed(Ctx* ctx, Matrix* A, const V* val, const double* b, double* x, dou
   auto lkern = k_pcg_local<BS, V, X, REL>;
   LPlan L;
   GT_TRY(local_plan(ctx, A, lkern, false, sizeof(X), sizeof(V), &L));
-  int smem = L.est;
-  for (bool local = L.ok;;) {
+  uint8_t& known = A->local_sets[local_form<X, REL>(false)];
+  int smem = known ? L.most : L.est;
+  for (bool local = L.ok && known < 2;;) {
     int nb = L.nb;
     const void* gkern = nullptr;
     if (!local) GT_TRY((pcg_kernel<BS, V, X, REL>(ctx, A, &gkern, &nb)));
@@ -815,6 +823,7 @@ int run_typed(Ctx* ctx, Matrix* A, const V* val, const double* b, double* x, dou
     if (local && !err && h.done == LOVERFLOW) {
       // nothing was computed: more shared memory, or the global vectors
       P.release();
+      known = smem < L.most ? 1 : 2;
       if (smem < L.most) smem = L.most;
       else local = false;
       continue;
@@ -841,7 +850,8 @@ int run_sliced(Ctx* ctx, Matrix* A, const V* val, const double* b, double* x, do
   int64_t local = rows * 13 / 4 + 512;
   if (spread >= 0) local = std::min<int64_t>(local, rows + 2 * spread);
   const int64_t need = rows * 5 / 4 * 2 * (int64_t)sizeof(X) + local * (int64_t)(sizeof(X) + 4 + (REL && sizeof(X) == 4 ? 8 : 0)) + 8192;
-  if (need > L.most + 8192) return PCG_NOFIT;
+  uint8_t& known = A->local_sets[local_form<X, REL>(true)];
+  if (need > L.most + 8192 || known == 2) return PCG_NOFIT;
   // out of memory: the copies that only this form takes go back too
   auto without = [&](int s) -> int {
     if (s != GT_ERR_OOM) return s;
@@ -853,6 +863,7 @@ int run_sliced(Ctx* ctx, Matrix* A, const V* val, const double* b, double* x, do
   const int rs = sell_ready(A, REL, sizeof(V) == 4, &ready);
   if (rs != GT_OK) return without(rs);
   if (!ready) return PCG_NOFIT;
+  if (known == 1) smem = L.most;
   if (smem == 0) smem = (int)std::min<int64_t>(L.most, (need + 1023) & ~int64_t(1023));
   GT_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L.most));
   PSolve<1, V, X, REL> P;
@@ -885,6 +896,7 @@ int run_sliced(Ctx* ctx, Matrix* A, const V* val, const double* b, double* x, do
   }
   if (!e && h.done == LOVERFLOW) {
     P.release();
+    known = smem < L.most ? 1 : 2;
     if (smem < L.most) return run_sliced<V, X, REL>(ctx, A, val, b, x, rtol, maxit, delta, from, out, L.most);
     return PCG_NOFIT;
   }
@@ -1053,7 +1065,7 @@ static int run_groups_typed(Ctx* ctx, Place place, const std::vector<Matrix*>& A
   std::vector<int> order;
   for (int i : grid) {
     GT_TRY(local_plan(ctx, As[i], gkern, false, sizeof(X), sizeof(V), &plan[i]));
-    (plan[i].ok ? order : alone).push_back(i);
+    (plan[i].ok && !As[i]->local_sets[local_form<X, REL>(false)] ? order : alone).push_back(i);
   }
   std::stable_sort(order.begin(), order.end(), [&](int a, int c) { return plan[a].est > plan[c].est; });
   size_t i0 = 0;

@@ -123,6 +123,28 @@ def _scattered(cell, order, ncomp, n, T):
     return GT.assemble_matrix_and_vector(a, GT.source(1.0 if ncomp == 1 else [0.5] * ncomp), T, V)
 
 
+@pytest.mark.parametrize("T,mode", [(np.float64, "fp64"), ("mixed", "ir"), ("mixed", "fp32")])
+@pytest.mark.parametrize("n", [56, 66])  # below and above 262,144 rows
+def test_scattered_nodes(n, T, mode):
+    """A CTA's rows touch columns all over the system, whose local sets do not
+    fit in shared memory.  The kernel on global vectors, or one launch per
+    phase, solves it, and a second solve goes there at once, with the same
+    result."""
+    A, b = _scattered("tet", 1, 1, n, T)
+    rtol = RTOL if mode != "fp32" else 1e-4
+    count, xs = [], []
+    for _ in range(2):
+        l0 = A.ctx.launches()
+        x, info = GT.solve(A, b, rtol=rtol, mode=mode)
+        count.append(A.ctx.launches() - l0)
+        xs.append(x)
+        assert info["converged"]
+        if mode != "fp32":  # (stops by its recurrence residual)
+            _check(A, b, x)
+    assert np.array_equal(xs[0], xs[1])
+    assert count[1] < count[0] or (n, mode) == (56, "fp32")  # (fits)
+
+
 @pytest.mark.parametrize("mode", ["fp64", "ir"])
 @pytest.mark.parametrize("cell,order,ncomp,n", [
     ("hex", 2, 1, 25), ("quad", 2, 1, 250), ("quad", 2, 2, 170), ("hex", 1, 3, 41), ("hex", 2, 3, 17)])
