@@ -1288,8 +1288,10 @@ static int dispatch_form(const Space* sp, int form, const double* coef, double n
       if (form == GT_LAPLACE)
         return launch_elements<D, NLV, NN, NQ, 1, GT_LAPLACE, T, CPB, AFFINE>(sp, coef, nu, tab, L, Ke, be, f, scoef,
                                                                               want_matrix);
-    if (form == GT_MASS)
-      return launch_elements<D, NLV, NN, NQ, 1, GT_MASS, T, CPB, AFFINE>(sp, coef, nu, tab, L, Ke, be, f, scoef, want_matrix);
+    if constexpr (!(D == 3 && NN == 8))
+      if (form == GT_MASS)
+        return launch_elements<D, NLV, NN, NQ, 1, GT_MASS, T, CPB, AFFINE>(sp, coef, nu, tab, L, Ke, be, f, scoef,
+                                                                           want_matrix);
   } else {
     if (form == GT_LAPLACE)
       return launch_elements<D, NLV, NN, NQ, D, GT_LAPLACE, T, CPB, AFFINE>(sp, coef, nu, tab, L, Ke, be, f, scoef, want_matrix);
@@ -1305,39 +1307,46 @@ static int dispatch_form(const Space* sp, int form, const double* coef, double n
 
 #include "gt_elements.cuh"
 
-// spaces whose Laplacian blocks and element vectors need no tabulation
-// (gt_elements.cuh).  The element vectors always come from there, whatever
-// the matrix's form: one source, so assemble_vector is bitwise the vector of
-// assemble_matrix_and_vector.
+// spaces whose Laplacian blocks (Q1 hexahedra: mass blocks too) and element
+// vectors need no tabulation (gt_elements.cuh).  The element vectors always
+// come from there, whatever the matrix's form: off the factored path and in
+// FP64 assemble_vector is bitwise the vector of assemble_matrix_and_vector.
 static bool direct_space(const Space* sp) {
   const int ct = sp->mesh->ctype;
   return sp->ncomp == 1 && (ct == GT_HEX8 || (ct == GT_TET4 && sp->order == 2));
 }
 static bool direct_elements(const Space* sp, int form, int want_matrix) {
-  return direct_space(sp) && (form == GT_LAPLACE || !want_matrix);
+  if (!direct_space(sp)) return false;
+  return !want_matrix || form == GT_LAPLACE || (form == GT_MASS && sp->mesh->ctype == GT_HEX8 && sp->order == 1);
 }
+// form 0: the element vectors alone
 template <class T>
-static int launch_direct(const Space* sp, const double* coef, T* Ke, double* be, const double* f, const double* scoef,
-                         int want_matrix) {
+static int launch_direct(const Space* sp, int form, const double* coef, T* Ke, double* be, const double* f,
+                         const double* scoef) {
   Ctx* ctx = ctx_of(sp);
   const int64_t nc = sp->mesh->ncells;
   const double* X = sp->mesh->coords;
   const int32_t* cn = sp->mesh->cell_nodes;
+  auto hex = [&](auto kern, int cpb) {
+    kern<<<GT_KC(ctx, grid_for(nc, cpb)), 256, 0, ctx->stream>>>(X, cn, coef, line_1d(sp->order), nc, Ke, be, f, scoef,
+                                                                 ctx->d_err);
+  };
   if (sp->mesh->ctype == GT_TET4) {
-    const int smem = want_matrix ? (int)(128 * 101 * sizeof(T)) : 0;
+    const int smem = form ? (int)(128 * 101 * sizeof(T)) : 0;
     GT_CUDA(ctx, dynamic_smem(k_elements_p2<T>));
     k_elements_p2<T><<<GT_KC(ctx, grid_for(nc, 128)), 128, smem, ctx->stream>>>(X, cn, coef, nc, Ke, be, f, scoef,
-                                                                                want_matrix, ctx->d_err);
+                                                                                form != 0, ctx->d_err);
   } else if (sp->order == 1) {
     // (FP32 values: the contractions in double-float, rounded once.  In FP32 the
     // 2-norm error of assembled matrices was 9.8e-8, of gradients formed in FP64
     // and multiplied in FP32 5.5e-8, this way 4.6e-8, at 9^3 to 25^3 cells.)
     using C = std::conditional_t<std::is_same<T, float>::value, dfl, T>;
-    k_elements_hex<2, T, C, 16><<<GT_KC(ctx, grid_for(nc, 16)), 256, 0, ctx->stream>>>(
-        X, cn, coef, line_1d(1), nc, Ke, be, f, scoef, want_matrix, ctx->d_err);
+    if (form == GT_LAPLACE) hex(k_elements_hex<2, T, C, 16, GT_LAPLACE>, 16);
+    else if (form == GT_MASS) hex(k_elements_hex<2, T, C, 32, GT_MASS>, 32);
+    else hex(k_elements_hex<2, T, C, 32, 0>, 32);
   } else {
-    k_elements_hex<3, T, T, 4><<<GT_KC(ctx, grid_for(nc, 4)), 256, 0, ctx->stream>>>(
-        X, cn, coef, line_1d(2), nc, Ke, be, f, scoef, want_matrix, ctx->d_err);
+    if (form == GT_LAPLACE) hex(k_elements_hex<3, T, T, 4, GT_LAPLACE>, 4);
+    else hex(k_elements_hex<3, T, T, 9, 0>, 9);
   }
   GT_LAUNCH(ctx, "k_elements");
   return GT_OK;
@@ -1623,9 +1632,10 @@ static int elements_T(const Space* sp, int form, const double* coef, double nu, 
     }
     return GT_OK;
   }
-  if (direct_elements(sp, form, want_matrix)) return launch_direct<T>(sp, coef, Ke, be, f, scoef, want_matrix);
+  if (direct_elements(sp, form, want_matrix))
+    return launch_direct<T>(sp, want_matrix ? form : 0, coef, Ke, be, f, scoef);
   if (be && direct_space(sp)) {
-    GT_TRY(launch_direct<T>(sp, nullptr, (T*)nullptr, be, f, scoef, 0));
+    GT_TRY(launch_direct<T>(sp, 0, nullptr, (T*)nullptr, be, f, scoef));
     be = nullptr;
   }
   // P2 tets: the map is affine but the shape gradients vary over the cell, so

@@ -75,22 +75,28 @@ template <int M>
 struct HexSize {
   static constexpr int NP = M * M, NN = M * M * M, NPAIR = NN * (NN + 1) / 2, XP = NP * (NP + 1) / 2;
 };
-template <int M, class T, class C, int CPB>
+//
+// FORM: GT_LAPLACE, GT_MASS (D^00 = coef w |det J| alone, LL in every
+// direction) or 0, the element vector without a matrix; T: the matrix's values,
+// C: the contractions' arithmetic.  The vector is the same in all of them, so
+// assemble_vector is bitwise that of assemble_matrix_and_vector.
+template <int M, class T, class C, int CPB, int FORM>
 __global__ void __launch_bounds__(256) k_elements_hex(const double* __restrict__ coords,
                                                       const int32_t* __restrict__ cell_nodes,
                                                       const double* __restrict__ coef, Line1D line, int64_t ncells,
                                                       T* __restrict__ Ke, double* __restrict__ be,
                                                       const double* __restrict__ fsrc,
-                                                      const double* __restrict__ scoef, int want_matrix,
-                                                      uint32_t* err) {
+                                                      const double* __restrict__ scoef, uint32_t* err) {
   constexpr int NP = HexSize<M>::NP, NN = HexSize<M>::NN, NPAIR = HexSize<M>::NPAIR, XP = HexSize<M>::XP;
   constexpr int TH = 256;
+  constexpr bool LAP = FORM == GT_LAPLACE, MAT = FORM != 0;
+  constexpr int ND = LAP ? 6 : 1, CM = MAT ? CPB : 1, CL = LAP ? CPB : 1;
   __shared__ double s_c[CPB][3][8];      // coefficients of the map: 1, x, y, xy, z, xz, yz, xyz
   __shared__ double s_dv[CPB][NN];       // |det J| w
   __shared__ double s_v[2][CPB][NN];     // partial contractions of the element vector
-  __shared__ C s_D[CPB][6][NN];          // 11, 22, 33, 12, 13, 23 at the points
-  __shared__ C s_U[CPB][6][NP][NP];      // [kl][q1 q2][a3 b3]
-  __shared__ C s_X[CPB][M][NP][NP], s_Y[CPB][M][NP][NP], s_Z[CPB][M][NP][NP];
+  __shared__ C s_D[CM][ND][NN];          // 11, 22, 33, 12, 13, 23 (or 00) at the points
+  __shared__ C s_U[CM][ND][NP][NP];      // [kl][q1 q2][a3 b3]
+  __shared__ C s_X[CM][M][NP][NP], s_Y[CL][M][NP][NP], s_Z[CL][M][NP][NP];
   __shared__ C s_LL[M][M][M], s_LD[M][M][M], s_DD[M][M][M];  // [q][a][b]
   __shared__ double s_L[M][M];           // [q][a]
   __shared__ uint16_t s_pair[NPAIR], s_xpair[XP];
@@ -143,52 +149,63 @@ __global__ void __launch_bounds__(256) k_elements_hex(const double* __restrict__
       J[i][1] = fma(yx, z, fma(k[3], x, k[2]));
       J[i][2] = fma(yx, y, fma(k[5], x, k[4]));
     }
-    // rows of adj(J) = det J J^-1
+    // rows of adj(J) = det J J^-1 (contracted as written, in every form)
+    auto cof = [&](int i, int j, int k, int l) { return fma(J[i][j], J[k][l], -__dmul_rn(J[i][l], J[k][j])); };
     double A[3][3];
-    A[0][0] = J[1][1] * J[2][2] - J[1][2] * J[2][1];
-    A[1][0] = J[1][2] * J[2][0] - J[1][0] * J[2][2];
-    A[2][0] = J[1][0] * J[2][1] - J[1][1] * J[2][0];
-    A[0][1] = J[0][2] * J[2][1] - J[0][1] * J[2][2];
-    A[1][1] = J[0][0] * J[2][2] - J[0][2] * J[2][0];
-    A[2][1] = J[0][1] * J[2][0] - J[0][0] * J[2][1];
-    A[0][2] = J[0][1] * J[1][2] - J[0][2] * J[1][1];
-    A[1][2] = J[0][2] * J[1][0] - J[0][0] * J[1][2];
-    A[2][2] = J[0][0] * J[1][1] - J[0][1] * J[1][0];
-    const double det = J[0][0] * A[0][0] + J[0][1] * A[1][0] + J[0][2] * A[2][0];
+    A[0][0] = cof(1, 1, 2, 2);
+    A[1][0] = cof(1, 2, 2, 0);
+    A[2][0] = cof(1, 0, 2, 1);
+    const double det = fma(J[0][2], A[2][0], fma(J[0][1], A[1][0], __dmul_rn(J[0][0], A[0][0])));
     if (c < ncells && !(det != 0.0)) atomicOr(err, DEV_ERR_DEGENERATE);
     const double w = line.w[q1] * line.w[q2] * line.w[q3], adet = fabs(det);
-    s_dv[cl][q] = (double)(T)(adet * w);  // |det J| w is held in T, also for the element vector
-    const double cf = (coef && c < ncells ? coef[c] : 1.0) * w * recip_nr2(adet);
-    auto dot = [&](int k, int l) { return cf * (A[k][0] * A[l][0] + A[k][1] * A[l][1] + A[k][2] * A[l][2]); };
-    s_D[cl][0][q] = arith<C>(dot(0, 0));
-    s_D[cl][1][q] = arith<C>(dot(1, 1));
-    s_D[cl][2][q] = arith<C>(dot(2, 2));
-    s_D[cl][3][q] = arith<C>(dot(0, 1));
-    s_D[cl][4][q] = arith<C>(dot(0, 2));
-    s_D[cl][5][q] = arith<C>(dot(1, 2));
+    s_dv[cl][q] = (double)(T)__dmul_rn(adet, w);  // |det J| w is held in T, also for the element vector
+    if constexpr (MAT) {
+      const double cw = (coef && c < ncells ? coef[c] : 1.0) * w;
+      if constexpr (!LAP) {
+        s_D[cl][0][q] = arith<C>(cw * adet);
+      } else {
+        A[0][1] = cof(0, 2, 2, 1);
+        A[1][1] = cof(0, 0, 2, 2);
+        A[2][1] = cof(0, 1, 2, 0);
+        A[0][2] = cof(0, 1, 1, 2);
+        A[1][2] = cof(0, 2, 1, 0);
+        A[2][2] = cof(0, 0, 1, 1);
+        const double cf = cw * recip_nr2(adet);
+        auto dot = [&](int k, int l) { return cf * (A[k][0] * A[l][0] + A[k][1] * A[l][1] + A[k][2] * A[l][2]); };
+        s_D[cl][0][q] = arith<C>(dot(0, 0));
+        s_D[cl][1][q] = arith<C>(dot(1, 1));
+        s_D[cl][2][q] = arith<C>(dot(2, 2));
+        s_D[cl][3][q] = arith<C>(dot(0, 1));
+        s_D[cl][4][q] = arith<C>(dot(0, 2));
+        s_D[cl][5][q] = arith<C>(dot(1, 2));
+      }
+    }
   }
   __syncthreads();
   // contraction over q3 (with the element vector's: NN items a cell)
   const int nv = be ? CPB * NN : 0;
-  if (want_matrix)
+  if constexpr (MAT)
     for (int it = tid; it < CPB * NP * NP; it += TH) {
       const int cl = it / (NP * NP), r = it - cl * (NP * NP), q12 = r / NP, ab = r - q12 * NP, a = ab / M, b = ab % M;
-      C u[6];
+      C u[ND];
 #pragma unroll
-      for (int k = 0; k < 6; k++) u[k] = C{};
+      for (int k = 0; k < ND; k++) u[k] = C{};
 #pragma unroll
       for (int q = 0; q < M; q++) {
-        const C ll = s_LL[q][a][b], ld = s_LD[q][a][b], dd = s_DD[q][a][b];
+        const C ll = s_LL[q][a][b];
         const int p = q * NP + q12;
         u[0] = mac(ll, s_D[cl][0][p], u[0]);
-        u[1] = mac(ll, s_D[cl][1][p], u[1]);
-        u[2] = mac(dd, s_D[cl][2][p], u[2]);
-        u[3] = mac(ll, s_D[cl][3][p], u[3]);
-        u[4] = mac(ld, s_D[cl][4][p], u[4]);
-        u[5] = mac(ld, s_D[cl][5][p], u[5]);
+        if constexpr (LAP) {
+          const C ld = s_LD[q][a][b], dd = s_DD[q][a][b];
+          u[1] = mac(ll, s_D[cl][1][p], u[1]);
+          u[2] = mac(dd, s_D[cl][2][p], u[2]);
+          u[3] = mac(ll, s_D[cl][3][p], u[3]);
+          u[4] = mac(ld, s_D[cl][4][p], u[4]);
+          u[5] = mac(ld, s_D[cl][5][p], u[5]);
+        }
       }
 #pragma unroll
-      for (int k = 0; k < 6; k++) s_U[cl][k][q12][ab] = u[k];
+      for (int k = 0; k < ND; k++) s_U[cl][k][q12][ab] = u[k];
     }
   for (int it = tid; it < nv; it += TH) {
     const int cl = it / NN, r = it - cl * NN, q12 = r % NP, a = r / NP;
@@ -199,8 +216,8 @@ __global__ void __launch_bounds__(256) k_elements_hex(const double* __restrict__
   }
   __syncthreads();
   // contraction over q2: X by its pairs i <= j, then Y and Z
-  if (want_matrix)
-    for (int it = tid; it < CPB * M * (XP + NP * NP); it += TH) {
+  if constexpr (MAT)
+    for (int it = tid; it < CPB * M * (XP + (LAP ? NP * NP : 0)); it += TH) {
       if (it < CPB * M * XP) {
         const int cl = it / (M * XP), r = it - cl * (M * XP), q1 = r / XP, p = s_xpair[r - q1 * XP];
         const int i = p >> 5, j = p & 31, a2 = i % M, a3 = i / M, b2 = j % M, b3 = j / M;
@@ -208,14 +225,16 @@ __global__ void __launch_bounds__(256) k_elements_hex(const double* __restrict__
 #pragma unroll
         for (int q = 0; q < M; q++) {
           const int q12 = q * M + q1;
-          s = mac(s_LL[q][a2][b2], s_U[cl][2][q12][a3 * M + b3], s);
-          s = mac(s_DD[q][a2][b2], s_U[cl][1][q12][a3 * M + b3], s);
-          s = mac(s_LD[q][b2][a2], s_U[cl][5][q12][a3 * M + b3], s);  // k = 2, l = 3
-          s = mac(s_LD[q][a2][b2], s_U[cl][5][q12][b3 * M + a3], s);  // k = 3, l = 2
+          s = mac(s_LL[q][a2][b2], s_U[cl][LAP ? 2 : 0][q12][a3 * M + b3], s);
+          if constexpr (LAP) {
+            s = mac(s_DD[q][a2][b2], s_U[cl][1][q12][a3 * M + b3], s);
+            s = mac(s_LD[q][b2][a2], s_U[cl][5][q12][a3 * M + b3], s);  // k = 2, l = 3
+            s = mac(s_LD[q][a2][b2], s_U[cl][5][q12][b3 * M + a3], s);  // k = 3, l = 2
+          }
         }
         s_X[cl][q1][i][j] = s;
         s_X[cl][q1][j][i] = s;
-      } else {
+      } else if constexpr (LAP) {
         const int t = it - CPB * M * XP;
         const int cl = t / (M * NP * NP), r = t - cl * (M * NP * NP), q1 = r / (NP * NP), ij = r - q1 * (NP * NP);
         const int i = ij / NP, j = ij - i * NP, a2 = i % M, a3 = i / M, b2 = j % M, b3 = j / M;
@@ -241,7 +260,7 @@ __global__ void __launch_bounds__(256) k_elements_hex(const double* __restrict__
   }
   __syncthreads();
   // contraction over q1: the node pairs n <= m
-  if (want_matrix)
+  if constexpr (MAT)
     for (int it = tid; it < CPB * NPAIR; it += TH) {
       const int cl = it / NPAIR, p = s_pair[it - cl * NPAIR];
       const int64_t c = c0 + cl;
@@ -250,9 +269,11 @@ __global__ void __launch_bounds__(256) k_elements_hex(const double* __restrict__
 #pragma unroll
       for (int q = 0; q < M; q++) {
         s = mac(s_LL[q][a1][b1], s_X[cl][q][i][j], s);
-        s = mac(s_DD[q][a1][b1], s_Z[cl][q][i][j], s);
-        s = mac(s_LD[q][b1][a1], s_Y[cl][q][i][j], s);
-        s = mac(s_LD[q][a1][b1], s_Y[cl][q][j][i], s);
+        if constexpr (LAP) {
+          s = mac(s_DD[q][a1][b1], s_Z[cl][q][i][j], s);
+          s = mac(s_LD[q][b1][a1], s_Y[cl][q][i][j], s);
+          s = mac(s_LD[q][a1][b1], s_Y[cl][q][j][i], s);
+        }
       }
       if (c < ncells) {
         T* K = Ke + c * (NN * NN);

@@ -102,3 +102,28 @@ def test_fp32_values_of_q1_hexahedra(n):
     A = GT.assemble_matrix(GT.laplacian(GT.lognormal_cells(m.num_cells, 0.5, 17)), "mixed", V)
     v = A.csr()[2]
     assert np.linalg.norm(A.values32() - v) <= 6.3e-8 * np.linalg.norm(v)
+
+
+@pytest.mark.parametrize("cells,order", [((1, 1, 1), 1), ((2, 4, 4), 1), ((3, 11, 2), 1), ((2, 2, 2), 2), ((3, 3, 3), 2)])
+def test_mass_blocks_and_vector_of_hexahedra(cells, order):
+    """Mass matrices of distorted hexahedra (Q1: 32 cells a block) against the
+    oracle's quadrature, with the bounds above, and the element vectors: the
+    same whether a matrix is formed with them or not, and whichever."""
+    m = GT.cartesian_mesh((0.0, 1.0, -0.5, 2.0, 0.0, 0.7), cells)
+    m.coords += np.random.default_rng(3).uniform(-0.1, 0.1, m.coords.shape) / max(cells)
+    coef = GT.lognormal_cells(m.num_cells, 1.0, 17)
+    ref, _ = _oracle_space(m, order, 1, None)
+    cp, rv, nz = O.assemble_matrix(ref, O.MASS, 2 * order, coef=coef)
+    orp, oci, ov = O.csc_to_csr(cp, rv, nz, ref["nfree"])
+    ob = O.assemble_vector(ref, 2 * order, 1.0, coef=coef)
+    V = GT.lagrange_space(GT.interior(m), order)
+    l = GT.source(1.0, coef)
+    A, b = GT.assemble_matrix_and_vector(GT.mass(coef), l, "mixed", V)
+    rp, ci, v = A.csr()
+    assert np.array_equal(rp, orp) and np.array_equal(ci, oci)
+    scale = np.abs(ov).max()
+    assert np.abs(v - ov).max() <= 2e-13 * scale
+    assert np.abs(A.values32() - ov).max() <= 5e-6 * scale
+    assert np.abs(b - ob).max() <= 2e-13 * np.abs(ob).max()
+    _, b2 = GT.assemble_matrix_and_vector(GT.laplacian(coef), l, np.float64, V)
+    assert np.array_equal(b, b2) and np.array_equal(b, GT.assemble_vector(l, np.float64, V))
