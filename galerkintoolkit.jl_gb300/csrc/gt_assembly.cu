@@ -3796,10 +3796,9 @@ int gt_matrix_download_csr(gt_matrix* A, int64_t* rowptr, int32_t* colind, doubl
     double* d64 = nullptr;
     float* d32 = nullptr;
     auto stage = [&](auto* out, auto** own, int64_t cnt) -> decltype(out) {
-      cudaPointerAttributes at{};
-      if (cudaPointerGetAttributes(&at, out) == cudaSuccess && at.type == cudaMemoryTypeDevice && at.device == ctx->device)
-        return out;
-      cudaGetLastError();
+      bool here = false;
+      s = device_output(ctx, out, (size_t)cnt * sizeof(*out), sizeof(*out), &here);
+      if (s != GT_OK || here) return out;
       s = dalloc(ctx, own, cnt);
       return *own;
     };
@@ -3813,7 +3812,7 @@ int gt_matrix_download_csr(gt_matrix* A, int64_t* rowptr, int32_t* colind, doubl
     if (!A->val64) v64 = nullptr;
     if (!A->val32) v32 = nullptr;
     if (s == GT_OK && (colind || v64)) {
-      int32_t* oc = colind ? stage(colind, &ci, nnz) : nullptr;
+      int32_t* oc = colind ? stage(colind, &ci, nnz) : nullptr;  // (sets s)
       double* ov = s == GT_OK && v64 ? stage(v64, &d64, nnz) : nullptr;
       if (s == GT_OK) {
         launch_expand<double>(ctx, A, A->val64, oc, ov);

@@ -4,6 +4,8 @@
 #include <cstdlib>
 #include <cstring>
 
+#include <cuda.h>
+
 #include "gt_internal.cuh"
 
 namespace gt {
@@ -140,6 +142,43 @@ int take_device_error(Ctx* ctx, uint32_t* bits) {
   *bits = dev | ctx->held_err;
   ctx->held_err = 0;
   if (dev) GT_CUDA(ctx, cudaMemsetAsync(ctx->d_err, 0, sizeof(uint32_t), ctx->stream));
+  return GT_OK;
+}
+
+int device_output(Ctx* ctx, const void* out, size_t bytes, size_t align, bool* here) {
+  *here = false;
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, out) != cudaSuccess) {
+    cudaGetLastError();
+    return GT_OK;
+  }
+  if (at.type != cudaMemoryTypeDevice || at.device != ctx->device || (uintptr_t)out % align != 0) return GT_OK;
+  // the allocation's range, from the driver (the runtime has no call for it)
+  using Range = CUresult (*)(CUdeviceptr*, size_t*, CUdeviceptr);
+  using Attribute = CUresult (*)(void*, CUpointer_attribute, CUdeviceptr);
+  static const auto entry = [](const char* name) {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPointByVersion(name, &f, 12000, cudaEnableDefault, &q) != cudaSuccess) {
+      cudaGetLastError();
+      f = nullptr;
+    }
+    return f;
+  };
+  static const Range range = (Range)entry("cuMemGetAddressRange");
+  static const Attribute attribute = (Attribute)entry("cuPointerGetAttribute");
+  CUdeviceptr base = 0;
+  size_t size = 0;
+  if (!range || range(&base, &size, (CUdeviceptr)out) != CUDA_SUCCESS) return GT_OK;
+  if ((CUdeviceptr)out + bytes <= base + size) {
+    *here = true;
+    return GT_OK;
+  }
+  int plain = 0;  // one allocation of cudaMalloc, not several ranges mapped side by side
+  if (attribute && attribute(&plain, CU_POINTER_ATTRIBUTE_IS_LEGACY_CUDA_IPC_CAPABLE, (CUdeviceptr)out) == CUDA_SUCCESS &&
+      plain)
+    return set_error(ctx, GT_ERR_INVALID, "output buffer: " + std::to_string(bytes) + " bytes are written, " +
+                                              std::to_string(base + size - (CUdeviceptr)out) + " are allocated");
   return GT_OK;
 }
 

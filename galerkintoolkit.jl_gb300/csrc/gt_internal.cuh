@@ -184,6 +184,13 @@ struct Blocks {
 // reads the device error word (synchronises the stream) and clears it
 int take_device_error(Ctx* ctx, uint32_t* bits);
 
+// *here: a kernel may write bytes at out in place -- memory of the context's
+// device, aligned to align, all of it in out's allocation.  (Other pointers go
+// through a block of the pool and a copy, which takes host memory, other
+// devices and any alignment.)  GT_ERR_INVALID when an allocation of cudaMalloc
+// is too small for the output.
+int device_output(Ctx* ctx, const void* out, size_t bytes, size_t align, bool* here);
+
 // copy n elements from a host or device pointer (unified addressing)
 template <class T>
 int copy_in(Ctx* ctx, T* dst, const T* src, int64_t n) {

@@ -883,9 +883,8 @@ int gt_space_cell_dofs(const gt_space* sp, int32_t* out) {
   Ctx* ctx = sp->mesh->ctx;
   int64_t n = sp->mesh->ncells * sp->nloc;
   // a device output is written in place, a host one through a staging block
-  cudaPointerAttributes at{};
-  const bool here = cudaPointerGetAttributes(&at, out) == cudaSuccess && at.type == cudaMemoryTypeDevice && at.device == ctx->device;
-  cudaGetLastError();
+  bool here = false;
+  GT_TRY(device_output(ctx, out, sizeof(int32_t) * n, sizeof(int32_t), &here));
   int32_t* tmp = nullptr;
   if (!here) GT_TRY(dalloc(ctx, &tmp, n));
   k_expand_cell_dofs<<<GT_KC(ctx, grid_for(n, 256)), 256, 0, ctx->stream>>>(sp->cell_ndofs, sp->mesh->ncells, sp->nn, sp->ncomp,

@@ -119,3 +119,46 @@ def test_async_coordinate_upload():
         V.dmesh.set_coords(src.pin_memory() if pinned else src)
         got = GT.assemble_matrix(GT.laplacian(None), np.float64, V, V).csr()[2]
         assert np.array_equal(got, want)
+
+
+def _elasticity(ctx=None):
+    m = GT.cartesian_mesh((0, 1, 0, 1, 0, 1), (20, 20, 20))
+    V = GT.lagrange_space(GT.interior(m), 1, tensor_size=(3,), dirichlet_boundary=GT.boundary(m, ["2-face-5"]), ctx=ctx)
+    return V, GT.assemble_matrix(GT.elasticity(), "mixed", V)
+
+
+@pytest.mark.parametrize("offset", [0, 4])
+def test_block_csr_into_the_end_of_device_memory(offset):
+    """The scalar CSR of a block matrix and the cells' DOFs written into the last
+    bytes of device allocations, at any alignment, equal the host's."""
+    V, A = _elasticity()
+    rp, ci, v = A.csr()
+    host = [rp, ci, v, A.values32()]
+    dev = []
+    for a in host + [V.face_dofs()]:
+        buf = torch.empty(a.nbytes + 64, dtype=torch.uint8, device="cuda")
+        dev.append(buf[64 - offset:64 - offset + a.nbytes])
+    ptr = [C.c_void_p(d.data_ptr()) for d in dev]
+    assert A.ctx.lib.gt_matrix_download_csr(A.h, *ptr[:4]) == _lib.GT_OK
+    assert V.ctx.lib.gt_space_cell_dofs(V.h, ptr[4]) == _lib.GT_OK
+    for a, d in zip(host + [V.face_dofs()], dev):
+        assert np.array_equal(d.cpu().numpy(), np.ascontiguousarray(a).reshape(-1).view(np.uint8))
+
+
+def test_device_outputs_too_small_are_refused():
+    """Outputs that do not fit the allocation they point into are refused before
+    anything is written."""
+    ctx = GT.Context(0)
+    V, A = _elasticity(ctx)
+    buf = GT.api.DeviceArray(ctx, 1 << 18)  # 2 MB in a block of at most 5 MB
+    assert A.nnz * 4 > 5 << 20 and V.mesh.num_cells * 24 * 4 < 2 << 20
+    p = C.c_void_p(buf.data_ptr())
+    lib = ctx.lib
+    assert lib.gt_matrix_download_csr(A.h, None, None, p, None) == _lib.GT_ERR_INVALID
+    assert b"output buffer" in lib.gt_last_error(ctx.h)
+    assert lib.gt_matrix_download_csr(A.h, None, p, None, None) == _lib.GT_ERR_INVALID
+    assert lib.gt_matrix_download_csr(A.h, None, None, None, p) == _lib.GT_ERR_INVALID
+    assert lib.gt_matrix_download_csr(A.h, p, None, None, None) == _lib.GT_OK  # (the row pointers fit)
+    assert lib.gt_space_cell_dofs(V.h, p) == _lib.GT_OK
+    del A, V, buf
+    ctx.close()
