@@ -454,6 +454,19 @@ int gt_ctx_barrier_probe(gt_ctx* c, int ctas, int missing, int64_t timeout_ns) {
   return barrier_probe(c, ctas, missing, timeout_ns);
 }
 
+int gt_ctx_sum_probe(gt_ctx* c, int ctas, int missing, int64_t timeout_ns, int precision, const double* values,
+                     double* total) {
+  if (!c) return GT_ERR_INVALID;
+  cudaSetDevice(c->device);
+  return sum_probe(c, ctas, missing, timeout_ns, precision, values, total);
+}
+
+int gt_ctx_divide_probe(gt_ctx* c, int64_t n, const double* a, const double* b, double* q) {
+  if (!c) return GT_ERR_INVALID;
+  cudaSetDevice(c->device);
+  return divide_probe(c, n, a, b, q);
+}
+
 int gt_ctx_launch_count(gt_ctx* c, int64_t* launches) {
   if (!c || !launches) return GT_ERR_INVALID;
   *launches = c->launches;

@@ -386,6 +386,9 @@ int spmv64(Matrix* A, const double* x, double* y);
 // the persistent solver's grid barrier run alone (gt_pcg.cu): ctas CTAs wait
 // for ctas + missing arrivals with the given time limit
 int barrier_probe(Ctx* ctx, int ctas, int missing, int64_t timeout_ns);
+// the local kernel's sum over CTAs (with its wait) and its division, alone
+int sum_probe(Ctx* ctx, int ctas, int missing, int64_t timeout_ns, int precision, const double* values, double* total);
+int divide_probe(Ctx* ctx, int64_t n, const double* a, const double* b, double* q);
 
 // A chunk of iterations of a CG loop, captured once into a CUDA graph and
 // replayed for every chunk: one graph launch instead of about five kernel

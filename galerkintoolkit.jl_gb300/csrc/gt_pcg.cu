@@ -34,6 +34,30 @@ __global__ void __launch_bounds__(PT) k_barrier_probe(uint32_t* bar, uint32_t ta
   grid_sync(bar, target, err, &s_abort, timeout_ns);
 }
 
+// The local kernel's sum run alone: each thread of `gridDim.x` CTAs brings one
+// value, and the CTAs wait for nb arrivals.
+template <class X>
+__global__ void __launch_bounds__(LT) k_sum_probe(const double* __restrict__ values, int nb, double* slots, int32_t* err,
+                                                  double* total, uint64_t timeout_ns) {
+  __shared__ LShared S;
+  if (threadIdx.x == 0) S.abort = 0;
+  __syncthreads();
+  uint32_t epoch = 0;
+  const X v[1] = {(X)values[(size_t)blockIdx.x * LT + threadIdx.x]};
+  local_total<1, false>(
+      v, LT, nb, blockIdx.x, slots, epoch, err, S, nullptr,
+      [&](const double* tot) {
+        if (blockIdx.x == 0) *total = tot[0];
+      },
+      timeout_ns);
+}
+
+__global__ void k_divide_probe(const double* __restrict__ a, const double* __restrict__ b, int64_t n,
+                               double* __restrict__ q) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i < n) q[i] = quick_div(a[i], b[i]);
+}
+
 }  // namespace pcg
 
 using namespace pcg;
@@ -65,6 +89,55 @@ int barrier_probe(Ctx* ctx, int ctas, int missing, int64_t timeout_ns) {
   dfree(ctx, bar);
   dfree(ctx, err);
   return e ? set_error(ctx, GT_ERR_TIMEOUT, "barrier probe: the grid barrier timed out") : GT_OK;
+}
+
+int sum_probe(Ctx* ctx, int ctas, int missing, int64_t timeout_ns, int precision, const double* values,
+              double* total) {
+  if (ctas < 1 || missing < 0 || ctas + missing > LMAXCTA || ctas > ctx->num_sms || timeout_ns <= 0 ||
+      timeout_ns > 2000000000ll || !values || !total || (precision != GT_FP64 && precision != GT_FP32))
+    return set_error(ctx, GT_ERR_INVALID, "sum probe: 1 <= ctas <= SMs, 0 <= missing, at most 160 CTAs, timeout <= 2 s");
+  cudaStream_t s = ctx->stream;
+  const int nb = ctas + missing;
+  Blocks mem(ctx);
+  double *dv, *slots, *dt;
+  int32_t* err;
+  GT_TRY(mem.get(&dv, (int64_t)ctas * LT));
+  GT_TRY(mem.get(&slots, (int64_t)LSLOTS * nb + LCTRS));
+  GT_TRY(mem.get(&dt, 1));
+  GT_TRY(mem.get(&err, 2));
+  GT_TRY(copy_in(ctx, dv, values, (int64_t)ctas * LT));
+  GT_CUDA(ctx, cudaMemsetAsync(slots, 0, sizeof(double) * (LSLOTS * nb + LCTRS), s));
+  GT_CUDA(ctx, cudaMemsetAsync(err, 0, 2 * sizeof(int32_t), s));
+  uint64_t tns = (uint64_t)timeout_ns;
+  int n = nb;
+  void* kargs[] = {&dv, &n, &slots, &err, &dt, &tns};
+  const void* kern = precision == GT_FP64 ? (const void*)k_sum_probe<double> : (const void*)k_sum_probe<float>;
+  ctx->launches++;
+  GT_CUDA(ctx, cudaLaunchCooperativeKernel(kern, dim3(ctas), dim3(LT), kargs, 0, s));
+  GT_CUDA(ctx, cudaMemcpyAsync(ctx->h_scratch, err, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+  GT_CUDA(ctx, cudaMemcpyAsync(ctx->h_dscratch, dt, sizeof(double), cudaMemcpyDeviceToHost, s));
+  GT_CUDA(ctx, cudaStreamSynchronize(s));
+  int32_t e = 0;
+  memcpy(&e, ctx->h_scratch, sizeof(int32_t));
+  if (e) return set_error(ctx, GT_ERR_TIMEOUT, "sum probe: the sum timed out");
+  memcpy(total, ctx->h_dscratch, sizeof(double));
+  return GT_OK;
+}
+
+int divide_probe(Ctx* ctx, int64_t n, const double* a, const double* b, double* q) {
+  if (n < 1 || !a || !b || !q) return set_error(ctx, GT_ERR_INVALID, "divide probe: empty");
+  Blocks mem(ctx);
+  double *da, *db, *dq;
+  GT_TRY(mem.get(&da, n));
+  GT_TRY(mem.get(&db, n));
+  GT_TRY(mem.get(&dq, n));
+  GT_TRY(copy_in(ctx, da, a, n));
+  GT_TRY(copy_in(ctx, db, b, n));
+  k_divide_probe<<<GT_KC(ctx, grid_for(n, 256)), 256, 0, ctx->stream>>>(da, db, n, dq);
+  GT_LAUNCH(ctx, "k_divide_probe");
+  GT_TRY(copy_out(ctx, q, dq, n));
+  GT_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  return GT_OK;
 }
 
 // pcg_persistent for several systems on ctx, grouped into shared launches by

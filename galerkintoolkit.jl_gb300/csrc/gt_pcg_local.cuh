@@ -218,7 +218,8 @@ struct LCluster {
 // arrive within the time limit (error word set; every CTA returns).
 template <int K, bool CL, class T, class F>
 __device__ __forceinline__ bool local_total(const T (&v)[K], int nth, int nb, int blk, double* slots, uint32_t& epoch,
-                                            int32_t* err, LShared& S, LCluster* C, F&& ctl) {
+                                            int32_t* err, LShared& S, LCluster* C, F&& ctl,
+                                            uint64_t timeout_ns = BAR_TIMEOUT_NS) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int nw = (min(nth, LT) + 31) >> 5;
   epoch++;
@@ -286,7 +287,7 @@ __device__ __forceinline__ bool local_total(const T (&v)[K], int nth, int nb, in
           if ((spin & 255) == 255) {
             const uint64_t now = global_ns();
             if (t0 == 0) t0 = now;
-            timed_out = now - t0 > BAR_TIMEOUT_NS;
+            timed_out = now - t0 > timeout_ns;
           }
           if (__any_sync(0xffffffffu, timed_out)) {
             if (lane == 0) {

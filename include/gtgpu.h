@@ -106,6 +106,14 @@ int gt_ctx_fma_rate(gt_ctx* ctx, int precision, double* tflops);
  * after the limit and the call returns GT_ERR_TIMEOUT with the context still
  * usable -- the path a solve takes when a barrier does not complete. */
 int gt_ctx_barrier_probe(gt_ctx* ctx, int ctas, int missing, int64_t timeout_ns);
+/* The same for the sum and barrier of the solver on CTA-local vectors, with
+ * its result: every one of the 512 threads of each of `ctas` CTAs brings a value
+ * (values: 512 x ctas, used in FP64 or rounded to FP32 by precision), *total
+ * receives their sum.  ctas + missing at most 160, one CTA an SM. */
+int gt_ctx_sum_probe(gt_ctx* ctx, int ctas, int missing, int64_t timeout_ns, int precision, const double* values,
+                     double* total);
+/* q[i] = a[i] / b[i] by that solver's division (n entries) */
+int gt_ctx_divide_probe(gt_ctx* ctx, int64_t n, const double* a, const double* b, double* q);
 /* Number of kernels the context has launched so far. */
 int gt_ctx_launch_count(gt_ctx* ctx, int64_t* launches);
 /* Number of CUDA-graph launches the context has made so far (the solver

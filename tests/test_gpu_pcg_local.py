@@ -7,11 +7,15 @@ The solver stops when its FP64 residual is at most rtol ||b||.  The same
 residual formed here differs from it by rounding alone, at most
 (row length + 2) eps sum |a_ij| |x_j| per entry; that bound is added to rtol.
 """
+import math
+
 import numpy as np
 import pytest
 import scipy.sparse as sp
 
 import gtgpu as GT
+from gtgpu import _lib
+from gtgpu.api import _ptr
 
 pytestmark = pytest.mark.gpu
 
@@ -178,3 +182,80 @@ def test_fp32_mode(cell, order, ncomp, n):
     assert abs(info["rel_residual"] - r / np.linalg.norm(b)) <= 1e-6 * info["rel_residual"]
     again, _ = GT.solve(A, b, rtol=1e-4, mode="fp32")
     assert np.array_equal(x, again)
+
+
+def _sum(values, fp32=False, missing=0, timeout=200_000_000):
+    ctx = GT.default_context()
+    values = np.ascontiguousarray(values, np.float64)
+    out = np.full(1, np.nan)
+    st = ctx.lib.gt_ctx_sum_probe(ctx.h, values.size // 512, missing, timeout,
+                                  _lib.GT_FP32 if fp32 else _lib.GT_FP64, _ptr(values), _ptr(out))
+    return st, out[0]
+
+
+@pytest.mark.parametrize("ctas", [1, 2, 33, 152])
+@pytest.mark.parametrize("fp32", [False, True])
+def test_sums_on_the_integer_pipes(ctas, fp32):
+    """Over a warp's lanes, a CTA's warps and the CTAs numbers are aligned to the
+    largest one and rounded 56, 56 and 53 bits below it: with at most 32, 16 and
+    160 of them, the total is off by 2^-52 + 2^-53 + 2^-46 of the magnitudes' sum
+    at most, and sums of whole numbers below 2^30 are exact."""
+    rng = np.random.default_rng(ctas)
+    n = 512 * ctas
+    whole = rng.integers(-2 ** 14, 2 ** 14, n).astype(np.float64)
+    assert _sum(whole, fp32) == (0, whole.sum())
+    assert _sum(rng.permutation(whole), fp32) == (0, whole.sum())
+    for spread in (0, 8, 30):
+        v = rng.standard_normal(n) * 2.0 ** rng.uniform(-spread, spread, n)
+        if fp32:
+            v = v.astype(np.float32).astype(np.float64)
+        st, t = _sum(v, fp32)
+        assert st == 0 and abs(t - math.fsum(v)) <= 2.0 ** -45 * math.fsum(np.abs(v))
+    one = np.zeros(n)
+    one[n // 2] = -1.7e-42 if fp32 else -4.9e-324  # subnormal
+    assert _sum(one, fp32)[1] == np.float64(np.float32(one[n // 2]) if fp32 else one[n // 2])
+    tiny = rng.integers(-999, 999, n) * 2.0 ** (-149 if fp32 else -1074)
+    assert _sum(tiny, fp32)[1] == math.fsum(tiny)
+    assert _sum(np.zeros(n), fp32) == (0, 0.0)
+    big = np.zeros(n)
+    big[:3] = [1.5 * 2.0 ** (127 if fp32 else 1023), 2.0 ** (126 if fp32 else 1022), -(2.0 ** (126 if fp32 else 1022))]
+    assert _sum(big, fp32)[1] == big[0]
+    for bad in (np.nan, np.inf, -np.inf):
+        one[n // 2] = bad
+        assert np.isnan(_sum(one, fp32)[1])
+
+
+def test_sum_of_a_missing_arrival_gives_up():
+    v = np.ones(512 * 16)
+    assert _sum(v)[0] == _lib.GT_OK
+    st, _ = _sum(v, missing=1, timeout=50_000_000)
+    assert st == _lib.GT_ERR_TIMEOUT
+    assert _sum(v, missing=160)[0] == _lib.GT_ERR_INVALID
+    assert _sum(v) == (_lib.GT_OK, 512.0 * 16)  # the context goes on
+    A, b = _system("quad", 1, 1, 40, np.float64)
+    assert GT.solve(A, b, rtol=RTOL, mode="fp64")[1]["converged"]
+
+
+def test_quick_division():
+    """within an ulp of the quotient; the division itself where an exponent is
+    near the ends of the range, and for zeros, infinities and NaN"""
+    rng = np.random.default_rng(1)
+    n = 200_000
+    e = np.concatenate([rng.uniform(-500, 500, n), [-511, -511, 511.9, 511.9] * 50])
+    a = rng.uniform(1, 2, e.size) * 2.0 ** np.floor(e) * rng.choice([-1, 1], e.size)
+    b = rng.uniform(1, 2, e.size) * 2.0 ** np.floor(rng.permutation(e)) * rng.choice([-1, 1], e.size)
+    edge = np.array([0.0, -0.0, np.inf, -np.inf, np.nan, 5e-324, 1e-310, 1e308, 2.0 ** -512, 2.0 ** 513, 1.0, -3.0])
+    A, B = (x.ravel() for x in np.meshgrid(edge, edge))
+    a, b = np.concatenate([a, A]), np.concatenate([b, B])
+    q = np.empty_like(a)
+    ctx = GT.default_context()
+    assert ctx.lib.gt_ctx_divide_probe(ctx.h, a.size, _ptr(a), _ptr(b), _ptr(q)) == 0
+    with np.errstate(all="ignore"):
+        want = a / b
+        m = e.size
+        assert np.all(np.abs(q[:m] - want[:m]) <= np.spacing(np.abs(want[:m])))
+    ea, eb = (np.frexp(x[m:])[1] + 1022 for x in (a, b))
+    plain = (np.minimum(ea, eb) < 512) | (np.maximum(ea, eb) > 1535) | (a[m:] == 0) | (b[m:] == 0)
+    plain |= ~np.isfinite(a[m:]) | ~np.isfinite(b[m:])
+    assert np.array_equal(q[m:][plain], want[m:][plain], equal_nan=True)
+    assert np.all(np.abs(q[m:][~plain] - want[m:][~plain]) <= np.spacing(np.abs(want[m:][~plain])))
