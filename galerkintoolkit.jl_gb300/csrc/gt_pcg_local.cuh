@@ -772,8 +772,11 @@ __device__ __forceinline__ void pcg_local_body(const PArgs& a, int nb, int blk, 
       if (s_rp[mid] <= cap) lo = mid;
       else hi = mid - 1;
     }
-    // whole groups of rows (local_group), unless all fit
-    if (lo < nr) with_lanes<BS>(a.lanes, [&](auto jt) { lo -= lo % (32 / (BS * decltype(jt)::value)); });
+    // unless all fit, whole groups of rows (local_group) or, BS = 3, of the
+    // warps' rounds over them: residual() goes from resident to other rows there
+    if constexpr (XL)
+      if (lo < nr)
+        with_lanes<BS>(a.lanes, [&](auto jt) { lo -= lo % (32 / (BS * decltype(jt)::value) * (BS == 3 ? LNW : 1)); });
     S.rsm = lo;
   }
   __syncthreads();
@@ -842,10 +845,13 @@ __device__ __forceinline__ void pcg_local_body(const PArgs& a, int nb, int blk, 
       constexpr int J = decltype(jt)::value, GPW = 32 / (BS * J), U = BS == 1 ? 8 : 4;
       if constexpr (XL) {
         // (resident rows end between two of a warp's groups, or with the rows;
-        // two loops: the compiler then reads s_lc as shared memory)
+        // two loops: the compiler then reads s_lc as shared memory.  BS = 3: the
+        // second starts at a round of 32 rows; going on from the first's last
+        // row, the same rows, was up to 3.5% slower: 4^3 to 13^3 Q2 elasticity)
         const double* v64 = a.val64 + (size_t)k0 * BS * BS;
         int row0 = wid * GPW;
         for (; row0 < rsm; row0 += LNW * GPW) local_group<BS, J, U, double>(row0, rsm, s_rp, v64, s_lc, getl, put);
+        if constexpr (BS == 3) row0 = rsm + wid * GPW;
         for (; row0 < nr; row0 += LNW * GPW) local_group<BS, J, U, double>(row0, nr, s_rp, v64, glc, getl, put);
       } else {
         const auto* v64 = [&] {
