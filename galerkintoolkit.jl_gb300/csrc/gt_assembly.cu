@@ -614,8 +614,9 @@ __device__ __forceinline__ void thread_sort(int32_t* v) {
 // *redo the warp kernel recounts every row.
 // C16: the space's DOF spread is below 2^15, so every column differs from
 // its row by less than 2^15 and the list holds column - row in 16 bits:
-// 192 instead of 256 bytes of shared memory per thread, up to 9 instead of 6
-// blocks per SM (the pass is bound by shared-memory latency, not bandwidth).
+// 192 instead of 256 bytes of shared memory per thread, room for 9 instead of
+// 6 blocks per SM, of which the registers of NN = 4 let 7 in (the pass is bound
+// by shared-memory latency, not bandwidth).
 constexpr int kRowsMI = 32, kRowsS = 32;
 static_assert(kIncBucket == kRowsMI, "a bucket holds the incidences the row-per-thread pass takes");
 template <int NN, bool C16>

@@ -237,8 +237,8 @@ int pcg_persistent(Matrix* A, int mode, const double* b, double* x, double rtol,
                : run_dispatch<float, float, true>(A, A->val32, b, x, rtol, maxit, ctx->ir_delta, nullptr, &run);
     if (s == PCG_STALLED) {
       // the FP32 iteration stalled or lost its rate (eps32 * cond(A) too
-      // large): the same Krylov iteration goes on in FP64 from the current
-      // FP64 solution and the FP32 direction
+      // large): CG goes on in FP64 from the current FP64 solution, its
+      // directions restarted (the iteration count and ||b|| carry over)
       PRun r32 = run;
       PRun r64;
       s = sliced ? run_sliced<double, double, true>(ctx, A, A->val64, b, x, rtol, maxit, 0.0, &r32, &r64, 0) : PCG_NOFIT;

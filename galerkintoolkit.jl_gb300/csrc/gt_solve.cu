@@ -1123,8 +1123,8 @@ int solve(Matrix* A, const double* b, double* x, double rtol, int maxit, int mod
   if (mode != GT_SOLVE_FP64 && mode != GT_SOLVE_FP32 && mode != GT_SOLVE_IR)
     return set_error(ctx, GT_ERR_INVALID, "unknown solve mode");
   // the persistent kernel saves the per-phase launches and grid-wide
-  // reduction tails that dominate small systems; large systems keep more
-  // loads in flight with one launch per phase (measured crossover)
+  // reduction tails that dominate small systems; larger ones, whose CTA-local
+  // sets do not fit, keep more loads in flight with one launch per phase
   bool persistent = ctx->pcg_path == 2 || (ctx->pcg_path == 0 && n <= kPersistentMaxRows);
   int32_t it = 0, nupd = 0, it64 = 0;
   if (persistent) {

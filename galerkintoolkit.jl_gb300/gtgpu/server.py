@@ -296,10 +296,13 @@ class Server:
         # requests up to batch_rows scalar rows go through gt_batch (alone
         # or with others, up to batch_max); batching=False: one grid-wide
         # solve per request.  In a batch, requests up to small_rows are
-        # solved by one CTA or one cluster each, so that tier lasts as long as its largest
-        # member: the limit keeps it short (on GB300, under the 2000 req/s
-        # stream, 2048 scalar rows and batches of 16 completed 1.8x the
-        # requests of 32768 and 64 at a p50 of 10 ms instead of 0.4 s); the
+        # solved by one CTA or one cluster each, so that tier lasts as long as
+        # its largest member: the limit keeps it short (on GB300, under the
+        # 2000 req/s stream, 2048 scalar rows and batches of 16 completed 1.8x
+        # the requests of 32768 and 64 at a p50 of 10 ms instead of 0.4 s while
+        # one CTA solved every member; the limits were not chosen anew since
+        # members above 1,024 rows take clusters: 612 requests/s at a p50 of
+        # 9.7 ms, against 533 at 4.0 ms for one slot without batches); the
         # larger ones, when batch_rows lets them in, share grouped persistent
         # launches, each bitwise its own solve.  Measured with batch_rows
         # 262,144: 588 requests/s at a p50 of 138 ms against 604 at 9.3 ms
